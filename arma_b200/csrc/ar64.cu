@@ -4,28 +4,460 @@
 // zeta in place in C order; each point sums phi(k,i,j) * zeta(t-k,x-i,y-j)
 // over k, i, j ascending (truncated at the array start) into a running sum
 // that starts at 0, then adds the sum to the noise already stored at the
-// point.  Every point depends only on points with smaller t+x+y, so all points
-// of one hyperplane t+x+y = s are independent: one launch per hyperplane
-// computes them with each thread running the reference's sequential sum
-// (explicitly rounded multiply and add, no FMA contraction), which makes the
-// result bit-identical to the CPU.  The nt+nx+ny-2 launches are captured once
-// into a CUDA graph and replayed.
-#include <sstream>
+// point.  The sum is one chain of P explicitly rounded multiplies and adds (no
+// FMA contraction), so the result is bit-identical to the CPU.
+//
+// What bounds it.  A point's chain starts with its newest neighbour, (t,x,y-1),
+// so points run in parallel only on a hyperplane t+x+y = s, and a surface takes
+// nt+nx+ny-2 steps of P dependent additions, 8 cycles each: 2.7 ms for 400 x 128
+// x 128 of order 10^3 at 1965 MHz, whose arithmetic alone (a multiply and an add
+// per tap, 64 lanes of either per cycle and SM) takes 0.70 ms.
+//
+// One persistent launch covers any number of surfaces.  With u = x + y the
+// points of step s are t = s - u: a CTA owns a tile of TX rows x TU values of u
+// (a parallelogram in x, y) and walks the steps, a compute thread per cell.
+// Shared memory holds the last slices of the tile and its halo, by time (slot t
+// mod depth), zero outside the surface: a zero operand adds +-0, which leaves a
+// sum that starts at +0 as it is, so the chains need no truncation (coefficients
+// must be finite for that: others take the hyperplane kernel at the end of this
+// file).  A row of taps is read from there two rows ahead of its additions.  A
+// tile's halo comes from tiles with smaller x or u; a halo warp polls their step
+// counters and copies the new values from global memory, up to kMaxAhead steps
+// before their use, and a publication warp releases the tile's own counter, both
+// off the compute warps' path.  Tickets are handed out in dependency order, so a
+// CTA only waits on tiles that running CTAs own; every wait is bounded.
+//
+// Measured (B200, the filter alone): 400 x 128 x 128 of order 10^3 4.9 ms (one
+// launch per hyperplane, its taps read through L1: 70 ms), 14.7 cycles per tap
+// and step with four warps on an SM, where the taps' 2.5 shared-memory wavefronts
+// per warp queue, and 11.8 with two; 200 x 40 x 40 of order 7^3 0.70 ms (12.0).
+// Two cells of one u per thread, sharing their windows, moved fewer bytes but
+// issued 14.7 to 19 cycles per tap and step from its lone warp.
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <utility>
+#include <vector>
 
 #include "internal.h"
 
 namespace armab {
 namespace {
 
-constexpr int kThreads = 128;
+constexpr long long kSpinLimit = 1ll << 24;
+constexpr size_t kSmemLimit = 227 * 1024 - 64;  // less the kernel's static shared memory
+constexpr int kMaxAhead = 4;   // steps of halo kept ahead of their use
+constexpr int kUpstream = 5;   // tiles a tile's halo can come from
+constexpr int kBatch = 8;      // halo loads in flight per lane
 
-__global__ void __launch_bounds__(kThreads)
+struct Task64 {
+	int nt, nx, ny, pt, px, py;
+	int nbx, nc;      // tile rows, tiles per tile row
+	int ticket_base;
+	int ahead;        // halo steps kept ahead of their use
+	double* zeta;
+	const double* phi;
+	int* flags;       // per tile: the step (t + u) up to which it is done
+};
+
+// Layout of a tile's shared memory (doubles unless said otherwise).
+struct Layout64 {
+	int ld, slot, depth, phi, entries;
+	size_t bytes;
+};
+
+__host__ __device__ inline int even_up(int n) { return (n + 1) & ~1; }
+
+// Ring rows: TX plus px-1 above; columns: TU plus px+py-2 to the left.  A slot
+// is a multiple of 16 doubles, so that lanes of consecutive u (consecutive
+// columns of consecutive slots) fall in different banks.
+__host__ __device__ inline Layout64 layout64(int tx, int tu, int pt, int px, int py, int ahead) {
+	Layout64 l;
+	l.ld = tu + px + py - 2;
+	l.slot = ((tx + px - 1) * l.ld + 15) & ~15;
+	l.depth = tu + pt - 1 + ahead;
+	l.phi = (pt * px + 2) * even_up(py);  // and two rows that are loaded past the last
+	l.entries = (px - 1) * (tu + px + py - 2) + tx * (px + py - 2);
+	l.bytes = sizeof(double) * (size_t(l.slot) * l.depth + l.phi + even_up(l.entries));
+	return l;
+}
+
+__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
+	int v;
+	asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ void st_release_gpu(int* p, int v) {
+	asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int ld_acquire_cta(const int* p) {
+	int v;
+	const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+	asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+	return v;
+}
+__device__ __forceinline__ void st_release_cta(int* p, int v) {
+	const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+	asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int n) {
+	asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+	asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// Shared memory by 32-bit address (bytes), in program order: the loads stay
+// where they are written, ahead of their use and spread among the arithmetic.
+__device__ __forceinline__ double lds64(unsigned a) {
+	double v;
+	asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+	return v;
+}
+__device__ __forceinline__ void lds128(unsigned a, double& u, double& v) {
+	asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(u), "=d"(v) : "r"(a));
+}
+
+// (volatile: not moved into the next row's block)
+__device__ __forceinline__ double mul_here(double a, double b) {
+	double v;
+	asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(v) : "d"(a), "d"(b));
+	return v;
+}
+
+// One row of taps in three stages at once: the products m of this row are added
+// to the chain; the next row's products (taps c times window w) take their
+// place; the window (at zn) and taps (at cn) of the row after that load into w
+// and c as those are used up.  No addition waits for a product or a load of its
+// own row, so the chain runs at the add's latency.
+template <int PY, int M>
+__device__ __forceinline__ void row_step(double& s, double (&m)[PY], double (&w)[PY],
+                                         double (&c)[M], unsigned zn, unsigned cn) {
+#pragma unroll
+	for (int j = 0; j < PY; ++j) {
+		s = __dadd_rn(s, m[j]);
+		m[j] = mul_here(c[j], w[j]);
+		w[j] = lds64(zn - 8 * j);
+		if (j % 2 == 1 || j == PY - 1) lds128(cn + 8 * (j & ~1), c[j & ~1], c[(j & ~1) + 1]);
+	}
+}
+
+// What the warps of a CTA share about the current tile, and its named barriers
+// (0 is __syncthreads).  Step n of the compute warps ends at kBarHalo + n %
+// kHaloBars, where the halo warp has arrived when it has brought in step n + 1's
+// halo (up to kMaxAhead steps early), and each step's global stores are handed
+// over at kBarPub + n % kPubBars, which the compute warps only arrive at (up to
+// kPubBars steps early).
+struct Shared64 {
+	int done;       // steps completed by the compute warps
+	int published;  // steps whose stores the publication warp has taken over
+};
+constexpr int kHaloBars = kMaxAhead + 1, kPubBars = 8;
+constexpr int kBarHalo = 1, kBarPub = kBarHalo + kHaloBars;
+static_assert(kBarPub + kPubBars <= 16, "named barriers");
+
+// The halo warp: a list of the halo's cells inside the surface, then step
+// after step their new values.  A cell in row x' and column u' = U0 + d is read
+// from column max(U0, u' + b) of the tile on (b = X0 - x' rows above it, 0
+// beside it), so step n of the tile brings in its value of t = n - max(0, d +
+// b): a value that its owner computed at least max(1, b) steps before.  Tiles
+// further up than the five polled here are therefore covered by those, whose
+// own steps waited for them.  A wait that runs out sets the error word and lets
+// the compute warps run on without the halo: they end, and the call fails.
+template <int TX, int TU>
+__device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const Layout64& L, double* ring,
+                          int2* cells, Shared64* sh, int* err) {
+	const int lane = threadIdx.x & 31;
+	const int px = tk.px, left = px + tk.py - 2;
+	const int X0 = bx * TX, U0 = X0 + c * TU;
+	const int steps = tk.nt + TU - 1;
+	const int top = (px - 1) * (TU + left), all = top + TX * left;
+	int count = 0;
+	for (int q0 = 0; q0 < all; q0 += 32) {
+		const int q = q0 + lane;
+		int row = 0, col = 0;
+		if (q < top) {
+			row = q / (TU + left);
+			col = q % (TU + left);
+		} else if (q < all) {
+			row = px - 1 + (q - top) / left;
+			col = (q - top) % left;
+		}
+		const int x = X0 + row - (px - 1), d = col - left, y = U0 + d - x;
+		const int rel = max(0, d + max(0, X0 - x));
+		const bool ok = q < all && rel < TU && x >= 0 && x < tk.nx && y >= 0 && y < tk.ny;
+		const unsigned m = __ballot_sync(0xffffffffu, ok);
+		if (ok)
+			cells[count + __popc(m & ((1u << lane) - 1))] =
+			    make_int2(x * tk.ny + y, (row * L.ld + col) << 8 | rel);
+		count += __popc(m);
+	}
+	__syncwarp();
+	// the tiles they come from: two to the left, three above
+	const int* flag = nullptr;
+	int known = INT_MAX;  // the owner's steps t + u' below this are done
+	if (lane < kUpstream) {
+		const int ub = lane < 2 ? bx : bx - 1;
+		const int uc = lane < 2 ? c - 1 - lane : c + 1 - (lane - 2);
+		if (ub >= 0 && uc >= 0 && uc < tk.nc) {
+			flag = tk.flags + ub * tk.nc + uc;
+			known = ub * TX + uc * TU;
+		}
+	}
+	constexpr int kThreads = TX * TU + 32;
+	const long long plane = (long long)tk.nx * tk.ny;
+	int n = 0;
+	bool failed = false;
+	while (n < steps) {
+		// the steps n .. hi whose upstream values are there and whose ring
+		// slots are free (and whose barriers' previous round is over)
+		int hi = -1;
+		for (long long it = 0; it < kSpinLimit; ++it) {
+			const int freed = ld_acquire_cta(&sh->done) + tk.ahead;
+			hi = min(freed, known == INT_MAX ? INT_MAX : known - U0);
+			hi = min(__reduce_min_sync(0xffffffffu, hi), steps - 1);
+			if (hi >= n) break;
+			if (flag) known = max(known, ld_acquire_gpu(flag));
+			if ((it & 63) == 63 && *((volatile int*)err) != DEV_OK) failed = true;
+			if (__any_sync(0xffffffffu, failed)) break;
+			if (it > 0) __nanosleep(20);
+		}
+		if (hi < n) {  // no more waiting for the tiles upstream
+			if (lane == 0) atomicCAS(err, DEV_OK, DEV_TIMEOUT);
+			flag = nullptr;
+			known = INT_MAX;
+			failed = false;
+			continue;
+		}
+		// every (step, cell) of them, kBatch loads in flight per lane
+		const int total = (hi - n + 1) * count;
+		int e = lane, st = n, sm = n % L.depth;
+		auto settle = [&] {
+			while (e >= count) {
+				e -= count;
+				++st;
+				sm = sm + 1 == L.depth ? 0 : sm + 1;
+			}
+		};
+		for (int q0 = lane; q0 < total; q0 += 32 * kBatch) {
+			double v[kBatch];
+			int at[kBatch];
+#pragma unroll
+			for (int b = 0; b < kBatch; ++b) {
+				at[b] = -1;
+				if (q0 + 32 * b < total) {
+					settle();
+					const int2 cell = cells[e];
+					const int rel = cell.y & 255, t = st - rel;
+					if (t >= 0 && t < tk.nt) {
+						at[b] = (sm - rel + (sm < rel ? L.depth : 0)) * L.slot + (cell.y >> 8);
+						v[b] = __ldcg(tk.zeta + t * plane + cell.x);
+					}
+					e += 32;
+				}
+			}
+#pragma unroll
+			for (int b = 0; b < kBatch; ++b)
+				if (at[b] >= 0) ring[at[b]] = v[b];
+		}
+		// step n's halo is waited for at the end of step n - 1, step 0's by
+		// the CTA's barrier before the first
+		__syncwarp();
+		for (; n <= hi; ++n) {
+			if (n == 0) __syncthreads();
+			else bar_arrive(kBarHalo + (n - 1) % kHaloBars, kThreads);
+		}
+	}
+}
+
+// The publication warp: the barrier orders the compute warps' global stores of
+// a step before the release store that publishes it; steps that are handed over
+// meanwhile are published together.
+template <int TX, int TU>
+__device__ __forceinline__ void pub_warp(const Task64& tk, int bx, int c, Shared64* sh) {
+	constexpr int kThreads = TX * TU + 32;
+	int* flag = tk.flags + bx * tk.nc + c;
+	const int lane = threadIdx.x & 31;
+	const int U0 = bx * TX + c * TU, steps = tk.nt + TU - 1;
+	__syncthreads();  // step 0's halo
+	for (int n = 0; n < steps;) {
+		// this step, and those after it that the compute warps have left too
+		const int upto = max(n + 1, min(n + kPubBars, *((volatile int*)&sh->done) - 1));
+		const int last = min(__shfl_sync(0xffffffffu, upto, 0), steps);
+		for (; n < last; ++n) bar_sync(kBarPub + n % kPubBars, kThreads);
+		if (lane == 0) {
+			*((volatile int*)&sh->published) = n;
+			st_release_gpu(flag, n < steps ? U0 + n : INT_MAX);
+		}
+		__syncwarp();
+	}
+}
+
+template <int PY, int TX, int TU>
+__device__ __forceinline__ void compute_tile(const Task64& tk, int bx, int c, const Layout64& L,
+                                             double* ring, const double* sphi, Shared64* sh,
+                                             int* err) {
+	constexpr int NC = TX * TU;
+	constexpr int PYP = (PY + 1) & ~1;
+	const int l = threadIdx.x % TU, xl = threadIdx.x / TU;
+	const int px = tk.px, rows = tk.pt * px;
+	const int x = bx * TX + xl, y = bx * TX + c * TU + l - x;
+	const bool ok = x < tk.nx && y >= 0 && y < tk.ny;
+	const long long plane = (long long)tk.nx * tk.ny;
+	double* const z = tk.zeta + (long long)x * tk.ny + y;
+	double* const own = ring + (xl + px - 1) * L.ld + l + px + PY - 2;
+	unsigned own_a = static_cast<unsigned>(__cvta_generic_to_shared(own));
+	unsigned taps = static_cast<unsigned>(__cvta_generic_to_shared(sphi));
+	// one row up and one column left; one slot
+	unsigned row_bytes = 8u * unsigned(L.ld + 1), slot_bytes = 8u * unsigned(L.slot);
+	// (opaque: nothing is computed ahead for all widths of the kernel's switch)
+	asm volatile("" : "+r"(own_a), "+r"(taps), "+r"(row_bytes), "+r"(slot_bytes));
+	const int steps = tk.nt + TU - 1;
+	int slot = l == 0 ? 0 : L.depth - l;  // of t = n - l
+	double e = ok && l == 0 ? z[0] : 0.0;
+	__syncthreads();  // step 0's halo
+	for (int n = 0; n < steps; ++n) {
+		const int t = n - l;
+		// the next step's noise
+		const double f = ok && t + 1 >= 0 && t + 1 < tk.nt ? z[(t + 1) * plane] : 0.0;
+		double s = 0.0;
+		{
+			// rows of taps r = (k, i): row x-i of slice t-k
+			double w[PY], p[PYP], m[PY];
+			int ks = slot, i = 0;
+			unsigned pa = taps, za = own_a + unsigned(ks) * slot_bytes;
+			auto advance = [&] {  // to the next row
+				pa += 8 * PYP;
+				const bool wrap = i + 1 == px;
+				i = wrap ? 0 : i + 1;
+				const int kn = ks == 0 ? L.depth - 1 : ks - 1;
+				ks = wrap ? kn : ks;
+				za = wrap ? own_a + unsigned(ks) * slot_bytes : za - row_bytes;
+			};
+			// row 0's products and row 1's operands
+#pragma unroll
+			for (int j = 0; j < PY; ++j) w[j] = lds64(za - 8 * j);
+#pragma unroll
+			for (int j = 0; j < PYP; j += 2) lds128(pa + 8 * j, p[j], p[j + 1]);
+			w[0] = e;  // lag (0, 0, 0): the cell's own noise
+			advance();
+#pragma unroll
+			for (int j = 0; j < PY; ++j) {
+				m[j] = mul_here(p[j], w[j]);
+				w[j] = lds64(za - 8 * j);
+			}
+#pragma unroll
+			for (int j = 0; j < PYP; j += 2) lds128(pa + 8 * j, p[j], p[j + 1]);
+			// (the last two rows load rows past the last, within the ring and
+			// the padding after the taps: not used)
+			auto row = [&] {
+				advance();
+				row_step<PY>(s, m, w, p, za, pa);
+			};
+			// eight rows to a branch: a branch costs a lone warp about 30 cycles
+			int left = rows;
+			for (; left >= 8; left -= 8) {
+				row();
+				row();
+				row();
+				row();
+				row();
+				row();
+				row();
+				row();
+			}
+			for (; left > 0; --left) row();
+		}
+		s = __dadd_rn(e, s);
+		const bool live = ok && t >= 0 && t < tk.nt;
+		if (live) own[slot * L.slot] = s;
+		// every cell of step n is in the ring, and step n + 1's halo
+		if (n + 1 < steps) bar_sync(kBarHalo + n % kHaloBars, NC + 32);
+		// (released before this step's global stores: it waits for none)
+		if (threadIdx.x == 0) st_release_cta(&sh->done, n + 1);
+		if (live) z[t * plane] = s;
+		// the barrier's previous round is over once the publication warp has
+		// left it (it waits for nothing but these barriers)
+		for (long long it = 0; *((volatile int*)&sh->published) < n + 1 - kPubBars; ++it)
+			if (it == kSpinLimit * 64) {
+				atomicCAS(err, DEV_OK, DEV_TIMEOUT);
+				break;
+			}
+		__syncwarp();
+		bar_arrive(kBarPub + n % kPubBars, NC + 32);
+		e = f;
+		slot = slot + 1 == L.depth ? 0 : slot + 1;
+	}
+}
+
+template <int TX, int TU>
+__global__ void __launch_bounds__(TX * TU + 64)
+ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
+                 int* __restrict__ counter, int* __restrict__ err) {
+	constexpr int NC = TX * TU, NTHREADS = NC + 64;
+	extern __shared__ __align__(16) double smem64[];
+	__shared__ Shared64 sh;
+	__shared__ int s_ticket;
+	const int tid = threadIdx.x;
+	for (;;) {
+		if (tid == 0)
+			s_ticket = *((volatile int*)err) == DEV_OK ? atomicAdd(counter, 1) : tickets;
+		__syncthreads();
+		const int ticket = s_ticket;
+		if (ticket >= tickets) return;
+		int lo = 0, hi = ntasks - 1;
+		while (lo < hi) {
+			const int mid = (lo + hi + 1) / 2;
+			if (tasks[mid].ticket_base <= ticket) lo = mid; else hi = mid - 1;
+		}
+		const Task64 tk = tasks[lo];
+		const int bx = (ticket - tk.ticket_base) / tk.nc, c = (ticket - tk.ticket_base) % tk.nc;
+		const Layout64 L = layout64(TX, TU, tk.pt, tk.px, tk.py, tk.ahead);
+		double* ring = smem64;
+		double* sphi = ring + size_t(L.slot) * L.depth;
+		int2* cells = reinterpret_cast<int2*>(sphi + L.phi);
+		const int pyp = even_up(tk.py);
+		for (int q = tid; q < L.slot * L.depth; q += NTHREADS) ring[q] = 0.0;
+		for (int q = tid; q < L.phi; q += NTHREADS) {
+			const int j = q % pyp;
+			const int row = q / pyp;
+			sphi[q] = j < tk.py && row < tk.pt * tk.px ? tk.phi[row * tk.py + j] : 0.0;
+		}
+		if (tid == 0) {
+			sh.done = 0;
+			sh.published = 0;
+		}
+		__syncthreads();
+		if (tid >= NC + 32) {
+			pub_warp<TX, TU>(tk, bx, c, &sh);
+		} else if (tid >= NC) {
+			halo_warp<TX, TU>(tk, bx, c, L, ring, cells, &sh, err);
+		} else {
+			switch (tk.py) {
+#define ARMA_PY_CASE(N) case N: compute_tile<N, TX, TU>(tk, bx, c, L, ring, sphi, &sh, err); break;
+				ARMA_PY_CASE(1) ARMA_PY_CASE(2) ARMA_PY_CASE(3) ARMA_PY_CASE(4)
+				ARMA_PY_CASE(5) ARMA_PY_CASE(6) ARMA_PY_CASE(7) ARMA_PY_CASE(8)
+				ARMA_PY_CASE(9) ARMA_PY_CASE(10) ARMA_PY_CASE(11) ARMA_PY_CASE(12)
+				ARMA_PY_CASE(13) ARMA_PY_CASE(14) ARMA_PY_CASE(15) ARMA_PY_CASE(16)
+#undef ARMA_PY_CASE
+				default: break;
+			}
+		}
+		__syncthreads();
+	}
+}
+
+// One launch per hyperplane, every thread the reference's truncated sum: for
+// coefficients that are not finite, whose products with the tiles' zero padding
+// would not vanish.
+constexpr int kPlaneThreads = 128;
+__global__ void __launch_bounds__(kPlaneThreads)
 ar64_plane_kernel(double* __restrict__ zeta, const double* __restrict__ phi,
                   int nt, int nx, int ny, int pt, int px, int py, int s, int t_lo) {
 	const int t = t_lo + blockIdx.y;
 	const int rem = s - t;                 // x + y
 	const int x_lo = max(0, rem - (ny - 1));
-	const int x = x_lo + blockIdx.x * kThreads + threadIdx.x;
+	const int x = x_lo + blockIdx.x * kPlaneThreads + threadIdx.x;
 	const int x_hi = min(nx - 1, rem);
 	if (t >= nt || x > x_hi) return;
 	const int y = rem - x;
@@ -37,49 +469,116 @@ ar64_plane_kernel(double* __restrict__ zeta, const double* __restrict__ phi,
 			const double* prow = phi + (k * px + i) * py;
 			const double* zrow = zeta + (t - k) * st + (x - i) * sx + y;
 			for (int j = 0; j < m3; ++j)
-				sum = __dadd_rn(sum, __dmul_rn(__ldg(prow + j), __ldg(zrow - j)));
+				sum = __dadd_rn(sum, __dmul_rn(prow[j], zrow[-j]));
 		}
 	}
 	double* p = zeta + t * st + x * sx + y;
 	*p = __dadd_rn(*p, sum);
 }
 
+void launch_planes(Ctx* c, const Ar64Surface& s) {
+	for (int q = 0; q < s.nt + s.nx + s.ny - 2; ++q) {
+		const int t_lo = std::max(0, q - (s.nx - 1) - (s.ny - 1));
+		const int t_hi = std::min(s.nt - 1, q);
+		const int xs = std::min(s.nx, q + 1);
+		// the launch's second dimension holds at most 65535 slices
+		for (int t = t_lo; t <= t_hi; t += 65535) {
+			const dim3 grid((xs + kPlaneThreads - 1) / kPlaneThreads,
+			                std::min(t_hi - t + 1, 65535));
+			ar64_plane_kernel<<<grid, kPlaneThreads, 0, c->stream>>>(
+			    s.zeta, s.phi, s.nt, s.nx, s.ny, s.pt, s.px, s.py, q, t);
+			ARMA_CUDA_TRY(cudaGetLastError());
+			c->launches += 1;
+		}
+	}
+}
+
+// The halo steps a tile of this shape can keep ahead; 0: it does not fit.
+int ahead_of(int tx, int tu, const Ar64Surface& s) {
+	for (int a = kMaxAhead; a > 0; --a)
+		if (layout64(tx, tu, s.pt, s.px, s.py, a).bytes <= kSmemLimit) return a;
+	return 0;
+}
+
+int tiles_per_row(int tx, int tu, int ny) { return (ny + tx - 1 + tu - 1) / tu; }
+
+template <int TX, int TU>
+void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
+	// longest dependency chains first
+	auto chain = [](const Ar64Surface& s) {
+		return double(s.nt + s.nx + s.ny) * s.pt * s.px * s.py;
+	};
+	std::stable_sort(surfs.begin(), surfs.end(), [&](const Ar64Surface& a, const Ar64Surface& b) {
+		return chain(a) > chain(b);
+	});
+	std::vector<Task64> tasks;
+	long long tickets = 0;
+	size_t smem = 0;
+	for (const Ar64Surface& s : surfs) {
+		Task64 t;
+		t.nt = s.nt; t.nx = s.nx; t.ny = s.ny;
+		t.pt = s.pt; t.px = s.px; t.py = s.py;
+		t.nbx = (s.nx + TX - 1) / TX;
+		t.nc = tiles_per_row(TX, TU, s.ny);
+		t.ticket_base = int(tickets);
+		t.ahead = ahead_of(TX, TU, s);
+		t.zeta = s.zeta;
+		t.phi = s.phi;
+		t.flags = nullptr;
+		tickets += (long long)t.nbx * t.nc;
+		ARMA_REQUIRE(tickets < INT_MAX / 4, ARMA_EINVAL, "surface too large");
+		smem = std::max(smem, layout64(TX, TU, s.pt, s.px, s.py, t.ahead).bytes);
+		tasks.push_back(t);
+	}
+	// step counters of every tile, then the ticket counter
+	int* flags = static_cast<int*>(scratch_take(c, sizeof(int) * (size_t(tickets) + 1)));
+	ARMA_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t(tickets) + 1), c->stream));
+	for (Task64& t : tasks) t.flags = flags + t.ticket_base;
+	auto* d_tasks = static_cast<Task64*>(scratch_take(c, sizeof(Task64) * tasks.size()));
+	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task64) * tasks.size(),
+	                         cudaMemcpyHostToDevice, c->stream));
+	constexpr int threads = TX * TU + 64;
+	auto kernel = ar64_tile_kernel<TX, TU>;
+	ARMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                                   int(kSmemLimit)));
+	int per_sm = 0;
+	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+	ARMA_REQUIRE(per_sm > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
+	const int grid = int(std::min<long long>(tickets, (long long)per_sm * c->num_sms));
+	kernel<<<grid, threads, smem, c->stream>>>(d_tasks, int(tasks.size()), int(tickets),
+	                                           flags + tickets, c->d_err);
+	ARMA_CUDA_TRY(cudaGetLastError());
+	c->launches += 1;
+	c->check_pending = true;
+}
+
 }  // namespace
 
-void launch_ar64(Ctx* c, const double* d_phi, const int order[3],
-                 const int shape[3], double* d_zeta) {
+void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces) {
 	ProfScope prof_(c, "ar64");
-	const int nt = shape[0], nx = shape[1], ny = shape[2];
-	const int pt = order[0], px = order[1], py = order[2];
-	if ((long long)nt * nx * ny == 0) return;
-	std::ostringstream key;
-	key << "ar64:" << (const void*)d_zeta << ':' << (const void*)d_phi << ':' << nt << ','
-	    << nx << ',' << ny << ':' << pt << ',' << px << ',' << py;
-	const int nplanes = nt + nx + ny - 2;
-	auto it = c->graphs.find(key.str());
-	if (it == c->graphs.end()) {
-		cudaStream_t cap;
-		ARMA_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-		cudaGraph_t graph;
-		ARMA_CUDA_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-		for (int s = 0; s < nplanes; ++s) {
-			const int t_lo = max(0, s - (nx - 1) - (ny - 1));
-			const int t_hi = min(nt - 1, s);
-			const int nts = t_hi - t_lo + 1;
-			const int xs = min(nx, s + 1);
-			dim3 grid((xs + kThreads - 1) / kThreads, nts);
-			ar64_plane_kernel<<<grid, kThreads, 0, cap>>>(d_zeta, d_phi, nt, nx, ny, pt, px,
-			                                               py, s, t_lo);
+	// Tile shapes: 16 x 16 (eight compute warps) when the batch fills the GPU,
+	// 8 x 16 and 4 x 16 to spread a smaller one over more SMs, where fewer warps
+	// share the bandwidth of shared memory; 8 x 8 for orders whose ring does not
+	// fit otherwise.
+	std::vector<Ar64Surface> groups[4];
+	long long t8 = 0, t4 = 0;
+	for (const Ar64Surface& s : surfaces)
+		if (s.finite) {
+			t8 += (long long)((s.nx + 7) / 8) * tiles_per_row(8, 16, s.ny);
+			t4 += (long long)((s.nx + 3) / 4) * tiles_per_row(4, 16, s.ny);
 		}
-		ARMA_CUDA_TRY(cudaStreamEndCapture(cap, &graph));
-		cudaGraphExec_t exec;
-		ARMA_CUDA_TRY(cudaGraphInstantiate(&exec, graph, 0));
-		ARMA_CUDA_TRY(cudaGraphDestroy(graph));
-		ARMA_CUDA_TRY(cudaStreamDestroy(cap));
-		it = c->graphs.emplace(key.str(), exec).first;
+	const int want = t4 <= c->num_sms ? 2 : t8 <= c->num_sms ? 1 : 0;
+	for (const Ar64Surface& s : surfaces) {
+		if (!s.finite) launch_planes(c, s);
+		else if (want == 0 && ahead_of(16, 16, s)) groups[0].push_back(s);
+		else if (want <= 1 && ahead_of(8, 16, s)) groups[1].push_back(s);
+		else if (ahead_of(4, 16, s)) groups[2].push_back(s);
+		else groups[3].push_back(s);
 	}
-	ARMA_CUDA_TRY(cudaGraphLaunch(it->second, c->stream));
-	c->launches += uint64_t(nplanes);
+	if (!groups[0].empty()) launch_tiles<16, 16>(c, groups[0]);
+	if (!groups[1].empty()) launch_tiles<8, 16>(c, groups[1]);
+	if (!groups[2].empty()) launch_tiles<4, 16>(c, groups[2]);
+	if (!groups[3].empty()) launch_tiles<8, 8>(c, groups[3]);
 }
 
 }  // namespace armab

@@ -278,6 +278,7 @@ void resolve_profile(Ctx* c) {
 
 void check_device_error(Ctx* c) {
 	int h = 0;
+	c->check_pending = false;
 	ARMA_CUDA_TRY(copy_async(c, &h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 	ARMA_CUDA_TRY(cudaStreamSynchronize(c->stream));
 	if (h == DEV_TIMEOUT) {
@@ -333,7 +334,6 @@ int arma_ctx_destroy(arma_ctx* ctx) {
 			cudaEventDestroy(p.start);
 			cudaEventDestroy(p.stop);
 		}
-		for (auto& kv : ctx->c.graphs) cudaGraphExecDestroy(kv.second);
 		for (auto& kv : ctx->c.nit_tables) cudaFree(kv.second);
 		for (auto& ch : ctx->chunks) pool_free(&ctx->c, ch.first);
 		cudaStreamSynchronize(ctx->c.stream);
@@ -367,6 +367,7 @@ int arma_ctx_synchronize(arma_ctx* ctx) {
 	return guard([&] {
 		ARMA_REQUIRE(ctx, ARMA_EINVAL, "null context");
 		ARMA_CUDA_TRY(cudaSetDevice(ctx->c.device));
+		if (ctx->c.check_pending) check_device_error(&ctx->c);
 		ARMA_CUDA_TRY(cudaStreamSynchronize(ctx->c.stream));
 	});
 }
@@ -750,14 +751,33 @@ std::vector<Ar32Surface> ar32_surfaces(Ctx* c, int n, const double* const* phis,
 	return out;
 }
 
+// The FP64 filter of n surfaces in one launch, their coefficients in one
+// upload (a copy from pageable memory has been staged when it returns).
+void ar64_surfaces(Ctx* c, int n, const double* const* phis, const int* const* orders,
+                   const int* const* shapes, double* const* zetas) {
+	std::vector<size_t> off(n + 1, 0);
+	for (int k = 0; k < n; ++k)
+		off[k + 1] = off[k] + size_t(orders[k][0]) * orders[k][1] * orders[k][2];
+	std::vector<double> buf(off[n]);
+	double* d = static_cast<double*>(scratch_take(c, sizeof(double) * buf.size()));
+	std::vector<Ar64Surface> s(n);
+	for (int k = 0; k < n; ++k) {
+		std::copy(phis[k], phis[k] + (off[k + 1] - off[k]), buf.begin() + off[k]);
+		const bool finite = std::all_of(phis[k], phis[k] + (off[k + 1] - off[k]),
+		                                [](double v) { return std::isfinite(v); });
+		s[k] = Ar64Surface{shapes[k][0], shapes[k][1], shapes[k][2], orders[k][0], orders[k][1],
+		                   orders[k][2], zetas[k],     d + off[k],   finite};
+	}
+	ARMA_CUDA_TRY(copy_async(c, d, buf.data(), sizeof(double) * buf.size(),
+	                         cudaMemcpyHostToDevice, c->stream));
+	launch_ar64(c, s);
+}
+
 void ar_filter(Ctx* c, const double* phi, const int order[3], const int shape[3],
                int precision, void* d_zeta) {
-	const int P = order[0] * order[1] * order[2];
 	if (precision == ARMA_FP64) {
-		double* d_phi = static_cast<double*>(scratch_take(c, sizeof(double) * P));
-		ARMA_CUDA_TRY(copy_async(c, d_phi, phi, sizeof(double) * P, cudaMemcpyHostToDevice,
-		                              c->stream));
-		launch_ar64(c, d_phi, order, shape, static_cast<double*>(d_zeta));
+		double* z = static_cast<double*>(d_zeta);
+		ar64_surfaces(c, 1, &phi, &order, &shape, &z);
 	} else {
 		const int tx = ar32c_tile_x(), ty = ar32c_tile_y();
 		float* z = static_cast<float*>(d_zeta);
@@ -975,8 +995,18 @@ void batch(Ctx* c, arma_surface* s, int n, int precision, bool host, bool redo =
 	}
 	if (precision == ARMA_FP64) {
 		white_noise_batch(c, s, n, precision, dz);
-		for (int k = 0; k < n; ++k) ar_filter(c, s[k].phi, s[k].order, s[k].shape, precision, dz[k]);
+		std::vector<const double*> phis(n);
+		std::vector<const int*> ords(n), shps(n);
+		std::vector<double*> zs(n);
+		for (int k = 0; k < n; ++k) {
+			phis[k] = s[k].phi;
+			ords[k] = s[k].order;
+			shps[k] = s[k].shape;
+			zs[k] = static_cast<double*>(dz[k]);
+		}
+		ar64_surfaces(c, n, phis.data(), ords.data(), shps.data(), zs.data());
 		renorm_surfaces(c, s, n, precision, dz, host, luts);
+		check_device_error(c);
 		return;
 	}
 	long long* d_pairs = nullptr;

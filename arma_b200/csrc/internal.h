@@ -58,8 +58,8 @@ struct Ctx {
 	uint64_t h2d_bytes = 0;          // bytes copied host -> device through copy_async
 	uint64_t d2h_bytes = 0;          // bytes copied device -> host through copy_async
 	int num_sms = 148;
-	// cached CUDA graphs for the FP64 plane sweep, keyed by a string
-	std::map<std::string, cudaGraphExec_t> graphs;
+	// a launch whose bounded waits nothing has checked yet (check_device_error)
+	bool check_pending = false;
 	// NIT inverse-CDF tables by specification (double table, then float table)
 	std::map<std::vector<double>, double*> nit_tables;
 	// optional per-kernel-class timing with CUDA events on `stream`
@@ -211,9 +211,17 @@ struct NoiseSpec {
 void enqueue_white_noise_batch(Ctx* c, const std::vector<NoiseSpec>& specs, int precision,
                                long long* d_pairs);
 
-// FP64 exact-order AR filter.
-void launch_ar64(Ctx* c, const double* d_phi, const int order[3],
-                 const int shape[3], double* d_zeta);
+// FP64 exact-order AR filter of a batch of surfaces, in place (ar64.cu).
+// Asynchronous; the error word of its bounded waits is left for the next
+// check_device_error.
+struct Ar64Surface {
+	int nt, nx, ny;
+	int pt, px, py;
+	double* zeta;       // device, noise in, surface out
+	const double* phi;  // device, pt*px*py
+	bool finite;        // every coefficient is finite
+};
+void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces);
 
 // FP32 compensated AR filter for a batch of surfaces (ar32c.cu).
 struct Ar32Surface {
