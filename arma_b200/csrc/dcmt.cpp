@@ -301,59 +301,78 @@ bool passes_screen(const Screen& sc, uint32_t r15) {
 	return true;
 }
 
-// ------------------------------------------------------------ full primitivity test
-// t^(2^p) == t mod chi, by p squarings with Barrett reduction.
-bool frobenius_fixes_t(const std::vector<Word>& chi_in, int p) {
-	const size_t n = size_t(p) / 64 + 1;  // words holding degree <= p
-	std::vector<Word> chi(n + 1, 0);
-	std::copy(chi_in.begin(), chi_in.begin() + std::min(chi_in.size(), n + 1), chi.begin());
-	// mu = floor(t^(2p) / chi) by long division (degree p)
-	std::vector<Word> rem(2 * n + 2, 0), mu(n + 1, 0);
-	flip(rem.data(), 2L * p);
-	for (long d = 2L * p; d >= p; --d) {
-		if (!bit_of(rem.data(), d)) continue;
-		const long sh = d - p;
-		flip(mu.data(), sh);
-		const size_t ws = size_t(sh) >> 6;
-		const int bs = int(sh & 63);
-		for (size_t i = 0; i <= n; ++i) {
-			rem[ws + i] ^= chi[i] << bs;
-			if (bs && ws + i + 1 < rem.size()) rem[ws + i + 1] ^= chi[i] >> (64 - bs);
+// ------------------------------------------------------------ squarings mod chi
+// a -> a^2 mod chi for polynomials of degree < p, by Barrett reduction
+// (Karatsuba products); about 65 us at p = 19937.
+class Squarer {
+public:
+	Squarer(const std::vector<Word>& chi_in, int p) : p_(p), n_(size_t(p) / 64 + 1) {
+		const size_t n = n_, m = n + 1;  // words holding degree <= p; operand length
+		chi_.assign(m, 0);
+		std::copy(chi_in.begin(), chi_in.begin() + std::min(chi_in.size(), m), chi_.begin());
+		// mu = floor(t^(2p) / chi) by long division (degree p)
+		std::vector<Word> rem(2 * n + 2, 0);
+		mu_.assign(m, 0);
+		flip(rem.data(), 2L * p);
+		for (long d = 2L * p; d >= p; --d) {
+			if (!bit_of(rem.data(), d)) continue;
+			const long sh = d - p;
+			flip(mu_.data(), sh);
+			const size_t ws = size_t(sh) >> 6;
+			const int bs = int(sh & 63);
+			for (size_t i = 0; i <= n; ++i) {
+				rem[ws + i] ^= chi_[i] << bs;
+				if (bs && ws + i + 1 < rem.size()) rem[ws + i + 1] ^= chi_[i] >> (64 - bs);
+			}
 		}
+		sq_.assign(2 * m, 0);
+		hi_.assign(m, 0);
+		qv_.assign(2 * m, 0);
+		qq_.assign(m, 0);
+		qc_.assign(2 * m, 0);
+		scratch_.assign(16 * m + 64, 0);
 	}
-	const size_t m = n + 1;  // operand length for the products
-	std::vector<Word> a(m, 0), sq(2 * m, 0), hi(m, 0), qv(2 * m, 0), qq(m, 0), qc(2 * m, 0);
-	std::vector<Word> scratch(16 * m + 64);
-	std::vector<Word> chim(m, 0), mum(m, 0);
-	std::copy(chi.begin(), chi.begin() + std::min(chi.size(), m), chim.begin());
-	std::copy(mu.begin(), mu.end(), mum.begin());
-	a[0] = 2;  // t
-	for (int it = 0; it < p; ++it) {
+	size_t words() const { return n_; }  // of an operand
+	void square(Word* a) {
+		const size_t m = n_ + 1;
 		// sq = a^2 (degree <= 2p - 2)
-		std::fill(sq.begin(), sq.end(), 0);
-		for (size_t i = 0; i < n; ++i) {
+		std::fill(sq_.begin(), sq_.end(), 0);
+		for (size_t i = 0; i < n_; ++i) {
 			Word lo, h2;
 			if (kHavePclmul)
 				clmul_hw(a[i], a[i], lo, h2);
 			else
 				clmul_sw(a[i], a[i], lo, h2);
-			sq[2 * i] = lo;
-			sq[2 * i + 1] = h2;
+			sq_[2 * i] = lo;
+			sq_[2 * i + 1] = h2;
 		}
 		// q = ((sq >> p) * mu) >> p
-		shift_right(sq.data(), sq.size(), p, hi.data(), m);
-		mul_kara(hi.data(), mum.data(), m, qv.data(), scratch.data());
-		shift_right(qv.data(), qv.size(), p, qq.data(), m);
+		shift_right(sq_.data(), sq_.size(), p_, hi_.data(), m);
+		mul_kara(hi_.data(), mu_.data(), m, qv_.data(), scratch_.data());
+		shift_right(qv_.data(), qv_.size(), p_, qq_.data(), m);
 		// r = (sq + q chi) mod t^p
-		mul_kara(qq.data(), chim.data(), m, qc.data(), scratch.data());
-		for (size_t i = 0; i < n; ++i) a[i] = sq[i] ^ qc[i];
-		const int top = p & 63;
-		a[n - 1] &= top ? (Word(1) << top) - 1 : ~Word(0);
-		if (size_t(p) % 64 == 0) a[n - 1] = 0;
-		for (size_t i = n; i < m; ++i) a[i] = 0;
+		mul_kara(qq_.data(), chi_.data(), m, qc_.data(), scratch_.data());
+		for (size_t i = 0; i < n_; ++i) a[i] = sq_[i] ^ qc_[i];
+		const int top = p_ & 63;
+		a[n_ - 1] &= top ? (Word(1) << top) - 1 : ~Word(0);
+		if (size_t(p_) % 64 == 0) a[n_ - 1] = 0;
 	}
+
+private:
+	int p_;
+	size_t n_;
+	std::vector<Word> chi_, mu_, sq_, hi_, qv_, qq_, qc_, scratch_;
+};
+
+// ------------------------------------------------------------ full primitivity test
+// t^(2^p) == t mod chi, by p squarings.
+bool frobenius_fixes_t(const std::vector<Word>& chi, int p) {
+	Squarer sq(chi, p);
+	std::vector<Word> a(sq.words(), 0);
+	a[0] = 2;  // t
+	for (int it = 0; it < p; ++it) sq.square(a.data());
 	if (a[0] != 2) return false;
-	for (size_t i = 1; i < n; ++i)
+	for (size_t i = 1; i < a.size(); ++i)
 		if (a[i]) return false;
 	return true;
 }
@@ -555,6 +574,27 @@ bool is_primitive(const arma_mt_params& prm) {
 	for (Word w : chi) ones ^= __builtin_parityll(w);
 	if (!ones) return false;
 	return frobenius_fixes_t(chi, s.p);
+}
+
+std::vector<uint64_t> characteristic_polynomial(const arma_mt_params& prm) {
+	const int p = 32 * prm.nn - prm.rr;
+	if (prm.rr < 0 || prm.rr > 31 || prm.mm < 1 || prm.mm >= prm.nn) return {};
+	if (prm.wmask != 0xffffffffu || prm.umask != 0xffffffffu << prm.rr || prm.lmask != ~prm.umask)
+		return {};
+	std::vector<Word> chi = char_poly(Shape{p, prm.nn, prm.mm, prm.rr}, prm.aaa);
+	chi.resize(size_t(p) / 64 + 1);
+	return chi;
+}
+
+void square_powers_of_t(const std::vector<uint64_t>& chi, int p, int from, int upto,
+                        std::vector<std::vector<uint64_t>>* g) {
+	Squarer sq(chi, p);
+	for (int e = from; e <= upto; ++e) {
+		std::vector<Word> a = g->back();
+		a.resize(sq.words());
+		sq.square(a.data());
+		g->push_back(std::move(a));
+	}
 }
 
 long equidistribution(const arma_mt_params& prm, int v) {

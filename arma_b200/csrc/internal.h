@@ -158,20 +158,22 @@ struct MtJob {
 	unsigned long long offset, count;
 	uint32_t* out;
 	const uint32_t* state = nullptr;
-	// the windows at every segment start (launch_mt_prepare with the same
-	// segment length), or null: jump ahead here
+	// the windows at every segment start, 2^seg_log2 words apart (set by
+	// launch_mt_prepare), or null: jump ahead here
 	const uint32_t* seg_states = nullptr;
+	int seg_log2 = 0;
 };
 void launch_mt_generate(Ctx* c, const arma_mt_params& p, uint32_t seed,
                         uint64_t offset, uint64_t n, uint32_t* d_out);
 // Every job's stream in a few launches: streams longer than one segment of
-// 2^log2_seg words are split by jump-ahead into one CTA per segment.
+// 2^log2_seg words are split by jump-ahead into segments of at most that
+// length, shorter when they are few.
 constexpr int kMtLog2Seg = 20;
 void launch_mt_generate_batch(Ctx* c, const std::vector<MtJob>& jobs,
                               int log2_seg = kMtLog2Seg);
 // Only the jump-ahead windows of the jobs longer than one segment, into
 // jobs[q].seg_states (scratch), for later launch_mt_generate_batch calls on
-// subsets of the jobs with the same segment length.
+// subsets of the jobs.
 void launch_mt_prepare(Ctx* c, std::vector<MtJob>& jobs, int log2_seg = kMtLog2Seg);
 // After a chunk consumed 4 * *attempts words of `words` (n_words long): the
 // raw window in front of the next word (untempered copies of the nn words
@@ -409,6 +411,13 @@ namespace dcmt {
 bool mersenne_exponent(int p);
 bool is_primitive(const arma_mt_params& prm);
 long equidistribution(const arma_mt_params& prm, int v);  // k(v), -1 if undetermined
+// The closed form of the recurrence's characteristic polynomial (bit i of word i
+// / 64 = coefficient of t^i, degree p = 32 nn - rr); empty for masks that are
+// not a w = 32 set's.
+std::vector<uint64_t> characteristic_polynomial(const arma_mt_params& prm);
+// Appends t^(2^e) mod chi for e = from .. upto to g, whose last entry is t^(2^(from - 1)).
+void square_powers_of_t(const std::vector<uint64_t>& chi, int p, int from, int upto,
+                        std::vector<std::vector<uint64_t>>* g);
 int create(int p, int id, uint32_t seed, arma_mt_params* out);  // 0, or -1: no primitive set
 }  // namespace dcmt
 

@@ -11,12 +11,12 @@
 // arithmetic in 32-bit integers; sets with nn = 2 mm run one warp per segment
 // with no barrier (mt_generate_half_kernel).
 //
-// Long streams are cut into segments of J = 2^20 words generated by separate
-// CTAs.  The window of nn raw words at the start of segment k is obtained by
-// jumping: with g(t) = t^(J 2^l) mod phi(t) (phi the characteristic
-// polynomial, mt_jump.cc), the window D positions ahead is the XOR of the
-// windows of the raw sequence at the set bits of g.  Segment starts are built
-// as a binary tree: level l turns every known start k*2^(l+1) into
+// Long streams are cut into segments of J = 2^v words (segment_log2) generated
+// by separate CTAs or warps.  The window of nn raw words at the start of segment
+// k is obtained by jumping: with g(t) = t^(J 2^l) mod phi(t) (phi the
+// characteristic polynomial, mt_jump.cc), the window D positions ahead is the
+// XOR of the windows of the raw sequence at the set bits of g.  Segment starts
+// are built as a binary tree: level l turns every known start k*2^(l+1) into
 // k*2^(l+1) + 2^l.  All of it is bit-identical to the sequential generator.
 #include <algorithm>
 #include <cstring>
@@ -28,16 +28,19 @@
 
 namespace armab {
 
-// Defined in mt_jump.cc.
-bool mt_jump_tables(const arma_mt_params& prm, int log2_jump, int levels,
-                    std::vector<std::vector<int32_t>>* set_bits, int* degree);
+// Defined in mt_jump.cc: the coefficients of t^(2^e) mod phi, bit i of word i /
+// 32; false when the set has not full period.
+bool mt_jump_bits(const arma_mt_params& prm, int e, std::vector<uint32_t>* bits);
 
 namespace {
 
 constexpr int kRingBits = 12;
 constexpr int kRing = 1 << kRingBits;  // ring of raw words, >= nn + (nn-mm)
-constexpr int kLevels = 16;            // jump tables for J * 2^l, l < 16
-constexpr int kJumpThreads = 640;
+constexpr int kLevels = 16;            // at most 2^16 segments
+constexpr int kMinLog2Seg = 16;        // shortest segment of the rule below
+// more segments per SM than this are generated by a warp each
+constexpr size_t kWarpSegments = 6;
+constexpr int kJumpThreads = 384;
 
 struct SegJob {
 	arma_mt_params p;
@@ -52,9 +55,8 @@ struct SegJob {
 struct JumpJob {
 	arma_mt_params p;
 	const uint32_t* src;  // window at position a
-	uint32_t* dst;        // window at position a + D
-	const int32_t* bits;  // set bits of t^D mod phi
-	int nbits;
+	uint32_t* dst;        // window at position a + D (zero when parts > 1)
+	const uint32_t* bits; // t^D mod phi, bit i of word i / 32
 };
 
 __device__ __forceinline__ uint32_t temper(uint32_t y, const arma_mt_params& p) {
@@ -239,6 +241,87 @@ mt_generate_half_kernel(const SegJob* __restrict__ jobs, int njobs) {
 	}
 }
 
+// The same sets with one CTA per segment, a thread per slot, for few segments.
+// Words are a CTA's time here, not the GPU's, so a barrier is paid once per four
+// steps: from the window of the last two steps (x[0 .. 2 mm)) thread t computes
+// its own slot's next four words C, D, E, F, and its right neighbour's C and D,
+// which E and F need, once more from the window.  The neighbours of the last two
+// slots are the first words of the next step (x[2 mm], x[2 mm + 1]).
+// A set's recurrence and tempering constants held in registers (opaque to the
+// compiler, which otherwise loads them again in every step).
+__device__ __forceinline__ arma_mt_params in_registers(arma_mt_params p) {
+	asm volatile("" : "+r"(p.aaa), "+r"(p.umask), "+r"(p.lmask), "+r"(p.maskB), "+r"(p.maskC));
+	asm volatile("" : "+r"(p.shift0), "+r"(p.shift1), "+r"(p.shiftB), "+r"(p.shiftC));
+	asm volatile("" : "+r"(p.nn), "+r"(p.mm), "+r"(p.rr));
+	return p;
+}
+
+__device__ __forceinline__ uint32_t twist(uint32_t u, uint32_t v, const arma_mt_params& p) {
+	const uint32_t y = (u & p.umask) | (v & p.lmask);
+	return (y >> 1) ^ ((y & 1u) ? p.aaa : 0u);
+}
+
+__device__ __forceinline__ void half_four(const uint32_t* x, int t, int mm,
+                                          const arma_mt_params& p, uint32_t (&w)[4]) {
+	const uint32_t a0 = x[t], a1 = x[t + 1], a2 = x[t + 2], b0 = x[mm + t];
+	uint32_t b1, b2;
+	if (t + 2 < mm) {
+		b1 = x[mm + t + 1];
+		b2 = x[mm + t + 2];
+	} else {
+		const uint32_t n0 = x[mm] ^ twist(x[0], x[1], p), n1 = x[mm + 1] ^ twist(x[1], x[2], p);
+		b1 = t + 1 < mm ? x[mm + t + 1] : n0;
+		b2 = t + 1 < mm ? n0 : n1;
+	}
+	w[0] = b0 ^ twist(a0, a1, p);
+	const uint32_t c1 = b1 ^ twist(a1, a2, p);
+	w[1] = w[0] ^ twist(b0, b1, p);
+	const uint32_t d1 = c1 ^ twist(b1, b2, p);
+	w[2] = w[1] ^ twist(w[0], c1, p);
+	w[3] = w[2] ^ twist(w[1], d1, p);
+}
+
+constexpr int kFourThreads = 32 * kHalfQ;
+
+__global__ void __launch_bounds__(kFourThreads)
+mt_generate_four_kernel(const SegJob* __restrict__ jobs) {
+	__shared__ uint32_t win[2][kHalfMaxN + 2];  // (the last two slots read past their step)
+	const SegJob& jb = jobs[blockIdx.x];
+	const arma_mt_params p = in_registers(jb.p);
+	const int mm = p.mm, t = threadIdx.x;
+	if (jb.state) {
+		for (int k = t; k < p.nn; k += kFourThreads) win[0][k] = jb.state[k];
+	} else if (t == 0) {
+		seed_state(win[0], jb.seed, p);
+	}
+	__syncthreads();
+	// segment word w < count (<= 2^30) goes to out[first - offset + w] when that
+	// index is >= 0
+	const int count = int(jb.count);
+	const long long shift = (long long)jb.first - (long long)jb.offset;
+	const int wmin = shift < 0 ? int(-shift) : 0;
+	uint32_t* const base = jb.out + (shift > 0 ? shift : 0) - wmin;
+	int b = 0;
+	for (int w0 = 0; w0 < count; w0 += 4 * mm, b ^= 1) {
+		if (t < mm) {
+			uint32_t w[4];
+			half_four(win[b], t, mm, p, w);
+			win[b ^ 1][t] = w[2];
+			win[b ^ 1][mm + t] = w[3];
+			if (w0 >= wmin && w0 + 4 * mm <= count) {
+#pragma unroll
+				for (int q = 0; q < 4; ++q) base[w0 + q * mm + t] = temper(w[q], p);
+			} else {
+				for (int q = 0; q < 4; ++q) {
+					const int k = w0 + q * mm + t;
+					if (k >= wmin && k < count) base[k] = temper(w[q], p);
+				}
+			}
+		}
+		__syncthreads();
+	}
+}
+
 // Window of segment 0 of each jumped job: the seeded state, or a copy of the
 // job's own window.
 __global__ void mt_seed_kernel(const arma_mt_params* __restrict__ ps,
@@ -294,60 +377,100 @@ __global__ void mt_window_kernel(const WindowJob* __restrict__ jobs) {
 	if (threadIdx.x == 0 && jb.position) *jb.position += used;
 }
 
-// `parts` CTAs per jump: each computes the raw words y[0 .. p+n-2] from the
-// source window in shared memory, then its share of the destination window,
-// dst[w] = XOR over the set bits i of y[i + w], with the bit list split among
-// several threads per word and the partial XORs combined in shared memory.
-// More parts shorten a jump when few jumps run at once.
+// The window D ahead of a jump's source: dst[w] = XOR over the set bits i of
+// t^D mod phi of y[i + w], y the raw sequence from the source window on.
+// `parts` CTAs share a jump (more when few jumps run at once), each a range of
+// the bits; its warps share that range again.  A CTA computes the raw words it
+// needs into shared memory.  A lane owns kJumpWords consecutive words of the
+// window, so that a set bit costs a warp kJumpWords XORs in registers and the
+// words that 16 bits touch are read once for all of them (a lane's stride is
+// odd: no bank conflicts); two neighbouring set bits go in one three-input XOR.
+// At p = 19937: 10 us alone in 32 parts, 1.1 ms for the 2700 jumps of the batch
+// of 256 surfaces (one word per thread and a shared-memory read per set bit: 45
+// us alone, 4.3 ms).
+constexpr int kJumpWords = 21;                // 32 * 21 = 672 >= 624 words
+constexpr int kJumpSpan = 32 * kJumpWords;    // words of the window per pass
+constexpr int kJumpBits = 16;                 // bits whose words are read together
+
+__host__ __device__ inline int jump_degree(const arma_mt_params& p) { return 32 * p.nn - p.rr; }
+// raw words a jump can read: bits up to the degree, rounded up to whole groups,
+// plus the window's passes
+__host__ __device__ inline int jump_words(const arma_mt_params& p) {
+	const int passes = (p.nn + kJumpSpan - 1) / kJumpSpan;
+	return (jump_degree(p) + kJumpBits) / kJumpBits * kJumpBits + passes * kJumpSpan + kJumpBits;
+}
+
 __global__ void __launch_bounds__(kJumpThreads)
 mt_jump_kernel(const JumpJob* __restrict__ jobs, int parts) {
 	extern __shared__ uint32_t y[];
 	const JumpJob& jb = jobs[blockIdx.x / parts];
-	const arma_mt_params p = jb.p;
+	const arma_mt_params p = in_registers(jb.p);
 	const int n = p.nn, m = p.mm, chunk = n - m;
-	const int per = (n + parts - 1) / parts;
-	const int w0 = (blockIdx.x % parts) * per;
-	if (w0 >= n) return;  // uniform over the CTA
-	const int cnt = min(n, w0 + per) - w0;
-	const int deg = 32 * n - p.rr;
-	const int len = deg + n - 1;
+	const int groups = (jump_degree(p) + kJumpBits - 1) / kJumpBits;
+	const int per = (groups + parts - 1) / parts;
+	const int g0 = min(groups, int(blockIdx.x % parts) * per), g1 = min(groups, g0 + per);
+	if (g0 >= g1) return;  // uniform over the CTA
+	const int len = min(jump_words(p), g1 * kJumpBits + (n + kJumpSpan - 1) / kJumpSpan * kJumpSpan);
 	for (int k = threadIdx.x; k < n; k += blockDim.x) y[k] = jb.src[k];
 	__syncthreads();
-	for (int j0 = n; j0 < len; j0 += chunk) {
-		for (int t = threadIdx.x; t < chunk; t += blockDim.x) {
-			const int j = j0 + t;
-			if (j < len) {
-				const uint32_t v = (y[j - n] & p.umask) | (y[j - n + 1] & p.lmask);
-				y[j] = y[j - n + m] ^ (v >> 1) ^ ((v & 1u) ? p.aaa : 0u);
+	if (half_set(p)) {
+		for (int j0 = 0; j0 + n < len; j0 += 4 * m) {
+			const int t = threadIdx.x;
+			if (t < m) {
+				uint32_t w[4];
+				half_four(y + j0, t, m, p, w);
+#pragma unroll
+				for (int q = 0; q < 4; ++q)
+					if (j0 + n + q * m + t < len) y[j0 + n + q * m + t] = w[q];
+			}
+			__syncthreads();
+		}
+	} else {
+		for (int j0 = n; j0 < len; j0 += chunk) {
+			for (int t = threadIdx.x; t < chunk; t += blockDim.x)
+				if (j0 + t < len) y[j0 + t] = y[j0 + t - chunk] ^ twist(y[j0 + t - n], y[j0 + t - n + 1], p);
+			__syncthreads();
+		}
+	}
+	__shared__ uint32_t sum[kJumpSpan];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	constexpr int kWarps = kJumpThreads / 32;
+	const auto* pattern = reinterpret_cast<const uint16_t*>(jb.bits);  // little endian
+	for (int w0 = 0; w0 < n; w0 += kJumpSpan) {
+		for (int k = threadIdx.x; k < kJumpSpan; k += blockDim.x) sum[k] = 0u;
+		__syncthreads();
+		uint32_t acc[kJumpWords];
+#pragma unroll
+		for (int r = 0; r < kJumpWords; ++r) acc[r] = 0u;
+		for (int g = g0 + warp; g < g1; g += kWarps) {
+			const uint32_t pat = __shfl_sync(0xffffffffu, uint32_t(pattern[g]), 0);
+			const uint32_t* src = y + g * kJumpBits + w0 + lane * kJumpWords;
+			uint32_t v[kJumpWords + kJumpBits - 1];
+#pragma unroll
+			for (int r = 0; r < kJumpWords + kJumpBits - 1; ++r) v[r] = src[r];
+#pragma unroll
+			for (int k = 0; k < kJumpBits; k += 2) {
+				const uint32_t two = (pat >> k) & 3u;
+				if (two == 3u) {
+#pragma unroll
+					for (int r = 0; r < kJumpWords; ++r) acc[r] ^= v[k + r] ^ v[k + 1 + r];
+				} else if (two == 1u) {
+#pragma unroll
+					for (int r = 0; r < kJumpWords; ++r) acc[r] ^= v[k + r];
+				} else if (two == 2u) {
+#pragma unroll
+					for (int r = 0; r < kJumpWords; ++r) acc[r] ^= v[k + 1 + r];
+				}
 			}
 		}
+#pragma unroll
+		for (int r = 0; r < kJumpWords; ++r) atomicXor(&sum[lane * kJumpWords + r], acc[r]);
 		__syncthreads();
-	}
-	uint32_t* acc = y + len;  // lanes * cnt <= blockDim.x partial XORs
-	const int lanes = max(1, int(blockDim.x) / cnt);
-	const int wl = threadIdx.x % cnt, lane = threadIdx.x / cnt;
-	if (lane < lanes) {
-		const int nb = jb.nbits;
-		const int span = ((nb + lanes - 1) / lanes + 3) & ~3;  // multiple of 4: aligned int4 loads
-		const int b0 = min(nb, lane * span), b1 = min(nb, b0 + span);
-		const int w = w0 + wl;
-		uint32_t r0 = 0, r1 = 0, r2 = 0, r3 = 0;
-		int it = b0;
-		for (; it + 4 <= b1; it += 4) {
-			const int4 b = *reinterpret_cast<const int4*>(jb.bits + it);
-			r0 ^= y[b.x + w];
-			r1 ^= y[b.y + w];
-			r2 ^= y[b.z + w];
-			r3 ^= y[b.w + w];
+		for (int k = threadIdx.x; k < kJumpSpan && w0 + k < n; k += blockDim.x) {
+			if (parts > 1) atomicXor(&jb.dst[w0 + k], sum[k]);
+			else jb.dst[w0 + k] = sum[k];
 		}
-		for (; it < b1; ++it) r0 ^= y[jb.bits[it] + w];
-		acc[lane * cnt + wl] = r0 ^ r1 ^ r2 ^ r3;
-	}
-	__syncthreads();
-	for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-		uint32_t r = 0;
-		for (int l = 0; l < lanes; ++l) r ^= acc[l * cnt + t];
-		jb.dst[w0 + t] = r;
+		__syncthreads();
 	}
 }
 
@@ -358,40 +481,53 @@ std::vector<uint32_t> params_key(const arma_mt_params& p) {
 	return k;
 }
 
-// Jump tables are cached per (device, parameter set, segment length) for the
-// life of the process; every context on the device shares them.
-struct MtTable {
-	bool ok = false;
-	std::vector<int32_t*> bits;  // device arrays, one per level
-	std::vector<int> nbits;
-};
+// Jump tables on the device are cached per (device, parameter set, exponent)
+// for the life of the process; every context on the device shares them.
 std::mutex g_table_mutex;
-std::map<std::vector<uint32_t>, MtTable> g_tables;
+std::map<std::vector<uint32_t>, uint32_t*> g_tables;
 
-const MtTable& jump_table(Ctx* c, const arma_mt_params& p, int log2_seg) {
+// The device's t^(2^e) mod phi of a set, or null when it has not full period.
+const uint32_t* jump_table(Ctx* c, const arma_mt_params& p, int e) {
 	auto key = params_key(p);
 	key.push_back(uint32_t(c->device));
-	key.push_back(uint32_t(log2_seg));
+	key.push_back(uint32_t(e));
 	std::lock_guard<std::mutex> lock(g_table_mutex);
 	auto it = g_tables.find(key);
 	if (it != g_tables.end()) return it->second;
-	MtTable t;
-	std::vector<std::vector<int32_t>> bits;
-	int deg = 0;
-	t.ok = mt_jump_tables(p, log2_seg, kLevels, &bits, &deg);
-	if (t.ok) {
-		for (auto& b : bits) {
-			// pad to a multiple of 4 for vector loads (pads are never read)
-			std::vector<int32_t> v = b;
-			while (v.size() % 4) v.push_back(0);
-			int32_t* d = nullptr;
-			ARMA_CUDA_TRY(cudaMalloc(&d, sizeof(int32_t) * std::max<size_t>(v.size(), 4)));
-			ARMA_CUDA_TRY(cudaMemcpy(d, v.data(), sizeof(int32_t) * v.size(), cudaMemcpyHostToDevice));
-			t.bits.push_back(d);
-			t.nbits.push_back(int(b.size()));
-		}
+	std::vector<uint32_t> bits;
+	uint32_t* d = nullptr;
+	if (mt_jump_bits(p, e, &bits)) {
+		ARMA_CUDA_TRY(cudaMalloc(&d, sizeof(uint32_t) * bits.size()));
+		ARMA_CUDA_TRY(cudaMemcpy(d, bits.data(), sizeof(uint32_t) * bits.size(),
+		                         cudaMemcpyHostToDevice));
 	}
-	return g_tables.emplace(key, std::move(t)).first->second;
+	return g_tables.emplace(key, d).first->second;
+}
+
+// Streams up to this length stay one segment: 85 us for its one CTA.
+constexpr unsigned long long kWhole = 1ull << 18;
+
+// Segments of a stream cut at 2^v words, v <= log2_seg.
+unsigned long long segments_of(unsigned long long total, int v, int log2_seg) {
+	if (total <= std::min(kWhole, 1ull << log2_seg)) return 1;
+	return (total + (1ull << v) - 1) >> v;
+}
+
+// The segment length of a call, 2^v words with v at most the caller's: the
+// shortest that still gives no more than four segments per SM.  Generating a
+// segment takes one CTA 0.41 us per 1248 words and another level of the jump
+// tree 10 us, so a single stream is cut short (16.7 M words in 256 segments: 260
+// us; 16 segments of 2^20, a warp each: 1130 us), while the jumps of a large
+// batch keep its segments long (2.7 G words, 2700 segments of 2^20).
+int segment_log2(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg) {
+	auto count = [&](int v) {
+		unsigned long long n = 0;
+		for (const MtJob& j : jobs) n += segments_of(j.offset + j.count, v, log2_seg);
+		return n;
+	};
+	int v = log2_seg;
+	while (v > kMinLog2Seg && count(v - 1) <= 4ull * c->num_sms) --v;
+	return v;
 }
 
 }  // namespace
@@ -414,33 +550,34 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 		             ARMA_EINVAL, "MT state too large for the device generator");
 	}
 	if (jobs.empty()) return;
-	const unsigned long long J = 1ull << log2_seg;
-	// segments per job; jobs with more than one segment need jump tables
-	std::vector<int> K(jobs.size());
-	std::vector<const MtTable*> tab(jobs.size(), nullptr);
+	const int v_call = segment_log2(c, jobs, log2_seg);
+	// segments per job, 2^v[q] words each; jobs with more than one need jumps
+	std::vector<int> K(jobs.size()), v(jobs.size(), v_call);
 	int Kmax = 1;
 	size_t nstates = 0;
 	std::vector<char> ready(jobs.size(), 0);  // windows precomputed: no jumps here
 	std::vector<const uint32_t*> state0(jobs.size(), nullptr);  // per job: K windows of nn words
 	for (size_t q = 0; q < jobs.size(); ++q) {
 		const unsigned long long total = jobs[q].offset + jobs[q].count;
-		ARMA_REQUIRE((total + J - 1) / J <= (1ull << kLevels), ARMA_EINVAL, "MT stream too long");
-		K[q] = int(std::max(1ull, (total + J - 1) / J));
+		ARMA_REQUIRE(segments_of(total, log2_seg, log2_seg) <= (1ull << kLevels), ARMA_EINVAL,
+		             "MT stream too long");
 		if (jobs[q].seg_states) {
+			v[q] = jobs[q].seg_log2;
+			K[q] = int(segments_of(total, v[q], log2_seg));
 			ARMA_REQUIRE(K[q] > 1, ARMA_EINVAL, "MT job with windows but one segment");
 			ready[q] = 1;
 			state0[q] = jobs[q].seg_states;
 			continue;
 		}
-		if (K[q] > 1) {
-			tab[q] = &jump_table(c, jobs[q].p, log2_seg);
-			if (!tab[q]->ok) K[q] = 1;  // not a full-period set: one sequential segment
-		}
+		K[q] = int(segments_of(total, v[q], log2_seg));
+		// not a full-period set: one sequential segment
+		if (K[q] > 1 && !jump_table(c, jobs[q].p, v[q])) K[q] = 1;
 		if (K[q] > 1) nstates += size_t(K[q]) * jobs[q].p.nn;
-		Kmax = std::max(Kmax, K[q]);
+		if (K[q] > 1) Kmax = std::max(Kmax, K[q]);
 	}
 	if (nstates) {
 		uint32_t* states = static_cast<uint32_t*>(scratch_take(c, sizeof(uint32_t) * nstates));
+		ARMA_CUDA_TRY(cudaMemsetAsync(states, 0, sizeof(uint32_t) * nstates, c->stream));
 		size_t off = 0;
 		std::vector<arma_mt_params> ps;
 		std::vector<uint32_t> seeds;
@@ -467,52 +604,60 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 		                              cudaMemcpyHostToDevice, c->stream));
 		ARMA_CUDA_TRY(copy_async(c, d_dst, dst.data(), sizeof(uint32_t*) * dst.size(),
 		                              cudaMemcpyHostToDevice, c->stream));
-		mt_seed_kernel<<<int(ps.size()), 32, 0, c->stream>>>(d_ps, d_seeds, d_src, d_dst);
-		c->launches += 1;
-		// binary tree of jumps, widest stride first
+		// binary tree of jumps, widest stride first; every level's jumps in one
+		// table
 		int levels = 0;
 		while ((1 << levels) < Kmax) ++levels;
 		size_t smem = 0;
 		for (size_t q = 0; q < jobs.size(); ++q)
 			if (K[q] > 1 && !ready[q])
-				smem = std::max(smem, sizeof(uint32_t) * size_t(32 * jobs[q].p.nn - jobs[q].p.rr +
-				                                                jobs[q].p.nn + kJumpThreads));
-		ARMA_CUDA_TRY(cudaFuncSetAttribute(mt_jump_kernel,
-		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+				smem = std::max(smem, sizeof(uint32_t) * size_t(jump_words(jobs[q].p)));
+		std::vector<JumpJob> jj;
+		std::vector<size_t> level_at(levels + 1, 0);  // level lv: entries from level_at[lv + 1] on
 		for (int lv = levels - 1; lv >= 0; --lv) {
-			std::vector<JumpJob> jj;
+			level_at[lv + 1] = jj.size();
 			const int step = 1 << lv;
 			for (size_t q = 0; q < jobs.size(); ++q) {
 				if (K[q] <= 1 || ready[q]) continue;
 				const int nn = jobs[q].p.nn;
 				uint32_t* w = states + (state0[q] - states);
+				const uint32_t* bits = step < K[q] ? jump_table(c, jobs[q].p, v[q] + lv) : nullptr;
 				for (int base = 0; base + step < K[q]; base += 2 * step)
-					jj.push_back(JumpJob{jobs[q].p, w + size_t(base) * nn, w + size_t(base + step) * nn,
-					                     tab[q]->bits[lv], tab[q]->nbits[lv]});
+					jj.push_back(JumpJob{jobs[q].p, w + size_t(base) * nn,
+					                     w + size_t(base + step) * nn, bits});
 			}
-			if (jj.empty()) continue;
-			auto* d_jj = static_cast<JumpJob*>(scratch_take(c, sizeof(JumpJob) * jj.size()));
-			ARMA_CUDA_TRY(copy_async(c, d_jj, jj.data(), sizeof(JumpJob) * jj.size(),
-			                              cudaMemcpyHostToDevice, c->stream));
-			// few jumps at this level: split each over several CTAs
-			int parts = int(std::min<size_t>(8, std::max<size_t>(1, (2 * size_t(c->num_sms) +
-			                                                         jj.size() - 1) / jj.size())));
-			for (const JumpJob& j : jj)  // every CTA's share must fit one word per thread
-				parts = std::max(parts, (j.p.nn + kJumpThreads - 1) / kJumpThreads);
-			mt_jump_kernel<<<int(jj.size()) * parts, kJumpThreads, smem, c->stream>>>(d_jj, parts);
+		}
+		level_at[0] = jj.size();
+		auto* d_jj = static_cast<JumpJob*>(scratch_take(c, sizeof(JumpJob) * jj.size()));
+		ARMA_CUDA_TRY(copy_async(c, d_jj, jj.data(), sizeof(JumpJob) * jj.size(),
+		                              cudaMemcpyHostToDevice, c->stream));
+		mt_seed_kernel<<<int(ps.size()), 32, 0, c->stream>>>(d_ps, d_seeds, d_src, d_dst);
+		c->launches += 1;
+		ARMA_CUDA_TRY(cudaFuncSetAttribute(mt_jump_kernel,
+		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		for (int lv = levels - 1; lv >= 0; --lv) {
+			const size_t at = level_at[lv + 1], n = level_at[lv] - at;
+			if (n == 0) continue;
+			// few jumps at this level: split each over several CTAs, at most 32
+			// (a CTA first runs the recurrence up to its bits, about 4 us)
+			const int parts = int(std::min<size_t>(32, std::max<size_t>(1, 2 * size_t(c->num_sms) / n)));
+			mt_jump_kernel<<<unsigned(n) * parts, kJumpThreads, smem, c->stream>>>(d_jj + at, parts);
 			ARMA_CUDA_TRY(cudaGetLastError());
 			c->launches += 1;
 		}
 	}
 	if (prepare) {
 		for (size_t q = 0; q < jobs.size(); ++q)
-			if (K[q] > 1) (*prepare)[q].seg_states = state0[q];
+			if (K[q] > 1) {
+				(*prepare)[q].seg_states = state0[q];
+				(*prepare)[q].seg_log2 = v[q];
+			}
 		return;
 	}
-	// generation: one CTA per segment
+	// generation: one CTA or warp per segment
 	std::vector<SegJob> seg;
 	for (size_t q = 0; q < jobs.size(); ++q) {
-		const unsigned long long total = jobs[q].offset + jobs[q].count;
+		const unsigned long long total = jobs[q].offset + jobs[q].count, J = 1ull << v[q];
 		for (int k = 0; k < K[q]; ++k) {
 			const unsigned long long first = (unsigned long long)k * J;
 			if (K[q] > 1 && first + J <= jobs[q].offset) continue;  // entirely skipped
@@ -527,18 +672,24 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 			seg.push_back(s);
 		}
 	}
-	// segments of nn = 2 mm sets: one warp each (32-bit word indices); the
-	// rest: one CTA each
-	auto by_warp = [](const SegJob& j) {
-		return half_set(j.p) && j.count < (1ull << 30) && j.offset < (1ull << 30) &&
-		       j.first < (1ull << 40);
+	// segments of nn = 2 mm sets (32-bit word indices): one warp each when there
+	// are many, one CTA each when they are few; the others one CTA each in the
+	// general form
+	auto half = [&](const SegJob& j) {
+		return half_set(j.p) && j.p.mm > 2 && j.count < (1ull << 30) &&
+		       j.offset < (1ull << 30) && j.first < (1ull << 40);
 	};
-	std::stable_partition(seg.begin(), seg.end(), by_warp);
-	const int nhalf = int(std::count_if(seg.begin(), seg.end(), by_warp));
+	std::stable_partition(seg.begin(), seg.end(), half);
+	const int nhalf = int(std::count_if(seg.begin(), seg.end(), half));
+	const bool by_warp = size_t(nhalf) > kWarpSegments * size_t(c->num_sms);
 	auto* d_seg = static_cast<SegJob*>(scratch_take(c, sizeof(SegJob) * seg.size()));
 	ARMA_CUDA_TRY(copy_async(c, d_seg, seg.data(), sizeof(SegJob) * seg.size(),
 	                              cudaMemcpyHostToDevice, c->stream));
-	if (nhalf > 0) {
+	if (nhalf > 0 && !by_warp) {
+		mt_generate_four_kernel<<<nhalf, kFourThreads, 0, c->stream>>>(d_seg);
+		ARMA_CUDA_TRY(cudaGetLastError());
+		c->launches += 1;
+	} else if (nhalf > 0) {
 		// mm = 312 (the sets of period 2^19937 - 1) compiled in; others at run time
 		bool all312 = true;
 		for (int k = 0; k < nhalf; ++k) all312 = all312 && seg[k].p.mm == 312;

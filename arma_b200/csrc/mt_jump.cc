@@ -8,14 +8,16 @@
 // characteristic polynomial phi(t) of A.  For a jump of J words:
 //     g(t) = t^J mod phi(t)   =>   x[J + w] = XOR_{i : g_i = 1} x[i + w]
 // for w >= 1 (and the upper 32-rr bits of w = 0), i.e. the window of nn words
-// J positions ahead is an XOR of windows of the raw sequence.  phi is found by
-// Berlekamp-Massey on 2p bits of one bit position of the raw sequence (its
-// minimal polynomial has degree p when phi is primitive, as it is for
-// MT19937 and for dcmt-created sets); t^J for J = 2^q comes from q modular
-// squarings.
+// J positions ahead is an XOR of windows of the raw sequence.  phi is the closed
+// form of dcmt.cpp, checked against the sequence (Berlekamp-Massey on 2p bits of
+// one bit position where the masks are not a dcmt set's); t^J for J = 2^q comes
+// from q modular squarings.  A set's first tables take about 6 ms at p = 19937
+// (170 ms with Berlekamp-Massey and bitwise reductions).
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <vector>
 
 #include "internal.h"
@@ -113,62 +115,69 @@ Bits berlekamp_massey(const std::vector<uint8_t>& s, int* degree) {
 	return phi;
 }
 
-// Reduction context: phi and its 64 bit-shifted copies.
-struct Reducer {
-	int p;
-	std::vector<Bits> shifted;  // shifted[s] = phi << s, sized for aligned XOR
-	explicit Reducer(const Bits& phi, int deg) : p(deg), shifted(64) {
-		const size_t nw = size_t(deg) / 64 + 2;
-		for (int s = 0; s < 64; ++s) {
-			shifted[s].assign(nw, 0);
-			xor_shifted(shifted[s], phi, s, deg + 1);
-		}
-	}
-	// a (degree < 2p) mod phi, in place; result has degree < p
-	void reduce(Bits& a) const {
-		for (long d = 2L * p - 2; d >= p; --d) {
-			if (!get_bit(a, d)) continue;
-			const long sh = d - p;
-			const Bits& ph = shifted[sh & 63];
-			const size_t ws = size_t(sh) >> 6;
-			for (size_t i = 0; i < ph.size() && ws + i < a.size(); ++i) a[ws + i] ^= ph[i];
-		}
-	}
-	Bits square(const Bits& a) const {
-		Bits r(size_t(2 * p) / 64 + 2, 0);
-		for (long i = 0; i < p; ++i)
-			if (get_bit(a, i)) flip_bit(r, 2 * i);
-		reduce(r);
-		r.resize(size_t(p) / 64 + 1);
-		return r;
-	}
+// A parameter set's powers t^(2^e) mod phi, e = 0, 1, ...: found once, extended
+// as larger exponents are asked for.
+struct JumpPowers {
+	Bits phi;             // empty: not a full-period set
+	std::vector<Bits> g;  // g[e] = t^(2^e) mod phi
 };
+
+// Whether phi annihilates the sequence: 64 windows of words from a seeded state,
+// 2048 bit positions.
+bool annihilates(const Bits& phi, int p, const std::vector<uint32_t>& x, size_t start) {
+	for (size_t w = 0; w < 64; ++w) {
+		uint32_t v = 0;
+		for (int i = 0; i <= p; ++i)
+			if (get_bit(phi, i)) v ^= x[start + w + size_t(i)];
+		if (v) return false;
+	}
+	return true;
+}
+
+JumpPowers find_powers(const arma_mt_params& prm) {
+	JumpPowers r;
+	const int p = 32 * prm.nn - prm.rr;
+	// past the seeded words, whose first has bits outside the state
+	const size_t start = size_t(prm.nn);
+	const std::vector<uint32_t> x = raw_words(prm, 4357u, start + 2 * size_t(p) + 64);
+	r.phi = dcmt::characteristic_polynomial(prm);
+	if (r.phi.empty() || !annihilates(r.phi, p, x, start)) {
+		// masks of another shape: the minimal polynomial of 2p bits of one bit
+		// position
+		std::vector<uint8_t> s(2 * size_t(p));
+		for (size_t j = 0; j < s.size(); ++j) s[j] = uint8_t(x[start + j] & 1u);
+		int L = 0;
+		r.phi = berlekamp_massey(s, &L);
+		if (L != p) {  // not a full-period set: the caller generates sequentially
+			r.phi.clear();
+			return r;
+		}
+	}
+	Bits t(size_t(p) / 64 + 1, 0);
+	flip_bit(t, 1);
+	r.g.push_back(std::move(t));
+	return r;
+}
+
+std::mutex g_powers_mutex;
+std::map<std::vector<uint32_t>, JumpPowers> g_powers;
 
 }  // namespace
 
-bool mt_jump_tables(const arma_mt_params& prm, int log2_jump, int levels,
-                    std::vector<std::vector<int32_t>>* set_bits, int* degree) {
+bool mt_jump_bits(const arma_mt_params& prm, int e, std::vector<uint32_t>* bits) {
+	std::vector<uint32_t> key(sizeof(prm) / 4);
+	std::memcpy(key.data(), &prm, sizeof(prm));
+	key.back() = 0;  // the `i` field does not affect the stream
+	std::lock_guard<std::mutex> lock(g_powers_mutex);
+	auto it = g_powers.find(key);
+	if (it == g_powers.end()) it = g_powers.emplace(key, find_powers(prm)).first;
+	JumpPowers& jp = it->second;
+	if (jp.phi.empty()) return false;
 	const int p = 32 * prm.nn - prm.rr;
-	// 2p bits of bit 0 of the raw sequence, starting past the seeded words
-	const size_t start = size_t(prm.nn);
-	std::vector<uint32_t> x = raw_words(prm, 4357u, start + 2 * size_t(p) + 8);
-	std::vector<uint8_t> s(2 * size_t(p));
-	for (size_t j = 0; j < s.size(); ++j) s[j] = uint8_t(x[start + j] & 1u);
-	int L = 0;
-	Bits phi = berlekamp_massey(s, &L);
-	*degree = L;
-	if (L != p) return false;  // not a full-period set: the caller generates sequentially
-	Reducer red(phi, p);
-	Bits g(size_t(p) / 64 + 1, 0);
-	flip_bit(g, 1);  // t
-	for (int q = 0; q < log2_jump; ++q) g = red.square(g);
-	set_bits->assign(levels, {});
-	for (int lv = 0; lv < levels; ++lv) {
-		auto& v = (*set_bits)[lv];
-		for (long i = 0; i < p; ++i)
-			if (get_bit(g, i)) v.push_back(int32_t(i));
-		g = red.square(g);
-	}
+	if (int(jp.g.size()) <= e) dcmt::square_powers_of_t(jp.phi, p, int(jp.g.size()), e, &jp.g);
+	bits->assign((size_t(p) + 31) / 32, 0u);
+	for (long i = 0; i < p; ++i)
+		if (get_bit(jp.g[e], i)) (*bits)[size_t(i) >> 5] |= 1u << (i & 31);
 	return true;
 }
 
