@@ -11,18 +11,22 @@
 //   1. accumulate the terms on slices t-1 .. t-pt+1 (90% of the work for a
 //      10^3 model) from a shared-memory ring that holds those slices for the
 //      tile plus its west/north halo,
-//   2.-3. meanwhile a fifth warp publishes slice t-1, clears the ring slot of
-//      slice t, waits for the three neighbour tiles (x-1, y-1, both) to
-//      publish slice t (a per-tile counter in global memory; bounded spin)
-//      and loads slice t of the halo; then the compute warps add the
-//      current-slice terms that reach into the halo (the in-tile part of the
-//      current slice is held at zero),
+//   2.-3. wait for slice t's halo, which a fifth warp brings in a slice ahead
+//      (slot t cleared, the three neighbour tiles x-1, y-1 and both seen to
+//      have published slice t, their values copied; bounded polls of a
+//      per-tile counter in global memory), and add the current-slice terms
+//      that reach into it (the in-tile part of the current slice is held at
+//      zero),
 //   4. solve the remaining in-tile recursion zeta = S + A0 zeta exactly as a
 //      quarter-plane convolution zeta = H * S, where H is the impulse response
 //      of 1 / (1 - A0(z1,z2)) on the tile (precomputed in FP64),
 //   5. store the slice to the ring and to global memory; the fifth warp
-//      publishes it (release store after a fence) off the compute warps'
+//      publishes it (release store after a barrier) off the compute warps'
 //      critical path.
+// The ring has one slot more than the slices in use, so that the halo of slice
+// t+1 comes in while slice t is computed (512 x 256 x 256 points of order 10^3,
+// one tile per SM: 5.42 -> 5.20 ms; the batch of 256 surfaces 52.3 -> 51.8 ms;
+// one 64 x 32 x 32 surface 258 -> 241 us).
 // The coefficients are carried as hi + lo float pairs (rounding phi to one
 // float perturbs a high-gain recursion far more than FP32 summation does):
 // each (k,i) row of taps feeds two FP32 FMA chains over one register window,
@@ -55,9 +59,10 @@ constexpr int GROUP = TX * STRIPS; // threads covering the tile once
 constexpr int NCOMP = 2 * GROUP;   // compute threads: two groups split the tap rows
 constexpr int NTHREADS = NCOMP + 32; // plus the halo / publication warp
 // named barriers (0 is __syncthreads)
-constexpr int BAR_HALO = 1;        // halo warp -> compute: slot t cleared, halo of t loaded
-constexpr int BAR_COMP = 2;        // compute threads among themselves
-constexpr int BAR_DONE = 3;        // compute -> halo warp: slice t stored
+constexpr int BAR_HALO = 1;        // (2, by slice parity) halo warp -> compute: halo of t in slot t
+constexpr int BAR_COMP = 3;        // compute threads among themselves
+constexpr int BAR_PUB = 4;         // (PUB_BARS, by slice) compute -> halo warp: slice t stored
+constexpr int PUB_BARS = 8;
 constexpr int LH = 12;            // left (y) halo columns held in the ring
 constexpr int W = LH + TY;        // ring row width (floats)
 constexpr int SPAD = TY + 8;      // zero padding left of each S row
@@ -115,29 +120,45 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 	return v;
 }
 
+__device__ __forceinline__ int ld_acquire_cta(const int* p) {
+	int v;
+	const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+	asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+	return v;
+}
+
+__device__ __forceinline__ void st_release_cta(int* p, int v) {
+	const unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p));
+	asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void st_release(int* p, int v) {
 	asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Wait until every non-null flag is >= need; the three acquire loads of a
-// poll are issued together so one L2 round trip covers them.  seen[] holds the
-// values this thread's earlier acquire loads returned: a neighbour that is
-// already known to be at or past `need` is not polled again (that load's
-// acquire already ordered its slices before this thread's later loads), so a
-// tile whose neighbours run ahead pays no round trip.  Gives up after
-// kSpinLimit polls (or when another CTA already gave up) and reports
-// DEV_TIMEOUT; returns false then.
+// Whether every non-null flag is >= need; the three acquire loads of a poll are
+// issued together so one L2 round trip covers them.  seen[] holds the values
+// this thread's earlier acquire loads returned: a neighbour that is already
+// known to be at or past `need` is not polled again (that load's acquire already
+// ordered its slices before this thread's later loads), so a tile whose
+// neighbours run ahead pays no round trip.
+__device__ bool flags_reached(const int* f0, const int* f1, const int* f2, int need, int* seen) {
+	if (seen[0] >= need && seen[1] >= need && seen[2] >= need) return true;
+	const int a = f0 ? ld_acquire(f0) : need;
+	const int b = f1 ? ld_acquire(f1) : need;
+	const int c = f2 ? ld_acquire(f2) : need;
+	seen[0] = f0 ? a : INT_MAX;
+	seen[1] = f1 ? b : INT_MAX;
+	seen[2] = f2 ? c : INT_MAX;
+	return a >= need && b >= need && c >= need;
+}
+
+// Waits for that; gives up after kSpinLimit polls (or when another CTA already
+// gave up) and reports DEV_TIMEOUT; returns false then.
 __device__ bool wait_flags(const int* f0, const int* f1, const int* f2, int need, int* seen,
                            int* err) {
-	if (seen[0] >= need && seen[1] >= need && seen[2] >= need) return true;
 	for (long long it = 0; it < kSpinLimit; ++it) {
-		const int a = f0 ? ld_acquire(f0) : need;
-		const int b = f1 ? ld_acquire(f1) : need;
-		const int c = f2 ? ld_acquire(f2) : need;
-		seen[0] = f0 ? a : INT_MAX;
-		seen[1] = f1 ? b : INT_MAX;
-		seen[2] = f2 ? c : INT_MAX;
-		if (a >= need && b >= need && c >= need) return true;
+		if (flags_reached(f0, f1, f2, need, seen)) return true;
 		if ((it & 63) == 63 && *((volatile int*)err) != DEV_OK) return false;
 		__nanosleep(64);
 	}
@@ -158,7 +179,7 @@ __device__ bool wait_flags(const int* f0, const int* f1, const int* f2, int need
 // partials of an output are Kahan-added afterwards.  Lanes of one warp work
 // on different rows of H at once: H rows are HS floats apart in shared memory
 // so that their 16-byte loads fall in different banks.  The unit is inlined
-// into every tap-count instantiation of run_tile: as a call, the registers
+// into every tap-count instantiation of compute_tile: as a call, the registers
 // the caller keeps across it spilled, and the filter ran 7 % slower.
 __device__ __forceinline__ int h_rowbase(int x) {
 	// sum over x' < x of ceil((x'+1) / HCH), for HCH = 3
@@ -246,137 +267,157 @@ __device__ __forceinline__ void h_unit(const float* ss, const float* sh, int u, 
 	}
 }
 
-template <int PY>
-__device__ void run_tile(const Task& tk, int bx, int by, float* smem, unsigned char* s_lo,
-                         int* err) {
-	const int tid = threadIdx.x;
-	if (bx < tk.given_tx) {
-		// a given tile (the band above an x-strip, holding the upper strip's
-		// finished values): published as complete for every slice at once
-		if (tid == 0) st_release(tk.flags + bx * tk.tiles_y + by, tk.nt);
-		return;
+// Layout of a tile's shared memory (floats).
+struct Layout {
+	int hx, slot_sz, slots;   // halo rows, floats per ring slot, ring slots
+	int taps;                 // floats of one part of the coefficients (rows of PYP)
+	int pyp;
+};
+
+__host__ __device__ inline Layout tile_layout(int pt, int px, int py) {
+	Layout l;
+	l.hx = px - 1;
+	l.slot_sz = (TX + px - 1) * W;
+	l.slots = pt + 1;  // the pt slices in use and the next one's halo
+	l.pyp = (py + 3) & ~3;
+	l.taps = pt * px * l.pyp;
+	return l;
+}
+
+// Where the two sides of a CTA stand on the current tile.
+struct Progress {
+	int done;       // slices finished by the compute warps
+	int published;  // slices taken over for publication
+};
+
+// The halo / publication warp takes whichever of its two tasks is ready,
+// both off the compute warps' path:
+//   publish: a barrier orders the compute warps' global stores of the
+//   slices they have finished before the release store of the count;
+//   halo, a slice ahead of them: once slice t-2 is done (the last to
+//   read the old contents of slot t) it clears slot t and, when the three
+//   neighbour tiles have published slice t, loads slice t's halo.
+// Waiting for the neighbours runs out after kSpinLimit rounds without
+// progress: the error word is set, the tile runs on without its halo, and
+// the call fails.
+__device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Layout& L, float* ring,
+                                       Progress* sh, int* err) {
+	const int lane = threadIdx.x & 31;
+	const int hx = L.hx, slot_sz = L.slot_sz, slots = L.slots;
+	const int x0 = bx * TX, y0 = by * TY;
+	const long long sst = (long long)tk.nx * tk.ny;
+	// 16-byte halo chunks need 16-byte aligned rows in global memory
+	const bool vec_ok = (tk.ny % 4 == 0) &&
+	                    ((reinterpret_cast<uintptr_t>(tk.zeta) & 15) == 0) && ((sst % 4) == 0);
+	const int* fW = (bx > 0) ? tk.flags + (bx - 1) * tk.tiles_y + by : nullptr;
+	const int* fN = (by > 0) ? tk.flags + bx * tk.tiles_y + by - 1 : nullptr;
+	const int* fNW = (bx > 0 && by > 0) ? tk.flags + (bx - 1) * tk.tiles_y + by - 1 : nullptr;
+	int* own_flag = tk.flags + bx * tk.tiles_y + by;
+	int seen[3] = {-1, -1, -1};
+	int pub = tk.t0;            // slices published
+	int t = tk.t0;              // the next slice to bring the halo of
+	bool cleared = false;       // slot t
+	long long idle = 0;
+	while (pub < tk.nt) {
+		const int done = __shfl_sync(0xffffffffu, lane == 0 ? ld_acquire_cta(&sh->done) : 0, 0);
+		if (done > pub) {
+			for (; pub < done; ++pub) bar_sync(BAR_PUB + pub % PUB_BARS, NTHREADS);
+			if (lane == 0) {
+				*((volatile int*)&sh->published) = pub;
+				st_release(own_flag, pub);
+			}
+			__syncwarp();
+			idle = 0;
+		}
+		if (t >= tk.nt || done < t - 1) {
+			++idle;  // the compute warps are at work: they end every slice
+			if (idle > 64 * kSpinLimit) break;
+			continue;
+		}
+		float* cur = ring + (t % slots) * slot_sz;
+		if (!cleared) {
+			for (int q = lane; q < slot_sz / 4; q += 32)
+				reinterpret_cast<float4*>(cur)[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			__syncwarp();
+			cleared = true;
+		}
+		int ok = 1;
+		if (lane == 0) {
+			ok = flags_reached(fW, fN, fNW, t + 1, seen) ? 1 : 0;
+			if (!ok && (idle & 63) == 63 && *((volatile int*)err) != DEV_OK) ok = 1;
+			if (!ok && idle > kSpinLimit) {
+				atomicExch(err, DEV_TIMEOUT);
+				ok = 1;
+			}
+		}
+		ok = __shfl_sync(0xffffffffu, ok, 0);
+		if (!ok) {
+			++idle;
+			__nanosleep(32);
+			continue;
+		}
+		idle = 0;
+		// rows above the tile (all columns) and the left columns of the
+		// tile rows, in 16-byte chunks copied with L2-only asynchronous
+		// copies (scalar loads at ragged edges)
+		const float* zt = tk.zeta + t * sst;
+		const int top = hx * (W / 4);
+		const int nch = top + TX * (LH / 4);
+		for (int q = lane; q < nch; q += 32) {
+			int rr, c4;
+			if (q < top) {
+				rr = q / (W / 4);
+				c4 = q % (W / 4);
+			} else {
+				rr = hx + (q - top) / (LH / 4);
+				c4 = (q - top) % (LH / 4);
+			}
+			const int x = x0 - hx + rr, y = y0 - LH + 4 * c4;
+			if (x < 0 || x >= tk.nx) continue;  // stays zero
+			float* dst = cur + rr * W + 4 * c4;
+			const float* src = zt + (long long)x * tk.ny + y;
+			if (vec_ok && y >= 0 && y + 4 <= tk.ny) {
+				cp_async16(dst, src);
+			} else {
+				for (int e = 0; e < 4; ++e)
+					if (y + e >= 0 && y + e < tk.ny) dst[e] = __ldcg(src + e);
+			}
+		}
+		cp_async_wait_all();
+		__syncwarp();
+		bar_arrive(BAR_HALO + (t & 1), NTHREADS);
+		++t;
+		cleared = false;
 	}
+}
+
+template <int PY>
+__device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, const Layout& L,
+                                             float* smem, const unsigned char* s_lo, Progress* sh,
+                                             int* err) {
+	const int tid = threadIdx.x;
 	const int grp = tid / GROUP;                 // 0 or 1: halves of the tap rows
 	const int lt = tid % GROUP;
 	const int xl = lt / STRIPS;                  // tile-local row
 	const int yl0 = (lt % STRIPS) * R;           // tile-local first column
 	const int pt = tk.pt, px = tk.px;
-	const int hx = px - 1;
-	const int rows = TX + hx;
-	const int slot_sz = rows * W;
+	const int hx = L.hx, slot_sz = L.slot_sz, slots = L.slots;
 	constexpr int PYP = (PY + 3) & ~3;           // padded tap row
 	const int x0 = bx * TX, y0 = by * TY;
 	const long long sst = (long long)tk.nx * tk.ny;
 
-	float* ring = smem;                          // pt slots
-	float* sphi = ring + pt * slot_sz;           // pt*px*PYP (hi)
-	float* slo = sphi + pt * px * PYP;           // pt*px*PYP (lo)
-	float* sh = slo + pt * px * PYP;             // TX*HS
-	float* ss = sh + TX * HS;                    // TX*SW
+	float* ring = smem;                          // slots
+	float* sphi = ring + slots * slot_sz;        // hi
+	float* slo = sphi + L.taps;                  // lo
+	float* sh_h = slo + L.taps;                  // TX*HS
+	float* ss = sh_h + TX * HS;                  // TX*SW
 	float* part = ss + TX * SW;                  // HUNITS*PS: H-unit partials
 	float* comb = part;                          // GROUP*R: group 1 partials (before H)
-
-	// stage coefficients (rows padded with zeros), H, zero the ring and S pads
-	for (int q = tid; q < pt * px * PYP; q += NTHREADS) {
-		const int j = q % PYP, ki = q / PYP;
-		sphi[q] = j < PY ? tk.phi[ki * PY + j] : 0.0f;
-		slo[q] = j < PY ? tk.phi_lo[ki * PY + j] : 0.0f;
-	}
-	// rows whose lo parts are all zero skip their second FMA chain
-	for (int ki = tid; ki < pt * px; ki += NTHREADS) {
-		bool nz = false;
-		for (int j = 0; j < PY; ++j) nz = nz || tk.phi_lo[ki * PY + j] != 0.0f;
-		s_lo[ki] = nz ? 1 : 0;
-	}
-	for (int q = tid; q < TX * TY; q += NTHREADS) sh[(q / TY) * HS + q % TY] = tk.h[q];
-	for (int q = tid; q < pt * slot_sz; q += NTHREADS) ring[q] = 0.0f;
-	for (int q = tid; q < TX * SW; q += NTHREADS) ss[q] = 0.0f;
-	__syncthreads();
-	// history slices (a stream's previous chunk): the whole ring slot, tile
-	// and halo, straight from global memory (zero outside the surface)
-	for (int tt = max(0, tk.t0 - pt + 1); tt < tk.t0; ++tt) {
-		float* slot = ring + (tt % pt) * slot_sz;
-		const float* zs = tk.zeta + tt * sst;
-		for (int q = tid; q < slot_sz; q += NTHREADS) {
-			const int x = x0 - hx + q / W, y = y0 - LH + q % W;
-			if (x >= 0 && x < tk.nx && y >= 0 && y < tk.ny) slot[q] = __ldcg(zs + (long long)x * tk.ny + y);
-		}
-	}
-	__syncthreads();
-
-	__shared__ int s_ok;
-	if (tid >= NCOMP) {
-		// The halo / publication warp.  For slice t it waits until the compute
-		// threads have stored slice t-1 (which also ends their use of slot t's
-		// previous contents), publishes slice t-1, clears slot t, waits for the
-		// three neighbour tiles to publish slice t and loads slice t's halo,
-		// while the compute threads accumulate the previous slices' terms.
-		const int lane = tid - NCOMP;
-		// 16-byte halo chunks need 16-byte aligned rows in global memory
-		const bool vec_ok = (tk.ny % 4 == 0) &&
-		                    ((reinterpret_cast<uintptr_t>(tk.zeta) & 15) == 0) && ((sst % 4) == 0);
-		const int* fW = (bx > 0) ? tk.flags + (bx - 1) * tk.tiles_y + by : nullptr;
-		const int* fN = (by > 0) ? tk.flags + bx * tk.tiles_y + by - 1 : nullptr;
-		const int* fNW = (bx > 0 && by > 0) ? tk.flags + (bx - 1) * tk.tiles_y + by - 1 : nullptr;
-		int* own_flag = tk.flags + bx * tk.tiles_y + by;
-		int seen[3] = {-1, -1, -1};
-		for (int t = tk.t0; t < tk.nt; ++t) {
-			// the release store orders the compute threads' stores of slice
-			// t-1 (made visible to this thread by the barrier) before the flag
-			if (t > tk.t0) {
-				bar_sync(BAR_DONE, NTHREADS);
-				if (lane == 0) st_release(own_flag, t);
-			}
-			float* cur = ring + (t % pt) * slot_sz;
-			const float* zt = tk.zeta + t * sst;
-			for (int q = lane; q < slot_sz; q += 32) cur[q] = 0.0f;
-			__syncwarp();
-			int ok = 1;
-			if (lane == 0) ok = wait_flags(fW, fN, fNW, t + 1, seen, err) ? 1 : 0;
-			ok = __shfl_sync(0xffffffffu, ok, 0);
-			if (ok) {
-				// rows above the tile (all columns) and the left columns of the
-				// tile rows, in 16-byte chunks copied with L2-only asynchronous
-				// copies (scalar loads at ragged edges)
-				const int top = hx * (W / 4);
-				const int nch = top + TX * (LH / 4);
-				for (int q = lane; q < nch; q += 32) {
-					int rr, c4;
-					if (q < top) {
-						rr = q / (W / 4);
-						c4 = q % (W / 4);
-					} else {
-						rr = hx + (q - top) / (LH / 4);
-						c4 = (q - top) % (LH / 4);
-					}
-					const int x = x0 - hx + rr, y = y0 - LH + 4 * c4;
-					if (x < 0 || x >= tk.nx) continue;  // stays zero
-					float* dst = cur + rr * W + 4 * c4;
-					const float* src = zt + (long long)x * tk.ny + y;
-					if (vec_ok && y >= 0 && y + 4 <= tk.ny) {
-						cp_async16(dst, src);
-					} else {
-						for (int e = 0; e < 4; ++e)
-							if (y + e >= 0 && y + e < tk.ny) dst[e] = __ldcg(src + e);
-					}
-				}
-				cp_async_wait_all();
-			}
-			if (lane == 0) s_ok = ok;
-			bar_arrive(BAR_HALO, NTHREADS);
-			if (!ok) return;
-		}
-		if (tk.nt > tk.t0) {
-			bar_sync(BAR_DONE, NTHREADS);
-			if (lane == 0) st_release(own_flag, tk.nt);
-		}
-		return;
-	}
-
 	const int gx = x0 + xl;
 
-	for (int t = tk.t0; t < tk.nt; ++t) {
-		float* cur = ring + (t % pt) * slot_sz;
+	int st = tk.t0 % slots;  // slot of slice t
+	for (int t = tk.t0; t < tk.nt; ++t, st = st + 1 == slots ? 0 : st + 1) {
+		float* cur = ring + st * slot_sz;
 		float* zt = tk.zeta + t * sst;
 		// group 0 starts from the noise of its strip (own tile: written by an
 		// earlier kernel), group 1 from zero
@@ -448,12 +489,14 @@ __device__ void run_tile(const Task& tk, int bx, int by, float* smem, unsigned c
 			for (int r = 0; r < R; ++r) kahan_add(s[r], c[r], pk[r] + qk[r]);
 		};
 
-		// 1. previous slices (the halo warp meanwhile prepares slot t)
-		for (int k = 1; k < pt && k <= t; ++k) accumulate_rows(ring + ((t - k) % pt) * slot_sz, k);
+		// 1. previous slices
+		for (int k = 1, sk = st; k < pt && k <= t; ++k) {
+			sk = sk == 0 ? slots - 1 : sk - 1;
+			accumulate_rows(ring + sk * slot_sz, k);
+		}
 
 		// 2./3. slot t cleared, neighbours' slice t published, halo loaded
-		bar_sync(BAR_HALO, NTHREADS);
-		if (!s_ok) return;
+		bar_sync(BAR_HALO + (t & 1), NTHREADS);
 		accumulate_rows(cur, 0);
 
 		// 4. S = noise + all terms outside the unknown in-tile part
@@ -473,7 +516,7 @@ __device__ void run_tile(const Task& tk, int bx, int by, float* smem, unsigned c
 		bar_sync(BAR_COMP, NCOMP);
 
 		//    zeta = H * S over the quarter plane of the tile, in work units
-		if (tid < HUNITS) h_unit(ss, sh, tid, part);
+		if (tid < HUNITS) h_unit(ss, sh_h, tid, part);
 
 		// 5. sum each output's unit partials (Kahan, in dx order), store the
 		//    solved slice; the halo warp publishes it
@@ -499,15 +542,66 @@ __device__ void run_tile(const Task& tk, int bx, int by, float* smem, unsigned c
 			}
 			float* own = cur + hx * W + LH + ox * W + oy0;
 #pragma unroll
+			for (int e = 0; e < 4; ++e) own[e] = a[e] - ac[e];
+			bar_sync(BAR_COMP, NCOMP);  // slice t in the ring for every compute thread
+			// (released before this slice's global stores: it waits for none)
+			if (tid == 0) st_release_cta(&sh->done, t + 1);
+#pragma unroll
 			for (int e = 0; e < 4; ++e) {
-				const float v = a[e] - ac[e];
-				own[e] = v;
 				const int gy = y0 + oy0 + e;
-				if (ogx < tk.nx && gy < tk.ny) zt[(long long)ogx * tk.ny + gy] = v;
+				if (ogx < tk.nx && gy < tk.ny) zt[(long long)ogx * tk.ny + gy] = a[e] - ac[e];
 			}
 		}
-		bar_sync(BAR_COMP, NCOMP);  // slice t in the ring for every compute thread
-		bar_arrive(BAR_DONE, NTHREADS);
+		// the barrier's previous round is over once the publication warp has
+		// left it (it waits for nothing but these barriers)
+		for (long long it = 0; *((volatile int*)&sh->published) < t + 1 - PUB_BARS; ++it)
+			if (it == 64 * kSpinLimit) {
+				atomicExch(err, DEV_TIMEOUT);
+				break;
+			}
+		__syncwarp();
+		bar_arrive(BAR_PUB + t % PUB_BARS, NTHREADS);
+	}
+}
+
+// A tile's coefficients, H, zeroed ring and history into shared memory.
+__device__ __noinline__ void stage_tile(const Task& tk, int bx, int by, const Layout& L,
+                                        float* smem, unsigned char* s_lo) {
+	const int tid = threadIdx.x;
+	const int pt = tk.pt, px = tk.px, py = tk.py, pyp = L.pyp;
+	const int x0 = bx * TX, y0 = by * TY;
+	const long long sst = (long long)tk.nx * tk.ny;
+	float* ring = smem;
+	float* sphi = ring + L.slots * L.slot_sz;
+	float* slo = sphi + L.taps;
+	float* sh_h = slo + L.taps;
+	float* ss = sh_h + TX * HS;
+	// coefficient rows padded with zeros, H, the ring and S pads zero
+	for (int q = tid; q < L.taps; q += NTHREADS) {
+		const int j = q % pyp, ki = q / pyp;
+		sphi[q] = j < py ? tk.phi[ki * py + j] : 0.0f;
+		slo[q] = j < py ? tk.phi_lo[ki * py + j] : 0.0f;
+	}
+	// rows whose lo parts are all zero skip their second FMA chain
+	for (int ki = tid; ki < pt * px; ki += NTHREADS) {
+		bool nz = false;
+		for (int j = 0; j < py; ++j) nz = nz || tk.phi_lo[ki * py + j] != 0.0f;
+		s_lo[ki] = nz ? 1 : 0;
+	}
+	for (int q = tid; q < TX * TY; q += NTHREADS) sh_h[(q / TY) * HS + q % TY] = tk.h[q];
+	for (int q = tid; q < L.slots * L.slot_sz; q += NTHREADS) ring[q] = 0.0f;
+	for (int q = tid; q < TX * SW; q += NTHREADS) ss[q] = 0.0f;
+	__syncthreads();
+	// history slices (a stream's previous chunk): the whole ring slot, tile
+	// and halo, straight from global memory (zero outside the surface)
+	for (int tt = max(0, tk.t0 - pt + 1); tt < tk.t0; ++tt) {
+		float* slot = ring + (tt % L.slots) * L.slot_sz;
+		const float* zs = tk.zeta + tt * sst;
+		for (int q = tid; q < L.slot_sz; q += NTHREADS) {
+			const int x = x0 - L.hx + q / W, y = y0 - LH + q % W;
+			if (x >= 0 && x < tk.nx && y >= 0 && y < tk.ny)
+				slot[q] = __ldcg(zs + (long long)x * tk.ny + y);
+		}
 	}
 }
 
@@ -518,14 +612,16 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
              int* __restrict__ ticket_counter, int* __restrict__ err) {
 	extern __shared__ __align__(16) float smem[];
 	__shared__ int s_ticket;
+	__shared__ Progress sh;
 	__shared__ unsigned char s_lo[kMaxTapRows];  // per (k, i) tap row: lo part present
+	const int tid = threadIdx.x;
 	for (;;) {
-		if (threadIdx.x == 0) s_ticket = atomicAdd(ticket_counter, 1);
+		if (tid == 0)
+			s_ticket = *((volatile int*)err) == DEV_OK ? atomicAdd(ticket_counter, 1) : total_tickets;
 		__syncthreads();
 		const int ticket = s_ticket;
 		__syncthreads();
 		if (ticket >= total_tickets) return;
-		if (*((volatile int*)err) != DEV_OK) return;
 		// locate the surface owning this ticket
 		int lo = 0, hi = ntasks - 1;
 		while (lo < hi) {
@@ -535,22 +631,38 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 		const Task tk = tasks[lo];
 		const int local = ticket - tk.ticket_base;
 		const int bx = local / tk.tiles_y, by = local % tk.tiles_y;
-		switch (tk.py) {
-#define ARMA_PY_CASE(N) case N: run_tile<N>(tk, bx, by, smem, s_lo, err); break;
-			ARMA_PY_CASE(1) ARMA_PY_CASE(2) ARMA_PY_CASE(3) ARMA_PY_CASE(4) ARMA_PY_CASE(5)
-			ARMA_PY_CASE(6) ARMA_PY_CASE(7) ARMA_PY_CASE(8) ARMA_PY_CASE(9) ARMA_PY_CASE(10)
-			ARMA_PY_CASE(11) ARMA_PY_CASE(12) ARMA_PY_CASE(13)
+		if (bx < tk.given_tx) {
+			// a given tile (the band above an x-strip, holding the upper strip's
+			// finished values): published as complete for every slice at once
+			if (tid == 0) st_release(tk.flags + bx * tk.tiles_y + by, tk.nt);
+			continue;
+		}
+		const Layout L = tile_layout(tk.pt, tk.px, tk.py);
+		stage_tile(tk, bx, by, L, smem, s_lo);
+		if (tid == 0) {
+			sh.done = tk.t0;
+			sh.published = tk.t0;
+		}
+		__syncthreads();
+		if (tid >= NCOMP) {
+			halo_warp(tk, bx, by, L, smem, &sh, err);
+		} else {
+			switch (tk.py) {
+#define ARMA_PY_CASE(N) case N: compute_tile<N>(tk, bx, by, L, smem, s_lo, &sh, err); break;
+				ARMA_PY_CASE(1) ARMA_PY_CASE(2) ARMA_PY_CASE(3) ARMA_PY_CASE(4) ARMA_PY_CASE(5)
+				ARMA_PY_CASE(6) ARMA_PY_CASE(7) ARMA_PY_CASE(8) ARMA_PY_CASE(9) ARMA_PY_CASE(10)
+				ARMA_PY_CASE(11) ARMA_PY_CASE(12) ARMA_PY_CASE(13)
 #undef ARMA_PY_CASE
-			default: break;
+				default: break;
+			}
 		}
 		__syncthreads();
 	}
 }
 
 size_t smem_bytes(int pt, int px, int py) {
-	const int rows = TX + px - 1;
-	const int pyp = (py + 3) & ~3;
-	return sizeof(float) * (size_t(pt) * rows * W + 2 * size_t(pt) * px * pyp + TX * HS + TX * SW +
+	const Layout l = tile_layout(pt, px, py);
+	return sizeof(float) * (size_t(l.slots) * l.slot_sz + 2 * size_t(l.taps) + TX * HS + TX * SW +
 	                        std::max(GROUP * R, HUNITS * PS));
 }
 
