@@ -31,7 +31,8 @@ namespace {
 constexpr int kAcThreads = 256;
 constexpr int kMaxLine = 1024;
 constexpr int kAcStages = 10;          // 2^10 = 1024
-constexpr int kAcBand = 3072;          // points of a band (48 KB)
+constexpr int kAcBand = 3072;          // most points of a band (48 KB)
+constexpr int kAcLeast = 256;          // fewest
 
 struct AcPlan {
 	int n, m;
@@ -330,10 +331,15 @@ void allow_smem(K* kernel, size_t bytes) {
 	                                   int(bytes)));
 }
 
-// Columns per CTA: about kAcBand points, at least four (64 bytes of a row), the
+// Points of a band: enough bands for four per SM, within [kAcLeast, kAcBand].
+int band_points(Ctx* c, long long total) {
+	return int(std::min<long long>(kAcBand, std::max<long long>(kAcLeast, total / (4ll * c->num_sms))));
+}
+
+// Columns per CTA: about `points` points, at least four (64 bytes of a row), the
 // bands of a row equally wide.
-int columns_per_band(int n, int cols) {
-	const int most = std::max(4, kAcBand / n);
+int columns_per_band(int n, int cols, int points) {
+	const int most = std::max(4, points / n);
 	const int bands = (cols + most - 1) / most;
 	return (cols + bands - 1) / bands;
 }
@@ -341,7 +347,7 @@ int columns_per_band(int n, int cols) {
 template <int WHAT>
 void launch_columns(Ctx* c, double2* w, long long slabs, int cols, const double2* roots,
                     const AcPlan& P) {
-	const int band = columns_per_band(P.n, cols);
+	const int band = columns_per_band(P.n, cols, band_points(c, slabs * P.n * cols));
 	const size_t smem = ac_smem(P, P.n * band);
 	allow_smem(columns_kernel<WHAT>, smem);
 	columns_kernel<WHAT><<<dim3((cols + band - 1) / band, unsigned(slabs)), kAcThreads, smem,
@@ -366,7 +372,7 @@ void launch_auto_covariance(Ctx* c, const void* d_in, const int shape[3], int pr
 	const double2 *rt = roots, *rx = roots + nt, *ry = roots + nt + nx;
 	roots_kernel<<<(nt + nx + ny + kAcThreads - 1) / kAcThreads, kAcThreads, 0, c->stream>>>(
 	    roots, nt, nx, ny);
-	const int pairs = int(std::min<long long>((lines + 1) / 2, std::max(1, kAcBand / (ny + 1))));
+	const int pairs = int(std::min<long long>((lines + 1) / 2, std::max(1, band_points(c, lines / 2 * ny) / (ny + 1))));
 	const size_t smem = ac_smem(py, pairs * (ny + 1));
 	const unsigned grid = unsigned(((lines + 1) / 2 + pairs - 1) / pairs);
 	if (precision == ARMA_FP64) {
