@@ -17,7 +17,7 @@
 // other prime by direct summation, one output per thread.
 //
 // Bound by the lines' butterflies (their index arithmetic and shared-memory
-// round trips; the passes move 0.5 GB, 80 us): 256 x 128 x 128 FP64 200 us; one
+// round trips; the passes move 0.5 GB, 80 us): 256 x 128 x 128 FP64 167 us; one
 // complex pass per axis with every line by direct summation took 5540 us.  Bands
 // of 3072 points: 1024 ran 20 to 40 % slower, 4096 the same.
 #include <algorithm>
@@ -37,11 +37,14 @@ constexpr int kAcLeast = 256;          // fewest
 struct AcPlan {
 	int n, m;
 	int r[kAcStages];
+	int h[kAcStages], tws[kAcStages];  // sub-block length, twiddle stride n / (r h)
+	Divider by_h[kAcStages], by_per[kAcStages], by_r[kAcStages];  // per: work items of a line
 	bool spare;  // a direct stage: the band needs a second buffer
 };
 
 AcPlan ac_plan(int n) {
-	AcPlan p{n, 0, {0}, false};
+	AcPlan p{};
+	p.n = n;
 	int rest = n;
 	for (int f : {4, 2, 3, 5, 7})
 		while (rest % f == 0) {
@@ -54,6 +57,16 @@ AcPlan ac_plan(int n) {
 			rest /= f;
 			p.spare = true;
 		}
+	int L = n;
+	for (int s = 0; s < p.m; ++s) {
+		const int r = p.r[s];
+		p.h[s] = L / r;
+		p.tws[s] = n / L;
+		p.by_h[s] = Divider(p.h[s]);
+		p.by_per[s] = Divider(r > 7 ? n : n / r);
+		p.by_r[s] = Divider(r);
+		L = p.h[s];
+	}
 	return p;
 }
 
@@ -88,13 +101,6 @@ __global__ void roots_kernel(double2* __restrict__ roots, int n0, int n1, int n2
 __device__ void ac_twiddles(double2* tw, const double2* __restrict__ roots, int n) {
 	for (int k = threadIdx.x; k < n; k += kAcThreads) tw[k] = roots[k];
 }
-
-// q / d for 0 <= q < 2^16 and a divisor fixed per stage
-struct Divider {
-	unsigned d, m;
-	__device__ explicit Divider(int v) : d(v), m(v == 1 ? 0u : unsigned((0x100000000ull + v - 1) / v)) {}
-	__device__ int div(int q) const { return m ? int(__umulhi(unsigned(q), m)) : q; }
-};
 
 template <bool INV, int R>
 __device__ __forceinline__ void ac_butterfly(double2* x, int hs, int step, int rs, const double2* tw) {
@@ -152,15 +158,14 @@ template <bool INV>
 __device__ double2* fft_band(double2* a, double2* b, int lines, int ls, int es, const AcPlan& P,
                              const double2* tw, bool across) {
 	const int n = P.n;
-	int L = INV ? 1 : n;  // block length before (forward) or after (inverse) the stage
+	const Divider by_lines(lines);
 	for (int si = 0; si < P.m; ++si) {
-		const int r = P.r[INV ? P.m - 1 - si : si];
-		if (INV) L *= r;
-		const int h = L / r, tws = n / L, rs = n / r;
+		const int st = INV ? P.m - 1 - si : si;
+		const int r = P.r[st], h = P.h[st], L = r * h, tws = P.tws[st], rs = tws * h;
 		const bool direct = r > 7;
-		const int per = direct ? n : n / r;  // work items of a line
+		const int per = int(P.by_per[st].d);
 		const bool by_line = across || (h < 32 && lines >= 8);
-		const Divider dl(by_line ? lines : per), dh(h), dr(direct ? r : 1);
+		const Divider dl = by_line ? by_lines : P.by_per[st], dh = P.by_h[st], dr = P.by_r[st];
 		for (int q = threadIdx.x; q < lines * per; q += kAcThreads) {
 			const int hi = dl.div(q), lo = q - hi * int(dl.d);
 			const int line = by_line ? lo : hi, w = by_line ? hi : lo;
@@ -198,7 +203,6 @@ __device__ double2* fft_band(double2* a, double2* b, int lines, int ls, int es, 
 			a = b;
 			b = t;
 		}
-		if (!INV) L = h;
 	}
 	return a;
 }
@@ -206,10 +210,11 @@ __device__ double2* fft_band(double2* a, double2* b, int lines, int ls, int es, 
 // Where the forward transform leaves each frequency.
 __device__ void ac_positions(int* pos, const AcPlan& P) {
 	for (int p = threadIdx.x; p < P.n; p += kAcThreads) {
-		int h = P.n, w = 1, f = 0;
+		int rest = p, w = 1, f = 0;
 		for (int s = 0; s < P.m; ++s) {
-			h /= P.r[s];
-			f += ((p / h) % P.r[s]) * w;
+			const int q = P.by_h[s].div(rest);
+			f += q * w;
+			rest -= q * P.h[s];
 			w *= P.r[s];
 		}
 		pos[f] = p;

@@ -104,6 +104,16 @@ __device__ __forceinline__ T nit_lut_map(T z, const typename NitCoef<T>::type* _
 	return fma(fma(fma(k.w, t, k.z), t, k.y), t, k.x);
 }
 
+// q / d for 0 <= q < 2^16 by one multiplication, for a divisor fixed over a loop:
+// m = ceil(2^32 / d), 0 for d = 1.
+struct Divider {
+	unsigned d, m;
+	Divider() = default;
+	__host__ __device__ explicit Divider(int v)
+	    : d(unsigned(v)), m(v == 1 ? 0u : 0xffffffffu / unsigned(v) + 1u) {}
+	__device__ int div(int q) const { return m ? int(__umulhi(unsigned(q), m)) : q; }
+};
+
 // cudaMemcpyAsync that counts the bytes a context moves between host and
 // device (arma_ctx_transfer_bytes).
 inline cudaError_t copy_async(Ctx* c, void* dst, const void* src, size_t bytes,

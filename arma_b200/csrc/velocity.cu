@@ -625,6 +625,61 @@ __device__ double window_fixed(int i, int j, int nx, int ny, double dkx, double 
 	return isfinite(r) ? r : 0.0;
 }
 
+// exp(x) for -708 <= x <= 0: x = (64 m + j) ln 2 / 64 + r with ln 2 / 64 in two
+// parts, |r| <= ln 2 / 128, exp(x) = 2^m 2^(j / 64) (1 + r + .. + r^5 / 120) (the
+// table method of Tang, ACM TOMS 15(2), 1989); within 1 ulp or two.  tab[j] =
+// 2^(j / 64) in shared memory.
+__device__ __forceinline__ double exp_near(double x, const double* tab) {
+	constexpr double kLn2Hi = 2977044471.0 / 4294967296.0;   // ln 2 to 32 bits
+	constexpr double kLn2Lo = 1.90821492927058770002e-10;    // ln 2 - kLn2Hi
+	constexpr double kRound = 6755399441055744.0;            // 1.5 * 2^52
+	const double kd = fma(x, 64.0 / 0.69314718055994530942, kRound);
+	const int k = __double2loint(kd);
+	const double kf = kd - kRound;
+	double r = fma(kf, -kLn2Hi / 64.0, x);
+	r = fma(kf, -kLn2Lo / 64.0, r);
+	double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+	p = fma(r, p, 1.0 / 6.0);
+	p = fma(r, p, 0.5);
+	p = fma(r * r, p, r);
+	const double t = tab[k & 63];
+	const double v = fma(t, p, t);
+	return __hiloint2double(__double2hiint(v) + ((k >> 6) << 20), __double2loint(v));
+}
+
+constexpr int kExpTable = 64;
+__device__ __forceinline__ void make_exp_table(double* tab) {
+	if (threadIdx.x < kExpTable) tab[threadIdx.x] = exp2(double(threadIdx.x) / kExpTable);
+}
+
+// window_fixed for entries where nothing overflows (-350 <= l z <= 0, l finite and
+// positive: no entry of the reference's formula is non-finite there, so no fix
+// applies): with A = exp(l z), B = exp(-l (z + 2 h)) the window is 4 pi (A + B) /
+// (1 + A B), the same quotient as above.  At infinite depth one exponential and no
+// division: 30 FP64 instructions instead of 78 (400 x 128 x 128 FP32 at four
+// depths spent 205 us of the solver's 540 on windows).
+__device__ __noinline__ double window_fixed_call(int i, int j, int nx, int ny, double dkx,
+                                                 double dky, double z, double h) {
+	return window_fixed(i, j, nx, ny, dkx, dky, z, h);
+}
+__device__ __forceinline__ double window_at(int i, int j, int nx, int ny, double dkx, double dky,
+                                            double z, double h, const double* tab) {
+	const double u = dkx * i, v = dky * j;
+	const double s2 = u * u + v * v;
+	const double az = k2Pi * sqrt(s2) * z;
+	// exp(-l z)^2 overflows: the entry is non-finite, 0 away from row and column 0
+	if (az < -360.0 && i > 0 && j > 0) return 0.0;
+	if (s2 > 0.0 && s2 <= DBL_MAX && az <= 0.0 && az >= -350.0) {
+		const double A = exp_near(az, tab);
+		if (h == INFINITY) return k2Pi * 2.0 * A;
+		// -l (z + 2 h), formed as the reference's -2 l h minus l z
+		const double ah = -2.0 * (k2Pi * sqrt(s2)) * h;
+		const double B = exp_near(fmax(ah - az, -708.0), tab);
+		return k2Pi * 2.0 * (A + B) / fma(A, B, 1.0);
+	}
+	return window_fixed_call(i, j, nx, ny, dkx, dky, z, h);
+}
+
 // ---------------------------------------------------------------- 6. finish
 // Re / N with the reference's edge extrapolation (src/velocity/basic_solver.cc:
 // 62-68): column 0 (rows >= 1) from columns 1-2, then row 0 from rows 1-2
@@ -643,6 +698,18 @@ __device__ __forceinline__ double finish_at(int x, int y, int nx, int ny, F f) {
 	if (x == 0 && y > 0 && nx > 2)
 		return interp3(1, y - 1, cur(1, y - 1), 1, y, cur(1, y), 2, y - 1, cur(2, y - 1), 0, y);
 	return f(x, y);
+}
+
+// Row 0 and column 0 of rows [x0, x1) of a plane at `out` (its row 0): by
+// themselves, so that their FP64 interpolation does not run in every warp of the
+// plane's other points.
+template <class T, class F>
+__device__ __forceinline__ void finish_edges(T* out, int x0, int x1, int nx, int ny, F f) {
+	const int rows = x1 - x0, count = rows + (x0 == 0 ? ny - 1 : 0);
+	for (int e = threadIdx.x; e < count; e += blockDim.x) {
+		const int x = e < rows ? x0 + e : 0, y = e < rows ? 0 : e - rows + 1;
+		out[(long long)x * ny + y] = T(finish_at(x, y, nx, ny, f));
+	}
 }
 
 // ---------------------------------------------------------------- 2a. fused
@@ -680,6 +747,10 @@ constexpr int kMaxRadix = 64;
 struct FftPlan {
 	int n, m;
 	int r[kMaxStages];
+	// per forward stage, precomputed: sub-block length h, twiddle stride n / (r
+	// h), root stride n / r (also the butterflies of a line), their divisors
+	int h[kMaxStages], tws[kMaxStages], rs[kMaxStages];
+	Divider by_h[kMaxStages], by_per[kMaxStages];
 };
 
 template <class V>
@@ -693,10 +764,12 @@ __device__ void make_twiddles(V* tw, int n) {
 
 // Frequency held at position p after the forward stages.
 __device__ __forceinline__ int plan_freq(const FftPlan& P, int p) {
-	int h = P.n, w = 1, f = 0;
+	int w = 1, f = 0;
 	for (int s = 0; s < P.m; ++s) {
-		h /= P.r[s];
-		f += ((p / h) % P.r[s]) * w;
+		// digit s: p / h within its block of r h points
+		const int q = P.by_h[s].div(p);
+		f += q * w;
+		p -= q * P.h[s];
 		w *= P.r[s];
 	}
 	return f;
@@ -794,24 +867,17 @@ __device__ __noinline__ void butterfly_any(V* x, int hs, int r, int j, int tws, 
 template <class V, bool INV>
 __device__ void fft_lines(V* a, int nlines, int lstride, int estride, const FftPlan& P,
                           const V* tw, bool lines_fastest, bool rows_padded = false) {
-	const int n = P.n;
+	const Divider by_lines(nlines);
 	for (int si = 0; si < P.m; ++si) {
 		const int s = INV ? P.m - 1 - si : si;
-		int L = n;
-		for (int t = 0; t < s; ++t) L /= P.r[t];
-		const int r = P.r[s], h = L / r, per = (n / L) * h;
-		const int tws = n / L, rs = n / r;
+		const int r = P.r[s], h = P.h[s], L = r * h, per = P.rs[s];
+		const int tws = P.tws[s], rs = P.rs[s];
 		const bool lf = lines_fastest || (rows_padded && h < 32 && nlines >= 8);
+		const Divider dl = lf ? by_lines : P.by_per[s], dh = P.by_h[s];  // (nlines * n < 2^16)
 		for (int q = threadIdx.x; q < nlines * per; q += blockDim.x) {
-			int line, bj;
-			if (lf) {
-				line = q % nlines;
-				bj = q / nlines;
-			} else {
-				line = q / per;
-				bj = q % per;
-			}
-			const int b = bj / h, j = bj % h;
+			const int hi = dl.div(q), lo = q - hi * int(dl.d);
+			const int line = lf ? lo : hi, bj = lf ? hi : lo;
+			const int b = dh.div(bj), j = bj - b * h;
 			V* x = a + line * lstride + (b * L + j) * estride;
 			const int hs = h * estride;
 			switch (r) {
@@ -845,6 +911,9 @@ velocity_fused_kernel(const VelSlice<float>* __restrict__ sl, int nx, int ny, Ff
 	float2* twy = twx + nx;                            // ny
 	int* wix = reinterpret_cast<int*>(twy + ny);       // nx window row indices
 	int* wiy = wix + nx;                               // ny window column indices
+	__shared__ double exp_tab[kExpTable];
+	make_exp_table(exp_tab);
+	const Divider dny(ny);
 	const int s = blockIdx.x;
 	const VelSlice<float> S = sl[s];
 	const int n2 = nx * ny;
@@ -856,7 +925,7 @@ velocity_fused_kernel(const VelSlice<float>* __restrict__ sl, int nx, int ny, Ff
 	{
 		double re, im;
 		solver_input(S, nx, ny, q, re, im);
-		a[(q / ny) * ld + q % ny] = make_float2(float(re), float(im));
+		a[q + dny.div(q)] = make_float2(float(re), float(im));
 	}
 	__syncthreads();
 	fft_lines<float2, false>(a, nx, ld, 1, py, twy, false, true);  // rows
@@ -865,7 +934,7 @@ velocity_fused_kernel(const VelSlice<float>* __restrict__ sl, int nx, int ny, Ff
 	// reloaded per depth; the first depth works on it in place
 	float2* spec = spectra ? spectra + (long long)s * n2 : nullptr;
 	if (spec)
-		for (int q = threadIdx.x; q < n2; q += blockDim.x) spec[q] = a[(q / ny) * ld + q % ny];
+		for (int q = threadIdx.x; q < n2; q += blockDim.x) spec[q] = a[q + dny.div(q)];
 	// wnmax = 1 / min_k per axis; k-grid step ub / (n-1)
 	const double wx = 1.0 / kinfo[s * 4 + 0], wy = 1.0 / kinfo[s * 4 + 1];
 	const double dkx = wx / max(nx - 1, 1), dky = wy / max(ny - 1, 1);
@@ -873,18 +942,22 @@ velocity_fused_kernel(const VelSlice<float>* __restrict__ sl, int nx, int ny, Ff
 	for (int iz = 0; iz < nz; ++iz) {
 		__syncthreads();  // the previous depth's output read a[]
 		for (int q = threadIdx.x; q < n2; q += blockDim.x) {
-			const double w = window_fixed(wix[q / ny], wiy[q % ny], nx, ny, dkx, dky, zs[iz], depth);
-			const int qa = (q / ny) * ld + q % ny;
-			const float2 x = iz == 0 ? a[qa] : spec[q];
-			a[qa] = make_float2(float(x.x * w), float(x.y * w));
+			const int x = dny.div(q), qa = q + x;  // x ld + y
+			const double w =
+			    window_at(wix[x], wiy[q - x * ny], nx, ny, dkx, dky, zs[iz], depth, exp_tab);
+			const float2 v = iz == 0 ? a[qa] : spec[q];
+			a[qa] = make_float2(float(v.x * w), float(v.y * w));
 		}
 		__syncthreads();
 		fft_lines<float2, true>(a, ny, 1, ld, px, twx, true);
 		fft_lines<float2, true>(a, nx, ld, 1, py, twy, false, true);
 		float* out = S.out + (long long)iz * n2;
 		auto f = [&](int r, int c) -> double { return double(a[r * ld + c].x) * inv; };
-		for (int q = threadIdx.x; q < n2; q += blockDim.x)
-			out[q] = float(finish_at(q / ny, q % ny, nx, ny, f));
+		for (int q = threadIdx.x; q < n2; q += blockDim.x) {
+			const int x = dny.div(q);
+			if (x > 0 && q > x * ny) out[q] = float(double(a[q + x].x) * inv);
+		}
+		finish_edges(out, 0, nx, nx, ny, f);
 	}
 }
 
@@ -1121,14 +1194,13 @@ template <int M, int NY> struct RealLd {
 };
 
 // Even part of the window at natural-order frequency (kx, ky):
-// (W(k) + W(-k)) / 2 with W evaluated at the rotated grid indices.  Not
-// inlined: the FP64 window code would otherwise hold registers across the
-// FFT kernel's pairing loop.
-__device__ __noinline__ double window_even(int kx, int ky, int nx, int ny, double dkx, double dky,
-                                           double z, double depth) {
+// (W(k) + W(-k)) / 2 with W evaluated at the rotated grid indices.
+__device__ __forceinline__ double window_even(int kx, int ky, int nx, int ny, double dkx,
+                                              double dky, double z, double depth,
+                                              const double* tab) {
 	const int mx = kx == 0 ? 0 : nx - kx, my = ky == 0 ? 0 : ny - ky;
-	const double w1 = window_fixed(rotate_src(kx, nx), rotate_src(ky, ny), nx, ny, dkx, dky, z, depth);
-	const double w2 = window_fixed(rotate_src(mx, nx), rotate_src(my, ny), nx, ny, dkx, dky, z, depth);
+	const double w1 = window_at(rotate_src(kx, nx), rotate_src(ky, ny), nx, ny, dkx, dky, z, depth, tab);
+	const double w2 = window_at(rotate_src(mx, nx), rotate_src(my, ny), nx, ny, dkx, dky, z, depth, tab);
 	return 0.5 * (w1 + w2);
 }
 
@@ -1202,11 +1274,18 @@ __device__ __forceinline__ void real_input_rows(const VelSlice<float>& S, int NX
 	}
 }
 
+// part: everything for the one depth of a launch (kRealAll); or, with several
+// depths, the spectra of all slices (kRealSpectrum) and then a CTA per slice and
+// depth (kRealDepth), whose last wave is fuller than that of one CTA per slice
+// walking its depths: 400 slices of 128 x 128 at four depths, 296 CTAs at a time,
+// 540 us; split, with the cheaper windows and edges, 37 + 180.
+enum RealPart { kRealAll, kRealSpectrum, kRealDepth };
+
 template <int M, int NY, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 velocity_real_kernel(const VelSlice<float>* __restrict__ sl, const double* __restrict__ kinfo,
-                     const double* __restrict__ zs, int nz, double depth,
-                     float2* __restrict__ spectra) {
+                     const double* __restrict__ zs, double depth, float2* __restrict__ spectra,
+                     int part) {
 	constexpr int NX = 2 * M, LD = RealLd<M, NY>::v;
 	constexpr int L = NX > NY ? NX : NY;  // twiddle table: W_L^j
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1220,79 +1299,77 @@ velocity_real_kernel(const VelSlice<float>* __restrict__ sl, const double* __res
 		sincospi(2.0 * j / L, &sn, &cs);
 		tw[j] = make_float2(float(cs), float(-sn));
 	}
-	// zeta_t of rows 2p and 2p + 1 into z(p, y)
-	real_input_rows<NY, NT, LD>(S, NX, 0, M, A);
-	__syncthreads();
-	lines_fft<NY, false, NT, false>(A, M, LD, 1, tw, L / NY);  // rows
-	__syncthreads();
-	lines_fft<M, false, NT, true>(A, NY, 1, LD, tw, L / M);    // columns
-	__syncthreads();
-	float2* spec = spectra ? spectra + (long long)s * M * NY : nullptr;
-	if (spec) {
-		for (int q = threadIdx.x; q < M * NY; q += NT) spec[q] = A[(q / NY) * LD + q % NY];
-		__syncthreads();  // the pairing pass rewrites A
+	__shared__ double exp_tab[kExpTable];
+	make_exp_table(exp_tab);
+	float2* spec = spectra + (long long)s * M * NY;
+	if (part == kRealDepth) {  // one depth per CTA, from the spectrum
+		for (int q = threadIdx.x; q < M * NY; q += NT) A[(q / NY) * LD + q % NY] = spec[q];
+		__syncthreads();
+	} else {
+		// zeta_t of rows 2p and 2p + 1 into z(p, y)
+		real_input_rows<NY, NT, LD>(S, NX, 0, M, A);
+		__syncthreads();
+		lines_fft<NY, false, NT, false>(A, M, LD, 1, tw, L / NY);  // rows
+		__syncthreads();
+		lines_fft<M, false, NT, true>(A, NY, 1, LD, tw, L / M);    // columns
+		__syncthreads();
+		if (part == kRealSpectrum) {
+			for (int q = threadIdx.x; q < M * NY; q += NT) spec[q] = A[(q / NY) * LD + q % NY];
+			return;
+		}
 	}
+	const int iz = part == kRealDepth ? blockIdx.y : 0;
 	const double wx = 1.0 / kinfo[s * 4 + 0], wy = 1.0 / kinfo[s * 4 + 1];
 	const double dkx = wx / (NX - 1), dky = wy / (NY - 1);
 	const float inv = float(1.0 / double(M * NY));
-	for (int iz = 0; iz < nz; ++iz) {
-		if (iz > 0) {
-			__syncthreads();  // the previous depth's output read A
-			for (int q = threadIdx.x; q < M * NY; q += NT) A[(q / NY) * LD + q % NY] = spec[q];
-			__syncthreads();
+	const double z = zs[iz];
+	auto We = [&](int kx, int ky) {
+		return window_even(kx, ky, NX, NY, dkx, dky, z, depth, exp_tab);
+	};
+	const bool flat = window_flat(NX, NY, dkx, dky, z, depth);
+	const float flat_w = float(window_flat_value());
+	// one thread per pair {(a, b), (-a, -b)}: b in [0, NY/2], a in [0, M),
+	// with b in {0, NY/2} only a <= M/2 (the others are partners);
+	// consecutive threads on consecutive b (one row of A)
+	for (int q = threadIdx.x; q < M * (NY / 2 + 1); q += NT) {
+		const int a = q / (NY / 2 + 1), b = q % (NY / 2 + 1);
+		if ((b == 0 || b == NY / 2) && a > M / 2) continue;
+		const int am = a == 0 ? 0 : M - a, bm = b == 0 ? 0 : NY - b;
+		const float2 z1 = A[a * LD + b], z2 = A[am * LD + bm];
+		// E = (z1 + conj z2) / 2, O = (z1 - conj z2) / 2i
+		const float2 E = make_float2(0.5f * (z1.x + z2.x), 0.5f * (z1.y - z2.y));
+		const float2 O = make_float2(0.5f * (z1.y + z2.y), -0.5f * (z1.x - z2.x));
+		float2 E2, O2;
+		if (flat) {  // S = the constant, D = 0: the same values without the window calls
+			E2 = make_float2(flat_w * E.x, flat_w * E.y);
+			O2 = make_float2(flat_w * O.x, flat_w * O.y);
+		} else {
+			const double wa = We(a, b), wb = We(a + M, b);
+			const float Sv = float(0.5 * (wa + wb)), Dv = float(0.5 * (wa - wb));
+			const float2 w = tw[a * (L / NX)];  // W_nx^a
+			const float2 wO = cmul_tw<false>(O, w), wE = cmul_tw<true>(E, w);
+			E2 = make_float2(Sv * E.x + Dv * wO.x, Sv * E.y + Dv * wO.y);
+			O2 = make_float2(Sv * O.x + Dv * wE.x, Sv * O.y + Dv * wE.y);
 		}
-		const double z = zs[iz];
-		auto We = [&](int kx, int ky) {
-			return window_even(kx, ky, NX, NY, dkx, dky, z, depth);
-		};
-		const bool flat = window_flat(NX, NY, dkx, dky, z, depth);
-		const float flat_w = float(window_flat_value());
-		// one thread per pair {(a, b), (-a, -b)}: b in [0, NY/2], a in [0, M),
-		// with b in {0, NY/2} only a <= M/2 (the others are partners);
-		// consecutive threads on consecutive b (one row of A)
-		for (int q = threadIdx.x; q < M * (NY / 2 + 1); q += NT) {
-			const int a = q / (NY / 2 + 1), b = q % (NY / 2 + 1);
-			if ((b == 0 || b == NY / 2) && a > M / 2) continue;
-			const int am = a == 0 ? 0 : M - a, bm = b == 0 ? 0 : NY - b;
-			const float2 z1 = A[a * LD + b], z2 = A[am * LD + bm];
-			// E = (z1 + conj z2) / 2, O = (z1 - conj z2) / 2i
-			const float2 E = make_float2(0.5f * (z1.x + z2.x), 0.5f * (z1.y - z2.y));
-			const float2 O = make_float2(0.5f * (z1.y + z2.y), -0.5f * (z1.x - z2.x));
-			float2 E2, O2;
-			if (flat) {  // S = the constant, D = 0: the same values without the window calls
-				E2 = make_float2(flat_w * E.x, flat_w * E.y);
-				O2 = make_float2(flat_w * O.x, flat_w * O.y);
-			} else {
-				const double wa = We(a, b), wb = We(a + M, b);
-				const float Sv = float(0.5 * (wa + wb)), Dv = float(0.5 * (wa - wb));
-				const float2 w = tw[a * (L / NX)];  // W_nx^a
-				const float2 wO = cmul_tw<false>(O, w), wE = cmul_tw<true>(E, w);
-				E2 = make_float2(Sv * E.x + Dv * wO.x, Sv * E.y + Dv * wO.y);
-				O2 = make_float2(Sv * O.x + Dv * wE.x, Sv * O.y + Dv * wE.y);
-			}
-			A[a * LD + b] = make_float2(E2.x - O2.y, E2.y + O2.x);     // E' + i O'
-			A[am * LD + bm] = make_float2(E2.x + O2.y, -E2.y + O2.x);  // conj E' + i conj O'
-		}
-		__syncthreads();
-		lines_fft<M, true, NT, true>(A, NY, 1, LD, tw, L / M);    // columns
-		__syncthreads();
-		lines_fft<NY, true, NT, false>(A, M, LD, 1, tw, L / NY);  // rows
-		__syncthreads();
-		float* out = S.out + (long long)iz * n2;
-		auto f = [&](int r, int c) -> double {
-			const float2 v = A[(r >> 1) * LD + c];
-			return double((r & 1) ? v.y : v.x) * double(inv);
-		};
-		for (int q = threadIdx.x; q < n2; q += NT) {
-			const int x = q / NY, y = q % NY;
-			if (x > 0 && y > 0) {
-				const float2 v = A[(x >> 1) * LD + y];
-				out[q] = ((x & 1) ? v.y : v.x) * inv;
-			} else {
-				out[q] = float(finish_at(x, y, NX, NY, f));
-			}
-		}
+		A[a * LD + b] = make_float2(E2.x - O2.y, E2.y + O2.x);     // E' + i O'
+		A[am * LD + bm] = make_float2(E2.x + O2.y, -E2.y + O2.x);  // conj E' + i conj O'
 	}
+	__syncthreads();
+	lines_fft<M, true, NT, true>(A, NY, 1, LD, tw, L / M);    // columns
+	__syncthreads();
+	lines_fft<NY, true, NT, false>(A, M, LD, 1, tw, L / NY);  // rows
+	__syncthreads();
+	float* out = S.out + (long long)iz * n2;
+	auto f = [&](int r, int c) -> double {
+		const float2 v = A[(r >> 1) * LD + c];
+		return double((r & 1) ? v.y : v.x) * double(inv);
+	};
+	for (int q = threadIdx.x; q < n2; q += NT) {
+		const int x = q / NY, y = q % NY;
+		const float2 v = A[(x >> 1) * LD + y];
+		if (x > 0 && y > 0) out[q] = ((x & 1) ? v.y : v.x) * inv;
+	}
+	finish_edges(out, 0, NX, NX, NY, f);
 }
 
 // The instantiated (M, NY) shapes: M in {16, 32, 64, 128}, NY in {16..256},
@@ -1312,8 +1389,17 @@ bool launch_real_shape(Ctx* c, const VelSlice<float>* d_sl, int ns, int nx, int 
 		const size_t smem = sizeof(float2) * (size_t(M) * RealLd<M, NY>::v + L);
 		ARMA_CUDA_TRY(cudaFuncSetAttribute(velocity_real_kernel<M, NY, NT>,
 		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-		velocity_real_kernel<M, NY, NT><<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, nz, depth,
-		                                                              spectra);
+		auto kernel = velocity_real_kernel<M, NY, NT>;
+		if (nz == 1) {
+			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealAll);
+		} else {
+			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealSpectrum);
+			ARMA_CUDA_TRY(cudaGetLastError());
+			c->launches += 1;
+			for (int z0 = 0; z0 < nz; z0 += 65535)
+				kernel<<<dim3(ns, std::min(nz - z0, 65535)), NT, smem, c->stream>>>(
+				    d_sl, d_k, d_z, depth, spectra, kRealDepth);
+		}
 		return true;
 	}
 }
@@ -1367,6 +1453,8 @@ velocity_real2_kernel(const VelSlice<float>* __restrict__ sl, const double* __re
 		sincospi(2.0 * j / L, &sn, &cs);
 		tw[j] = make_float2(float(cs), float(-sn));
 	}
+	__shared__ double exp_tab[kExpTable];
+	make_exp_table(exp_tab);
 	real_input_rows<NY, NT, LD>(S, NX, rank * H, H, A);
 	__syncthreads();
 	lines_fft<NY, false, NT, false>(A, H, LD, 1, tw, L / NY);  // rows
@@ -1411,8 +1499,8 @@ velocity_real2_kernel(const VelSlice<float>* __restrict__ sl, const double* __re
 				E2 = make_float2(flat_w * E.x, flat_w * E.y);
 				O2 = make_float2(flat_w * O.x, flat_w * O.y);
 			} else {
-				const double wa = window_even(a, b, NX, NY, dkx, dky, z, depth);
-				const double wb = window_even(a + M, b, NX, NY, dkx, dky, z, depth);
+				const double wa = window_even(a, b, NX, NY, dkx, dky, z, depth, exp_tab);
+				const double wb = window_even(a + M, b, NX, NY, dkx, dky, z, depth, exp_tab);
 				const float Sv = float(0.5 * (wa + wb)), Dv = float(0.5 * (wa - wb));
 				const float2 w = tw[a * (L / NX)];  // W_nx^a
 				const float2 wO = cmul_tw<false>(O, w), wE = cmul_tw<true>(E, w);
@@ -1444,14 +1532,10 @@ velocity_real2_kernel(const VelSlice<float>* __restrict__ sl, const double* __re
 		};
 		for (int q = threadIdx.x; q < 2 * H * NY; q += NT) {
 			const int x = rank * 2 * H + q / NY, y = q % NY;
-			float* o = out + (long long)x * NY + y;
-			if (x > 0 && y > 0) {
-				const float2 v = A[((x >> 1) - rank * H) * LD + y];
-				*o = ((x & 1) ? v.y : v.x) * inv;
-			} else {
-				*o = float(finish_at(x, y, NX, NY, f));
-			}
+			const float2 v = A[((x >> 1) - rank * H) * LD + y];
+			if (x > 0 && y > 0) out[(long long)x * NY + y] = ((x & 1) ? v.y : v.x) * inv;
 		}
+		finish_edges(out, rank * 2 * H, (rank + 1) * 2 * H, NX, NY, f);
 	}
 	cl.sync();  // the other CTA may still read this one's shared memory
 }
@@ -1499,13 +1583,27 @@ bool make_plan(int n, FftPlan* P) {
 	for (int f = 3; rest > 1 && f <= kMaxRadix; f += 2)
 		while (rest % f == 0)
 			if (!push(f)) return false;
+	int L = n;
+	for (int s = 0; s < P->m; ++s) {
+		P->h[s] = L / P->r[s];
+		P->tws[s] = n / L;
+		P->rs[s] = n / P->r[s];
+		P->by_h[s] = Divider(P->h[s]);
+		P->by_per[s] = Divider(P->rs[s]);
+		L = P->h[s];
+	}
 	return rest == 1;
 }
 
 // ---------------------------------------------------------------- 2b. banded
 // Slices larger than the fused kernel's shared memory go through three
 // banded passes with the spectra in global memory (A: one per slice, B: one
-// per slice and depth), each band sized to ~64 KB of shared memory:
+// per slice and depth), each band at most ~64 KB of shared memory.  The two
+// passes that read spectra are bounded to three CTAs' registers (their radix
+// branches otherwise take more): 48 slices of 200 x 100 FP64 at three depths,
+// vel_cols 90 -> 83 us, vel_rows_inv 45 -> 39 by that bound (the call's kernels took
+// 321 us before the divisions by constants and the window's own exponential, 191
+// with them):
 //   vel_rows_fwd   R rows of zeta_t, forward row FFTs        -> A
 //   vel_cols       CB columns of A, forward column FFTs, then per depth the
 //                  window product and inverse column FFTs     -> B
@@ -1524,20 +1622,21 @@ vel_rows_fwd(const VelSlice<T>* __restrict__ sl, int nx, int ny, int R, FftPlan 
 	const VelSlice<T> S = sl[blockIdx.y];
 	const int r0 = blockIdx.x * R, rows = min(R, nx - r0);
 	make_twiddles(tw, ny);
+	const Divider dny(ny);
 	for (int q = threadIdx.x; q < rows * ny; q += blockDim.x)
 	{
 		double re, im;
 		solver_input(S, nx, ny, (long long)r0 * ny + q, re, im);
-		a[(q / ny) * ld + q % ny] = cpx(T(re), T(im));
+		a[q + dny.div(q)] = cpx(T(re), T(im));
 	}
 	__syncthreads();
 	fft_lines<V, false>(a, rows, ld, 1, py, tw, false, true);
 	V* dst = A + blockIdx.y * n2 + (long long)r0 * ny;
-	for (int q = threadIdx.x; q < rows * ny; q += blockDim.x) dst[q] = a[(q / ny) * ld + q % ny];
+	for (int q = threadIdx.x; q < rows * ny; q += blockDim.x) dst[q] = a[q + dny.div(q)];
 }
 
 template <class T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 vel_cols(int nx, int ny, FftPlan px, FftPlan py, int CB, const double* __restrict__ kinfo,
          const double* __restrict__ zs, int nz, double depth,
          const typename C2<T>::type* __restrict__ A, typename C2<T>::type* __restrict__ B) {
@@ -1547,37 +1646,45 @@ vel_cols(int nx, int ny, FftPlan px, FftPlan py, int CB, const double* __restric
 	V* work = nz > 1 ? spec + nx * CB : spec;  // one buffer when there is one depth
 	V* tw = spec + (nz > 1 ? 2 : 1) * nx * CB;  // nx
 	int* wix = reinterpret_cast<int*>(tw + nx);  // nx window row indices
-	int* wiy = wix + nx;                         // ny window column indices
+	int* wiy = wix + nx;                         // CB window column indices
+	__shared__ double exp_tab[kExpTable];
+	make_exp_table(exp_tab);
 	const long long n2 = (long long)nx * ny;
 	const int s = blockIdx.y, c0 = blockIdx.x * CB, cols = min(CB, ny - c0);
 	make_twiddles(tw, nx);
 	make_window_index(wix, px);
-	make_window_index(wiy, py);
+	for (int p = threadIdx.x; p < cols; p += blockDim.x) wiy[p] = rotate_src(plan_freq(py, c0 + p), ny);
+	const Divider dc(cols);
 	const V* src = A + s * n2 + c0;
-	for (int q = threadIdx.x; q < nx * cols; q += blockDim.x)
-		spec[q] = src[(long long)(q / cols) * ny + q % cols];
+	for (int q = threadIdx.x; q < nx * cols; q += blockDim.x) {
+		const int x = dc.div(q);
+		spec[q] = src[(long long)x * ny + q - x * cols];
+	}
 	__syncthreads();
 	fft_lines<V, false>(spec, cols, 1, cols, px, tw, true);
 	const double wx = 1.0 / kinfo[s * 4 + 0], wy = 1.0 / kinfo[s * 4 + 1];
 	const double dkx = wx / max(nx - 1, 1), dky = wy / max(ny - 1, 1);
 	for (int iz = 0; iz < nz; ++iz) {
 		for (int q = threadIdx.x; q < nx * cols; q += blockDim.x) {
-			const double w = window_fixed(wix[q / cols], wiy[c0 + q % cols], nx, ny, dkx, dky,
-			                              zs[iz], depth);
-			const V x = spec[q];
-			work[q] = cpx(T(x.x * w), T(x.y * w));
+			const int x = dc.div(q);
+			const double w = window_at(wix[x], wiy[q - x * cols], nx, ny, dkx, dky, zs[iz], depth,
+			                           exp_tab);
+			const V v = spec[q];
+			work[q] = cpx(T(v.x * w), T(v.y * w));
 		}
 		__syncthreads();
 		fft_lines<V, true>(work, cols, 1, cols, px, tw, true);
 		V* dst = B + ((long long)s * nz + iz) * n2 + c0;
-		for (int q = threadIdx.x; q < nx * cols; q += blockDim.x)
-			dst[(long long)(q / cols) * ny + q % cols] = work[q];
+		for (int q = threadIdx.x; q < nx * cols; q += blockDim.x) {
+			const int x = dc.div(q);
+			dst[(long long)x * ny + q - x * cols] = work[q];
+		}
 		__syncthreads();
 	}
 }
 
 template <class T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 vel_rows_inv(const VelSlice<T>* __restrict__ sl, int nx, int ny, int R, int nz, FftPlan py,
              const typename C2<T>::type* __restrict__ B) {
 	using V = typename C2<T>::type;
@@ -1590,17 +1697,22 @@ vel_rows_inv(const VelSlice<T>* __restrict__ sl, int nx, int ny, int R, int nz, 
 	const int r0 = blockIdx.x * R, rows = min(R, nx - r0);
 	make_twiddles(tw, ny);
 	const V* src = B + arr * n2;
+	const Divider dny(ny);
 	for (int q = threadIdx.x; q < (rows + 1) * ny; q += blockDim.x) {
-		const int row = r0 - 1 + q / ny;
-		a[(q / ny) * ld + q % ny] = row >= 0 ? src[(long long)row * ny + q % ny] : cpx(T(0), T(0));
+		const int i = dny.div(q), row = r0 - 1 + i;
+		a[q + i] = row >= 0 ? src[(long long)(r0 - 1) * ny + q] : cpx(T(0), T(0));
 	}
 	__syncthreads();
 	fft_lines<V, true>(a, rows + 1, ld, 1, py, tw, false, true);
 	const double inv = 1.0 / double(n2);
 	auto f = [&](int x, int y) -> double { return double(a[(x - r0 + 1) * ld + y].x) * inv; };
-	T* out = sl[arr / nz].out + (arr % nz) * n2 + (long long)r0 * ny;
-	for (int q = threadIdx.x; q < rows * ny; q += blockDim.x)
-		out[q] = T(finish_at(r0 + q / ny, q % ny, nx, ny, f));
+	T* out = sl[arr / nz].out + (arr % nz) * n2;
+	for (int q = threadIdx.x; q < rows * ny; q += blockDim.x) {
+		const int i = dny.div(q);
+		if (r0 + i > 0 && q > i * ny)
+			out[(long long)r0 * ny + q] = T(double(a[q + i + ld].x) * inv);
+	}
+	finish_edges(out, r0, r0 + rows, nx, ny, f);
 }
 
 // The banded path for one pass of slices.
@@ -1612,12 +1724,15 @@ void velocity_general(Ctx* c, const VelSlice<T>* d_sl, int ns, int nx, int ny, c
 	const long long n2 = (long long)nx * ny;
 	const int budget = int((64 << 10) / sizeof(V));  // elements of one 64 KB band
 	const int R = std::min(nx, std::max(4, budget / ny));
-	const int CB = std::min(ny, std::max(1, budget / nx));
+	// columns of half a band: 48 slices of 200 x 100 FP64 at three depths take
+	// 81 us, 90 with a quarter and 121 with an eighth (more CTAs, shorter runs of
+	// consecutive points in each row)
+	const int CB = std::min(ny, std::max(1, budget / 2 / nx));
 	V* A = static_cast<V*>(scratch_take(c, sizeof(V) * n2 * ns));
 	V* B = static_cast<V*>(scratch_take(c, sizeof(V) * n2 * ns * nz));
 	const size_t s1 = sizeof(V) * (size_t(R) * (ny + 1) + ny);
 	const size_t s2 = sizeof(V) * ((nz > 1 ? 2 : 1) * size_t(nx) * CB + nx) +
-	                  sizeof(int) * (size_t(nx) + ny);
+	                  sizeof(int) * (size_t(nx) + CB);
 	const size_t s3 = sizeof(V) * (size_t(R + 1) * (ny + 1) + ny);
 	ARMA_CUDA_TRY(cudaFuncSetAttribute(vel_rows_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                   int(s1)));
