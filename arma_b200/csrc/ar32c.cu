@@ -30,7 +30,9 @@
 // The coefficients are carried as hi + lo float pairs (rounding phi to one
 // float perturbs a high-gain recursion far more than FP32 summation does):
 // each (k,i) row of taps feeds two FP32 FMA chains over one register window,
-// continued across the rows of one k plane, and the plane totals are combined
+// the two of an output side by side in one packed FMA (fma.rn.f32x2, each half
+// rounded as fmaf: half the instructions), continued across the rows of one k
+// plane, and the plane totals are combined
 // with Kahan compensation (per row, the compensation cost 7 % more time for
 // 0.2-1.2e-6 less RMS error).  H is applied in plain FP32, one FMA chain per
 // output over up to three rows of H (up to 96 taps), the at most six chain
@@ -41,9 +43,20 @@
 // 5 %).  Tiles are handed out through a global ticket
 // counter in dependency order, so a CTA only ever waits on tiles that are
 // already owned by running CTAs.
+//
+// Bound by the issue slots and latencies of 12 compute warps per SM (with one
+// FMA per chain: FMA pipe 47 % busy, issue 66 %, shared-memory loads half).
+// Packed FMAs, one copy of the tap loop for all k, 16-byte accesses of noise, S
+// and results, and the H units numbered so that neighbouring lanes read the same
+// rows of H: the batch of 256 surfaces 51.7 -> 48.2 ms, 512 x 256 x 256 alone
+// 5.20 -> 5.06, 64 x 32 x 32 241 -> 217 us.  Without the packed FMAs the batch
+// took 52.4 ms, with the Kahan steps packed too 49.5; two rows of taps at once
+// cost 4 % (the code of several tap counts on an SM outgrows its instruction
+// cache).
 #include <algorithm>
 #include <climits>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
@@ -95,6 +108,25 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
 	const float t = s + y;
 	c = (t - s) - y;
 	s = t;
+}
+
+// a pair of floats in one 64-bit register pair
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+	unsigned long long v;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+	return v;
+}
+
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+	float2 r;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+	return r;
+}
+
+// (c.x + a.x b.x, c.y + a.y b.y), each half rounded as fmaf
+__device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a,
+                                     unsigned long long b) {
+	asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
 __device__ __forceinline__ void cp_async16(float* dst_smem, const float* src) {
@@ -172,19 +204,34 @@ __device__ bool wait_flags(const int* f0, const int* f1, const int* f2, int need
 // 3 and 4 blocks of R x R taps (the first block of each a triangle), so the
 // strips are paired (3, 0) and (2, 1): either pair costs two triangles and
 // three full blocks per row of H.  A unit is one strip pair of one output row
-// over at most HCH consecutive rows of H; units are numbered pair-major, then
-// by row, then by dx chunk, so row x's units start at HPAIR * pair +
-// h_rowbase(x).  Unit u writes its partial (strip X in slots 0..R-1, strip Y
-// in R..2R-1), one plain FP32 FMA chain per output, to part[u * PS ..]; the
-// partials of an output are Kahan-added afterwards.  Lanes of one warp work
-// on different rows of H at once: H rows are HS floats apart in shared memory
-// so that their 16-byte loads fall in different banks.  The unit is inlined
-// into every tap-count instantiation of compute_tile: as a call, the registers
-// the caller keeps across it spilled, and the filter ran 7 % slower.
-__device__ __forceinline__ int h_rowbase(int x) {
-	// sum over x' < x of ceil((x'+1) / HCH), for HCH = 3
-	const int q = x / 3, r = x % 3;
-	return x + 3 * q * (q - 1) / 2 + r * q;
+// over at most HCH consecutive rows of H; units are numbered pair-major, then by
+// chunk c of HCH rows of H, then by output row (chunk c has the rows x >= HCH c),
+// so neighbouring lanes read the same row of H and rows of S that are SW floats
+// apart, whose 16-byte loads fall in different banks.  Unit u writes its partial
+// (strip X in slots 0..R-1, strip Y in R..2R-1), one plain FP32 FMA chain per
+// output, to part[u * PS ..]; the partials of an output are Kahan-added
+// afterwards.  The unit is inlined into every tap-count instantiation of
+// compute_tile: as a call, the registers the caller keeps across it spilled, and
+// the filter ran 7 % slower; one copy for all of them, between switches over the
+// tap count, ran 2 to 8 % slower.
+// h_start: the first unit of chunk c within its pair.
+__device__ __forceinline__ int h_start(int c) { return TX * c - HCH * c * (c - 1) / 2; }
+
+// Unit u of the numbering: its strip pair, output row and rows of H.
+struct HUnit {
+	int pair, x, dx0, dx1;
+};
+
+__device__ __forceinline__ HUnit h_unit_of(int u) {
+	HUnit h;
+	h.pair = u >= HPAIR ? 1 : 0;
+	const int v = u - h.pair * HPAIR;
+	int c = 0;
+	while (h_start(c + 1) <= v) ++c;
+	h.x = HCH * c + v - h_start(c);
+	h.dx0 = HCH * c;
+	h.dx1 = min(h.dx0 + HCH, h.x + 1);
+	return h;
 }
 
 __device__ __forceinline__ void load_row(float* d, const float* s, int n4) {
@@ -210,13 +257,9 @@ __device__ __forceinline__ void h_block(float* acc, const float* src, const floa
 	}
 }
 
-__device__ __forceinline__ void h_unit(const float* ss, const float* sh, int u, float* part) {
-	const int pair = u >= HPAIR ? 1 : 0;
-	const int v = u - pair * HPAIR;
-	int x = 0;
-	while (x + 1 < TX && h_rowbase(x + 1) <= v) ++x;
-	const int dx0 = HCH * (v - h_rowbase(x));
-	const int dx1 = min(dx0 + HCH, x + 1);
+__device__ __forceinline__ void h_unit(const float* ss, const float* sh, const HUnit& h, int u,
+                                       float* part) {
+	const int pair = h.pair, x = h.x, dx0 = h.dx0, dx1 = h.dx1;
 	const int yx = pair ? 2 * R : 3 * R;  // first column of strip X
 	const int yy = pair ? R : 0;          // first column of strip Y
 	const int w3 = pair ? 0 : 2 * R;      // sources of the third block
@@ -270,7 +313,7 @@ __device__ __forceinline__ void h_unit(const float* ss, const float* sh, int u, 
 // Layout of a tile's shared memory (floats).
 struct Layout {
 	int hx, slot_sz, slots;   // halo rows, floats per ring slot, ring slots
-	int taps;                 // floats of one part of the coefficients (rows of PYP)
+	int taps;                 // coefficients (rows of PYP)
 	int pyp;
 };
 
@@ -332,6 +375,7 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 		if (t >= tk.nt || done < t - 1) {
 			++idle;  // the compute warps are at work: they end every slice
 			if (idle > 64 * kSpinLimit) break;
+			__nanosleep(100);
 			continue;
 		}
 		float* cur = ring + (t % slots) * slot_sz;
@@ -407,14 +451,18 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 	const long long sst = (long long)tk.nx * tk.ny;
 
 	float* ring = smem;                          // slots
-	float* sphi = ring + slots * slot_sz;        // hi
-	float* slo = sphi + L.taps;                  // lo
-	float* sh_h = slo + L.taps;                  // TX*HS
+	float* sphi = ring + slots * slot_sz;        // (hi, lo) pairs
+	float* sh_h = sphi + 2 * L.taps;             // TX*HS
 	float* ss = sh_h + TX * HS;                  // TX*SW
 	float* part = ss + TX * SW;                  // HUNITS*PS: H-unit partials
 	float* comb = part;                          // GROUP*R: group 1 partials (before H)
 	const int gx = x0 + xl;
 
+	bool all_lo = true;  // no row skips its lo chain
+	for (int q = 0; q < pt * px; ++q) all_lo = all_lo && s_lo[q];
+	const HUnit hu = h_unit_of(min(tid, HUNITS - 1));  // found once, not per slice
+	// 16-byte pieces of the tile's rows in global memory
+	const bool vec = tk.ny % 4 == 0 && (reinterpret_cast<uintptr_t>(tk.zeta) & 15) == 0;
 	int st = tk.t0 % slots;  // slot of slice t
 	for (int t = tk.t0; t < tk.nt; ++t, st = st + 1 == slots ? 0 : st + 1) {
 		float* cur = ring + st * slot_sz;
@@ -423,100 +471,126 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 		// earlier kernel), group 1 from zero
 		float s[R], c[R];
 #pragma unroll
-		for (int r = 0; r < R; ++r) {
-			const int gy = y0 + yl0 + r;
-			s[r] = (grp == 0 && gx < tk.nx && gy < tk.ny) ? zt[(long long)gx * tk.ny + gy] : 0.0f;
-			c[r] = 0.0f;
-		}
-		// One (k, i) row of taps at a time, rows alternating between the two
-		// groups: the hi and lo coefficient parts are applied as two FP32 FMA
-		// chains over the same register window, each chain running across the
-		// rows of the k plane; the plane total is Kahan-added to the running
-		// sum.
-		auto accumulate_rows = [&](const float* slot, int k) {
-			const float* prow = sphi + (k * px) * PYP;
-			const float* lrow = slo + (k * px) * PYP;
-			float pk[R], qk[R];
+		for (int r = 0; r < R; ++r) s[r] = c[r] = 0.0f;
+		if (grp == 0 && gx < tk.nx) {
+			const float* zn = zt + (long long)gx * tk.ny + y0 + yl0;
+			if (vec) {
 #pragma unroll
-			for (int r = 0; r < R; ++r) { pk[r] = 0.0f; qk[r] = 0.0f; }
-			for (int i = (k * px + grp) & 1; i < px; i += 2) {
-				const float* zr = slot + (xl + hx - i) * W + yl0;
-				float win[R + LH];
-#pragma unroll
-				for (int q = 0; q < (R + LH) / 4; ++q) {
-					const float4 v = reinterpret_cast<const float4*>(zr)[q];
-					win[4 * q] = v.x;
-					win[4 * q + 1] = v.y;
-					win[4 * q + 2] = v.z;
-					win[4 * q + 3] = v.w;
-				}
-				float ph[PYP];
-#pragma unroll
-				for (int q = 0; q < PYP / 4; ++q) {
-					const float4 v = reinterpret_cast<const float4*>(prow + i * PYP)[q];
-					ph[4 * q] = v.x;
-					ph[4 * q + 1] = v.y;
-					ph[4 * q + 2] = v.z;
-					ph[4 * q + 3] = v.w;
-				}
-				if (s_lo[k * px + i]) {  // warp-uniform: every thread handles this row
-					float pl[PYP];
-#pragma unroll
-					for (int q = 0; q < PYP / 4; ++q) {
-						const float4 u = reinterpret_cast<const float4*>(lrow + i * PYP)[q];
-						pl[4 * q] = u.x;
-						pl[4 * q + 1] = u.y;
-						pl[4 * q + 2] = u.z;
-						pl[4 * q + 3] = u.w;
+				for (int q = 0; q < R / 4; ++q)
+					if (y0 + yl0 + 4 * q < tk.ny) {
+						const float4 v = reinterpret_cast<const float4*>(zn)[q];
+						s[4 * q] = v.x;
+						s[4 * q + 1] = v.y;
+						s[4 * q + 2] = v.z;
+						s[4 * q + 3] = v.w;
 					}
+			} else {
 #pragma unroll
-					for (int r = 0; r < R; ++r) {
+				for (int r = 0; r < R; ++r)
+					if (y0 + yl0 + r < tk.ny) s[r] = zn[r];
+			}
+		}
+		// 1. the planes of slices t-1, t-2, ..; 2./3. slot t cleared, the
+		// neighbours' slice t published and its halo loaded, plane 0
+		const int np = min(pt - 1, t);
+		for (int m = 0, sk = st; m <= np; ++m) {
+			const bool last = m == np;
+			const int k = last ? 0 : m + 1;
+			if (last) {
+				bar_sync(BAR_HALO + (t & 1), NTHREADS);
+				sk = st;
+			} else {
+				sk = sk == 0 ? slots - 1 : sk - 1;
+			}
+			// One (k, i) row of taps at a time, rows alternating between the two
+			// groups: the chains of the hi and lo parts run across the rows of the
+			// plane, whose total is Kahan-added to the running sum.
+			const float* zb = ring + sk * slot_sz + (xl + hx) * W + yl0;
+			const float* prow = sphi + (k * px) * 2 * PYP;
+			unsigned long long pq[R];
 #pragma unroll
-						for (int j = 0; j < PY; ++j) {
-							pk[r] = fmaf(ph[j], win[LH + r - j], pk[r]);
-							qk[r] = fmaf(pl[j], win[LH + r - j], qk[r]);
+			for (int r = 0; r < R; ++r) pq[r] = 0ull;
+			auto rows = [&](auto every) {
+#pragma unroll 1
+				for (int i = (k * px + grp) & 1; i < px; i += 2) {
+					const float* zr = zb - i * W;
+					float win[R + LH];
+#pragma unroll
+					for (int q = 0; q < (R + LH) / 4; ++q) {
+						const float4 v = reinterpret_cast<const float4*>(zr)[q];
+						win[4 * q] = v.x;
+						win[4 * q + 1] = v.y;
+						win[4 * q + 2] = v.z;
+						win[4 * q + 3] = v.w;
+					}
+					unsigned long long ph[PYP];
+#pragma unroll
+					for (int q = 0; q < PYP / 2; ++q) {
+						const ulonglong2 v = reinterpret_cast<const ulonglong2*>(prow + i * 2 * PYP)[q];
+						ph[2 * q] = v.x;
+						ph[2 * q + 1] = v.y;
+					}
+					if (every.value || s_lo[k * px + i]) {  // warp-uniform
+						// by element of the window, last first: taps ascending per output
+#pragma unroll
+						for (int q = R + PY - 2; q >= 0; --q) {
+							const float w = win[LH - PY + 1 + q];
+							const unsigned long long ww = pack2(w, w);
+#pragma unroll
+							for (int r = 0; r < R; ++r) {
+								const int j = r - q + PY - 1;
+								if (j >= 0 && j < PY) fma2(pq[r], ph[j], ww);
+							}
+						}
+					} else {
+#pragma unroll
+						for (int r = 0; r < R; ++r) {
+							float2 p = unpack2(pq[r]);
+#pragma unroll
+							for (int j = 0; j < PY; ++j)
+								p.x = fmaf(unpack2(ph[j]).x, win[LH + r - j], p.x);
+							pq[r] = pack2(p.x, p.y);
 						}
 					}
-				} else {
-#pragma unroll
-					for (int r = 0; r < R; ++r) {
-#pragma unroll
-						for (int j = 0; j < PY; ++j) pk[r] = fmaf(ph[j], win[LH + r - j], pk[r]);
-					}
 				}
-			}
+			};
+			if (all_lo) rows(std::true_type{}); else rows(std::false_type{});
 #pragma unroll
-			for (int r = 0; r < R; ++r) kahan_add(s[r], c[r], pk[r] + qk[r]);
-		};
-
-		// 1. previous slices
-		for (int k = 1, sk = st; k < pt && k <= t; ++k) {
-			sk = sk == 0 ? slots - 1 : sk - 1;
-			accumulate_rows(ring + sk * slot_sz, k);
+			for (int r = 0; r < R; ++r) {
+				const float2 p = unpack2(pq[r]);
+				kahan_add(s[r], c[r], p.x + p.y);
+			}
 		}
-
-		// 2./3. slot t cleared, neighbours' slice t published, halo loaded
-		bar_sync(BAR_HALO + (t & 1), NTHREADS);
-		accumulate_rows(cur, 0);
 
 		// 4. S = noise + all terms outside the unknown in-tile part
 		if (grp == 1) {
 #pragma unroll
-			for (int r = 0; r < R; ++r) comb[lt * R + r] = s[r] - c[r];
+			for (int q = 0; q < R / 4; ++q)
+				reinterpret_cast<float4*>(comb)[q * GROUP + lt] =
+				    make_float4(s[4 * q] - c[4 * q], s[4 * q + 1] - c[4 * q + 1],
+				                s[4 * q + 2] - c[4 * q + 2], s[4 * q + 3] - c[4 * q + 3]);
 		}
 		bar_sync(BAR_COMP, NCOMP);
 		if (grp == 0) {
 #pragma unroll
-			for (int r = 0; r < R; ++r) {
-				const int gy = y0 + yl0 + r;
-				const bool valid = gx < tk.nx && gy < tk.ny;
-				ss[xl * SW + SPAD + yl0 + r] = valid ? (s[r] + (comb[lt * R + r] - c[r])) : 0.0f;
+			for (int q = 0; q < R / 4; ++q) {
+				const float4 v = reinterpret_cast<const float4*>(comb)[q * GROUP + lt];
+				const float g1[4] = {v.x, v.y, v.z, v.w};
+				float o[4];
+#pragma unroll
+				for (int e = 0; e < 4; ++e) {
+					const int r = 4 * q + e;
+					const bool valid = gx < tk.nx && y0 + yl0 + r < tk.ny;
+					o[e] = valid ? (s[r] + (g1[e] - c[r])) : 0.0f;
+				}
+				reinterpret_cast<float4*>(ss + xl * SW + SPAD + yl0)[q] =
+				    make_float4(o[0], o[1], o[2], o[3]);
 			}
 		}
 		bar_sync(BAR_COMP, NCOMP);
 
 		//    zeta = H * S over the quarter plane of the tile, in work units
-		if (tid < HUNITS) h_unit(ss, sh_h, tid, part);
+		if (tid < HUNITS) h_unit(ss, sh_h, hu, tid, part);
 
 		// 5. sum each output's unit partials (Kahan, in dx order), store the
 		//    solved slice; the halo warp publishes it
@@ -526,7 +600,7 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 			const int ox = tid / (2 * STRIPS);
 			const int ostrip = (tid / 2) % STRIPS;
 			const int oy0 = ostrip * R + (tid % 2) * 4;
-			const int opart = (ostrip == 0 || ostrip == 3 ? 0 : HPAIR) + h_rowbase(ox);
+			const int opart = (ostrip == 0 || ostrip == 3 ? 0 : HPAIR) + ox;
 			const int oslot = (ostrip >= 2 ? 0 : R) + (tid % 2) * 4;
 			const int ogx = x0 + ox;
 			float a[4], ac[4];
@@ -534,22 +608,26 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 			for (int e = 0; e < 4; ++e) { a[e] = 0.0f; ac[e] = 0.0f; }
 			const int nch = ox / HCH + 1;
 			for (int ch = 0; ch < nch; ++ch) {
-				const float4 v = *reinterpret_cast<const float4*>(part + (opart + ch) * PS + oslot);
+				const float4 v = *reinterpret_cast<const float4*>(part + (opart + h_start(ch) - HCH * ch) * PS + oslot);
 				kahan_add(a[0], ac[0], v.x);
 				kahan_add(a[1], ac[1], v.y);
 				kahan_add(a[2], ac[2], v.z);
 				kahan_add(a[3], ac[3], v.w);
 			}
-			float* own = cur + hx * W + LH + ox * W + oy0;
 #pragma unroll
-			for (int e = 0; e < 4; ++e) own[e] = a[e] - ac[e];
+			for (int e = 0; e < 4; ++e) a[e] -= ac[e];
+			const float4 z4 = make_float4(a[0], a[1], a[2], a[3]);
+			*reinterpret_cast<float4*>(cur + (hx + ox) * W + LH + oy0) = z4;
 			bar_sync(BAR_COMP, NCOMP);  // slice t in the ring for every compute thread
 			// (released before this slice's global stores: it waits for none)
 			if (tid == 0) st_release_cta(&sh->done, t + 1);
+			float* zo = zt + (long long)ogx * tk.ny + y0 + oy0;
+			if (ogx < tk.nx && vec) {
+				if (y0 + oy0 < tk.ny) *reinterpret_cast<float4*>(zo) = z4;
+			} else if (ogx < tk.nx) {
 #pragma unroll
-			for (int e = 0; e < 4; ++e) {
-				const int gy = y0 + oy0 + e;
-				if (ogx < tk.nx && gy < tk.ny) zt[(long long)ogx * tk.ny + gy] = a[e] - ac[e];
+				for (int e = 0; e < 4; ++e)
+					if (y0 + oy0 + e < tk.ny) zo[e] = a[e];
 			}
 		}
 		// the barrier's previous round is over once the publication warp has
@@ -573,14 +651,13 @@ __device__ __noinline__ void stage_tile(const Task& tk, int bx, int by, const La
 	const long long sst = (long long)tk.nx * tk.ny;
 	float* ring = smem;
 	float* sphi = ring + L.slots * L.slot_sz;
-	float* slo = sphi + L.taps;
-	float* sh_h = slo + L.taps;
+	float* sh_h = sphi + 2 * L.taps;
 	float* ss = sh_h + TX * HS;
 	// coefficient rows padded with zeros, H, the ring and S pads zero
 	for (int q = tid; q < L.taps; q += NTHREADS) {
 		const int j = q % pyp, ki = q / pyp;
-		sphi[q] = j < py ? tk.phi[ki * py + j] : 0.0f;
-		slo[q] = j < py ? tk.phi_lo[ki * py + j] : 0.0f;
+		sphi[2 * q] = j < py ? tk.phi[ki * py + j] : 0.0f;
+		sphi[2 * q + 1] = j < py ? tk.phi_lo[ki * py + j] : 0.0f;
 	}
 	// rows whose lo parts are all zero skip their second FMA chain
 	for (int ki = tid; ki < pt * px; ki += NTHREADS) {
