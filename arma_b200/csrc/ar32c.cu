@@ -743,6 +743,19 @@ size_t smem_bytes(int pt, int px, int py) {
 	                        std::max(GROUP * R, HUNITS * PS));
 }
 
+// CTAs per SM for a launch.  `tiles` is the work of all tiles over that of the
+// longest chain of slices: how many tiles run at once if none waits for an SM.
+// CTAs that share an SM slow each other's chains (a slice takes 1.35 and 1.8 times
+// as long with two and three), so below about one tile per SM the longest chain
+// is left an SM to itself, and below 2.4 it shares with one other.  Measured with
+// one, two and three per SM (ms): 0.9 tiles per SM 3.9 / 5.4 / 5.3; 1.3 7.8 / 6.4
+// / 8.4; 1.7 6.4 / 4.8 / 6.0; 2.0 11.2 / 8.6 / 8.9; 2.8 15.0 / 10.6 / 10.1; 3.1
+// 13.3 / 9.5 / 8.8; 4.8 28.4 / 20.2 / 19.0.
+int ctas_per_sm(double tiles, int sms, int most) {
+	const int n = tiles < 1.1 * sms ? 1 : tiles < 2.4 * sms ? 2 : 3;
+	return n < 3 ? std::min(n, most) : most;
+}
+
 // The filter's neighbour wait on a tile flag that nothing publishes: it runs
 // out after kSpinLimit polls and sets the error word (the failure path of
 // every bounded wait, exercised on purpose).
@@ -778,14 +791,20 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 		smem = std::max(smem, smem_bytes(s.pt, s.px, s.py));
 	}
 	// longest dependency chains first: a surface's wavefront needs about
-	// nt + tiles_x + tiles_y slice steps, each proportional to pt*px*py
+	// nt + tiles_x + tiles_y slice steps, each proportional to its taps and
+	// what H and the sums cost (as much as 160 taps)
+	auto slice = [](const Ar32Surface& s) { return double(s.pt * s.px * s.py + 160); };
 	auto chain = [&](const Ar32Surface& s) {
-		return double(s.nt + s.tiles_x + s.tiles_y) * s.pt * s.px * s.py;
+		return (s.nt - s.t0 + s.tiles_x + s.tiles_y) * slice(s);
 	};
 	std::sort(order.begin(), order.end(),
 	          [&](int a, int b) { return chain(surfaces[a]) > chain(surfaces[b]); });
 	size_t nflags = 0;
-	for (const auto& s : surfaces) nflags += size_t(s.tiles_x) * s.tiles_y;
+	double work = 0;
+	for (const auto& s : surfaces) {
+		nflags += size_t(s.tiles_x) * s.tiles_y;
+		work += double(s.tiles_x - s.given_tx) * s.tiles_y * (s.nt - s.t0) * slice(s);
+	}
 	int* flags = static_cast<int*>(scratch_take(c, sizeof(int) * nflags));
 	ARMA_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * nflags, c->stream));
 	std::vector<Task> tasks;
@@ -817,7 +836,10 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel, NTHREADS,
 	                                                            smem));
 	ARMA_REQUIRE(per_sm > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
-	if (c->tuning.ar_ctas_per_sm > 0) per_sm = std::min(per_sm, c->tuning.ar_ctas_per_sm);
+	if (c->tuning.ar_ctas_per_sm > 0)
+		per_sm = std::min(per_sm, c->tuning.ar_ctas_per_sm);
+	else if (!order.empty())
+		per_sm = ctas_per_sm(work / chain(surfaces[order[0]]), c->num_sms, per_sm);
 	const int grid = std::min(total, per_sm * c->num_sms);
 	ProfScope prof_(c, "ar32c");
 	ar32c_kernel<<<grid, NTHREADS, smem, c->stream>>>(d_tasks, int(tasks.size()), total, d_ticket,
@@ -975,6 +997,7 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 	    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
 		return fail(ARMA_ECUDA, "occupancy query failed");
 	if (per_sm <= 0) return fail(ARMA_ENOTSUP, "AR tile does not fit in shared memory");
+	per_sm = ctas_per_sm(double(ntiles) * t.nt / (t.nt + tiles_x + tiles_y), sms, per_sm);
 	const int grid = std::min(ntiles, per_sm * sms);
 	if (cudaMemcpyAsync(base + kOffTask, &t, sizeof(t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 	    cudaMemcpyAsync(d_coef, cbuf, sizeof(float) * ncoef, cudaMemcpyHostToDevice, st) !=

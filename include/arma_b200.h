@@ -95,7 +95,8 @@ int arma_ctx_profile_reset(arma_ctx* ctx);
  *                    (default 20); shorter segments give more CTAs and more
  *                    jump-ahead work;
  *   ar_ctas_per_sm   CTAs of the persistent FP32 filter launch per SM, 0 =
- *                    as many as fit (default);
+ *                    one, two or as many as fit, by how many of the batch's
+ *                    tiles can run at once (default);
  *   host_groups      arma_batch_generate_host (FP32) splits the batch, in
  *                    order of the filter's dependency chain, into this many
  *                    groups, 1..16 (default 16), computed on two alternating
