@@ -28,11 +28,15 @@
 // CTA only waits on tiles that running CTAs own; every wait is bounded.
 //
 // Measured (B200, the filter alone): 400 x 128 x 128 of order 10^3 4.9 ms (one
-// launch per hyperplane, its taps read through L1: 70 ms), 14.7 cycles per tap
-// and step with four warps on an SM, where the taps' 2.5 shared-memory wavefronts
-// per warp queue, and 11.8 with two; 200 x 40 x 40 of order 7^3 0.70 ms (12.0).
-// Two cells of one u per thread, sharing their windows, moved fewer bytes but
-// issued 14.7 to 19 cycles per tap and step from its lone warp.
+// launch per hyperplane, its taps read through L1: 70 ms); 200 x 40 x 40 of order
+// 7^3 0.66 ms.  The step is bound by shared memory: a warp's operand takes two
+// cycles of it and a broadcast pair of taps two more, so a step's tap takes 24
+// cycles with eight warps of one cell per thread on an SM, 14 with four, 11 with
+// two, against 8.2 for the chain.  Where throughput counts, a thread owns two
+// cells, (x, y) and (x+1, y-1) of one u, that share the taps and all but one
+// operand of a row (compute_pairs): four warps then move 256 cells in 21 cycles, 16
+// mixed surfaces 11.9 -> 10.2 ms.  Two warps of pairs are no faster than four of
+// single cells (13.5 and 13.9): a lone warp's issue bounds them.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -49,6 +53,8 @@ constexpr size_t kSmemLimit = 227 * 1024 - 64;  // less the kernel's static shar
 constexpr int kMaxAhead = 4;   // steps of halo kept ahead of their use
 constexpr int kUpstream = 5;   // tiles a tile's halo can come from
 constexpr int kBatch = 8;      // halo loads in flight per lane
+constexpr int kLead = 2;       // doubles before the ring: pairs load one column past its left edge
+constexpr int kPairTaps = 10;  // taps per row up to which two cells' operands fit in registers
 
 struct Task64 {
 	int nt, nx, ny, pt, px, py;
@@ -78,7 +84,7 @@ __host__ __device__ inline Layout64 layout64(int tx, int tu, int pt, int px, int
 	l.depth = tu + pt - 1 + ahead;
 	l.phi = (pt * px + 2) * even_up(py);  // and two rows that are loaded past the last
 	l.entries = (px - 1) * (tu + px + py - 2) + tx * (px + py - 2);
-	l.bytes = sizeof(double) * (size_t(l.slot) * l.depth + l.phi + even_up(l.entries));
+	l.bytes = sizeof(double) * (kLead + size_t(l.slot) * l.depth + l.phi + even_up(l.entries));
 	return l;
 }
 
@@ -142,6 +148,37 @@ __device__ __forceinline__ void row_step(double& s, double (&m)[PY], double (&w)
 	}
 }
 
+__device__ __forceinline__ void lds64_if(double& v, unsigned a, int on) {
+	asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t"
+	             "@q ld.shared.f64 %0, [%1];\n\t}" : "+d"(v) : "r"(a), "r"(on));
+}
+
+// The same for two cells: the products m0, m1 of this row are added to the two
+// chains; the next row's products take their place, its taps pc times its window
+// wc (chain 0) and the window before that, wp, one column on (chain 1); the window
+// (at zn) and taps (at pn_a) of the row after that load into wp, as that is used
+// up, and pn.  start: the row after next starts a slice, whose first window of
+// chain 1 (at zs) replaces wc as that is used up; by predicate, since a branch per
+// row costs a lone warp about 30 cycles of a row's 80.
+template <int PY, int N, int M>
+__device__ __forceinline__ void pair_step(double& s0, double& s1, double (&m0)[PY],
+                                         double (&m1)[PY], double (&wc)[N], double (&wp)[N],
+                                         const double (&pc)[M], double (&pn)[M], unsigned zn,
+                                         unsigned pn_a, unsigned zs, int start) {
+#pragma unroll
+	for (int j = 0; j < PY; ++j) {
+		if (j % 2 == 0) lds128(pn_a + 8 * j, pn[j], pn[j + 1]);
+		s0 = __dadd_rn(s0, m0[j]);
+		s1 = __dadd_rn(s1, m1[j]);
+		m0[j] = mul_here(pc[j], wc[j]);
+		m1[j] = mul_here(pc[j], wp[j + 1]);
+		wp[j] = lds64(zn - 8 * j);
+		if (j > 0) lds64_if(wc[j], zs - 8 * j, start);
+	}
+	wp[PY] = lds64(zn - 8 * PY);
+	lds64_if(wc[PY], zs - 8 * PY, start);
+}
+
 // What the warps of a CTA share about the current tile, and its named barriers
 // (0 is __syncthreads).  Step n of the compute warps ends at kBarHalo + n %
 // kHaloBars, where the halo warp has arrived when it has brought in step n + 1's
@@ -164,7 +201,7 @@ static_assert(kBarPub + kPubBars <= 16, "named barriers");
 // further up than the five polled here are therefore covered by those, whose
 // own steps waited for them.  A wait that runs out sets the error word and lets
 // the compute warps run on without the halo: they end, and the call fails.
-template <int TX, int TU>
+template <int TX, int TU, int NC>
 __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const Layout64& L, double* ring,
                           int2* cells, Shared64* sh, int* err) {
 	const int lane = threadIdx.x & 31;
@@ -204,7 +241,7 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 			known = ub * TX + uc * TU;
 		}
 	}
-	constexpr int kThreads = TX * TU + 32;
+	constexpr int kThreads = NC + 32;
 	const long long plane = (long long)tk.nx * tk.ny;
 	int n = 0;
 	bool failed = false;
@@ -273,9 +310,9 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 // The publication warp: the barrier orders the compute warps' global stores of
 // a step before the release store that publishes it; steps that are handed over
 // meanwhile are published together.
-template <int TX, int TU>
+template <int TX, int TU, int NC>
 __device__ __forceinline__ void pub_warp(const Task64& tk, int bx, int c, Shared64* sh) {
-	constexpr int kThreads = TX * TU + 32;
+	constexpr int kThreads = NC + 32;
 	int* flag = tk.flags + bx * tk.nc + c;
 	const int lane = threadIdx.x & 31;
 	const int U0 = bx * TX + c * TU, steps = tk.nt + TU - 1;
@@ -390,11 +427,129 @@ __device__ __forceinline__ void compute_tile(const Task64& tk, int bx, int c, co
 	}
 }
 
-template <int TX, int TU>
-__global__ void __launch_bounds__(TX * TU + 64)
+template <int PY, int TX, int TU>
+__device__ __forceinline__ void compute_pairs(const Task64& tk, int bx, int c, const Layout64& L, double* ring,
+                             const double* sphi, Shared64* sh, int* err) {
+	constexpr int NC = TX / 2 * TU;
+	constexpr int PYP = (PY + 1) & ~1;
+	const int l = threadIdx.x % TU, rp = threadIdx.x / TU;
+	const int px = tk.px, rows = tk.pt * px;
+	const int x = bx * TX + 2 * rp, U0 = bx * TX + c * TU, y = U0 + l - x;
+	const bool ok0 = x < tk.nx && y >= 0 && y < tk.ny;
+	const bool ok1 = x + 1 < tk.nx && y - 1 >= 0 && y - 1 < tk.ny;
+	const long long plane = (long long)tk.nx * tk.ny;
+	double* const z0 = tk.zeta + (long long)x * tk.ny + y;
+	double* const z1 = z0 + tk.ny - 1;
+	double* const own = ring + (2 * rp + px - 1) * L.ld + l + px + PY - 2;
+	unsigned own_a = static_cast<unsigned>(__cvta_generic_to_shared(own));
+	unsigned taps = static_cast<unsigned>(__cvta_generic_to_shared(sphi));
+	// one row up and one column left; one slot
+	unsigned row_bytes = 8u * unsigned(L.ld + 1), slot_bytes = 8u * unsigned(L.slot);
+	// (opaque: nothing is computed ahead for all widths of the kernel's switch)
+	asm volatile("" : "+r"(own_a), "+r"(taps), "+r"(row_bytes), "+r"(slot_bytes));
+	const int steps = tk.nt + TU - 1;
+	int slot = l == 0 ? 0 : L.depth - l;  // of t = n - l
+	double e0 = ok0 && l == 0 ? z0[0] : 0.0, e1 = ok1 && l == 0 ? z1[0] : 0.0;
+	__syncthreads();  // step 0's halo
+	for (int n = 0; n < steps; ++n) {
+		const int t = n - l;
+		// the next step's noise
+		const bool next = t + 1 >= 0 && t + 1 < tk.nt;
+		const double f0 = next && ok0 ? z0[(t + 1) * plane] : 0.0;
+		const double f1 = next && ok1 ? z1[(t + 1) * plane] : 0.0;
+		double s0 = 0.0, s1 = 0.0;
+		{
+			// Row of taps r = (k, i) at a time, both chains on the same taps:
+			// chain 0 reads window r, row x-i of slice t-k, chain 1 window r-1
+			// (row x+1-i) one column on; at i = 0 chain 1's row is read by
+			// itself.  Two windows and two rows of taps in turn.
+			double w[2][PY + 1], p[2][PYP], m0[PY], m1[PY];
+			int ks = slot, i = 0;
+			unsigned pa = taps, za = own_a + unsigned(ks) * slot_bytes;
+			auto advance = [&] {  // to the next row; 1 at the start of a slice
+				pa += 8 * PYP;
+				const int start = i + 1 == px ? 1 : 0;
+				i = start ? 0 : i + 1;
+				const int kn = ks == 0 ? L.depth - 1 : ks - 1;
+				ks = start ? kn : ks;
+				za = start ? own_a + unsigned(ks) * slot_bytes : za - row_bytes;
+				return start;
+			};
+			// row 0's products and row 1's operands
+#pragma unroll
+			for (int j = 0; j <= PY; ++j) {
+				w[1][j] = lds64(za + row_bytes - 8 * j);
+				w[0][j] = lds64(za - 8 * j);
+			}
+#pragma unroll
+			for (int j = 0; j < PYP; j += 2) lds128(pa + 8 * j, p[0][j], p[0][j + 1]);
+			w[1][1] = e1;  // lag (0, 0, 0): the cells' own noise
+			w[0][0] = e0;
+			int start = advance();
+#pragma unroll
+			for (int j = 0; j < PYP; j += 2) lds128(pa + 8 * j, p[1][j], p[1][j + 1]);
+#pragma unroll
+			for (int j = 0; j <= PY; ++j) {
+				if (j < PY) {
+					m0[j] = mul_here(p[0][j], w[0][j]);
+					m1[j] = mul_here(p[0][j], w[1][j + 1]);
+				}
+				w[1][j] = lds64(za - 8 * j);
+				if (j > 0) lds64_if(w[0][j], za + row_bytes - 8 * j, start);
+			}
+			// (the last two rows load rows past the last, within the ring and
+			// the padding after the taps: not used)
+			auto row = [&](auto odd) {
+				constexpr int b = decltype(odd)::value;
+				start = advance();
+				pair_step<PY>(s0, s1, m0, m1, w[1 - b], w[b], p[1 - b], p[b], za, pa,
+				             za + row_bytes, start);
+			};
+			using Even = std::integral_constant<int, 0>;
+			using Odd = std::integral_constant<int, 1>;
+			int left = rows;
+			for (; left >= 4; left -= 4) {
+				row(Even{});
+				row(Odd{});
+				row(Even{});
+				row(Odd{});
+			}
+			if (left > 0) row(Even{});
+			if (left > 1) row(Odd{});
+			if (left > 2) row(Even{});
+		}
+		s0 = __dadd_rn(e0, s0);
+		s1 = __dadd_rn(e1, s1);
+		const bool live = t >= 0 && t < tk.nt;
+		double* r = own + slot * L.slot;
+		if (live && ok0) r[0] = s0;
+		if (live && ok1) r[L.ld] = s1;
+		// every cell of step n is in the ring, and step n + 1's halo
+		if (n + 1 < steps) bar_sync(kBarHalo + n % kHaloBars, NC + 32);
+		// (released before this step's global stores: it waits for none)
+		if (threadIdx.x == 0) st_release_cta(&sh->done, n + 1);
+		if (live && ok0) z0[t * plane] = s0;
+		if (live && ok1) z1[t * plane] = s1;
+		// the barrier's previous round is over once the publication warp has
+		// left it (it waits for nothing but these barriers)
+		for (long long it = 0; *((volatile int*)&sh->published) < n + 1 - kPubBars; ++it)
+			if (it == kSpinLimit * 64) {
+				atomicCAS(err, DEV_OK, DEV_TIMEOUT);
+				break;
+			}
+		__syncwarp();
+		bar_arrive(kBarPub + n % kPubBars, NC + 32);
+		e0 = f0;
+		e1 = f1;
+		slot = slot + 1 == L.depth ? 0 : slot + 1;
+	}
+}
+
+template <int TX, int TU, int CELLS>
+__global__ void __launch_bounds__(TX * TU / CELLS + 64)
 ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
                  int* __restrict__ counter, int* __restrict__ err) {
-	constexpr int NC = TX * TU, NTHREADS = NC + 64;
+	constexpr int NC = TX * TU / CELLS, NTHREADS = NC + 64;
 	extern __shared__ __align__(16) double smem64[];
 	__shared__ Shared64 sh;
 	__shared__ int s_ticket;
@@ -413,7 +568,7 @@ ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
 		const Task64 tk = tasks[lo];
 		const int bx = (ticket - tk.ticket_base) / tk.nc, c = (ticket - tk.ticket_base) % tk.nc;
 		const Layout64 L = layout64(TX, TU, tk.pt, tk.px, tk.py, tk.ahead);
-		double* ring = smem64;
+		double* ring = smem64 + kLead;
 		double* sphi = ring + size_t(L.slot) * L.depth;
 		int2* cells = reinterpret_cast<int2*>(sphi + L.phi);
 		const int pyp = even_up(tk.py);
@@ -429,9 +584,17 @@ ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
 		}
 		__syncthreads();
 		if (tid >= NC + 32) {
-			pub_warp<TX, TU>(tk, bx, c, &sh);
+			pub_warp<TX, TU, NC>(tk, bx, c, &sh);
 		} else if (tid >= NC) {
-			halo_warp<TX, TU>(tk, bx, c, L, ring, cells, &sh, err);
+			halo_warp<TX, TU, NC>(tk, bx, c, L, ring, cells, &sh, err);
+		} else if constexpr (CELLS == 2) {
+			switch (tk.py) {
+#define ARMA_PY_CASE(N) case N: compute_pairs<N, TX, TU>(tk, bx, c, L, ring, sphi, &sh, err); break;
+				ARMA_PY_CASE(1) ARMA_PY_CASE(2) ARMA_PY_CASE(3) ARMA_PY_CASE(4) ARMA_PY_CASE(5)
+				ARMA_PY_CASE(6) ARMA_PY_CASE(7) ARMA_PY_CASE(8) ARMA_PY_CASE(9) ARMA_PY_CASE(10)
+#undef ARMA_PY_CASE
+				default: break;
+			}
 		} else {
 			switch (tk.py) {
 #define ARMA_PY_CASE(N) case N: compute_tile<N, TX, TU>(tk, bx, c, L, ring, sphi, &sh, err); break;
@@ -502,7 +665,7 @@ int ahead_of(int tx, int tu, const Ar64Surface& s) {
 
 int tiles_per_row(int tx, int tu, int ny) { return (ny + tx - 1 + tu - 1) / tu; }
 
-template <int TX, int TU>
+template <int TX, int TU, int CELLS>
 void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 	// longest dependency chains first
 	auto chain = [](const Ar64Surface& s) {
@@ -537,8 +700,8 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 	auto* d_tasks = static_cast<Task64*>(scratch_take(c, sizeof(Task64) * tasks.size()));
 	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task64) * tasks.size(),
 	                         cudaMemcpyHostToDevice, c->stream));
-	constexpr int threads = TX * TU + 64;
-	auto kernel = ar64_tile_kernel<TX, TU>;
+	constexpr int threads = TX * TU / CELLS + 64;
+	auto kernel = ar64_tile_kernel<TX, TU, CELLS>;
 	ARMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                   int(kSmemLimit)));
 	int per_sm = 0;
@@ -556,29 +719,38 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 
 void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces) {
 	ProfScope prof_(c, "ar64");
-	// Tile shapes: 16 x 16 (eight compute warps) when the batch fills the GPU,
-	// 8 x 16 and 4 x 16 to spread a smaller one over more SMs, where fewer warps
-	// share the bandwidth of shared memory; 8 x 8 for orders whose ring does not
-	// fit otherwise.
+	// Tile shapes, by how many cells can be at work at once if none waits for an
+	// SM (all steps of all tiles over the longest chain).  16 x 16 by pairs moves
+	// the most cells per cycle and is the slowest step (21 cycles a tap): taken
+	// where more than 96 cells per SM are at work.  8 x 16 (14 cycles a tap) below
+	// that, 4 x 16 (11) where all its tiles have an SM to themselves.  Measured, 16
+	// x 16 / 8 x 16 / 4 x 16 (ms): 40 cells per SM 3.9 / 2.7 / 3.1; 79 (400 x 128 x
+	// 128 of order 10^3) 7.0 / 4.9 / 5.5; 108 3.7 / 4.4 / 4.6; 142 10.1 / 10.9 /
+	// 12.1; 415 (16 mixed surfaces) 10.2 / 13.7 / 17.5; 200 x 40 x 40 alone, 30 tiles
+	// of 4 x 16, 1.14 / 0.76 / 0.65.  8 x 16 too for rows of more taps than a pair's
+	// registers hold, 4 x 16 and 8 x 8 for orders whose ring does not fit otherwise.
 	std::vector<Ar64Surface> groups[4];
-	long long t8 = 0, t4 = 0;
+	long long t4 = 0;
+	double work = 0, chain = 0;
 	for (const Ar64Surface& s : surfaces)
 		if (s.finite) {
-			t8 += (long long)((s.nx + 7) / 8) * tiles_per_row(8, 16, s.ny);
+			const double taps = double(s.pt) * s.px * s.py;
 			t4 += (long long)((s.nx + 3) / 4) * tiles_per_row(4, 16, s.ny);
+			work += 256.0 * ((s.nx + 15) / 16) * tiles_per_row(16, 16, s.ny) * (s.nt + 15) * taps;
+			chain = std::max(chain, (double(s.nt) + s.nx + s.ny) * taps);
 		}
-	const int want = t4 <= c->num_sms ? 2 : t8 <= c->num_sms ? 1 : 0;
+	const int want = t4 <= c->num_sms ? 2 : work <= 96.0 * c->num_sms * chain ? 1 : 0;
 	for (const Ar64Surface& s : surfaces) {
 		if (!s.finite) launch_planes(c, s);
-		else if (want == 0 && ahead_of(16, 16, s)) groups[0].push_back(s);
+		else if (want == 0 && s.py <= kPairTaps && ahead_of(16, 16, s)) groups[0].push_back(s);
 		else if (want <= 1 && ahead_of(8, 16, s)) groups[1].push_back(s);
 		else if (ahead_of(4, 16, s)) groups[2].push_back(s);
 		else groups[3].push_back(s);
 	}
-	if (!groups[0].empty()) launch_tiles<16, 16>(c, groups[0]);
-	if (!groups[1].empty()) launch_tiles<8, 16>(c, groups[1]);
-	if (!groups[2].empty()) launch_tiles<4, 16>(c, groups[2]);
-	if (!groups[3].empty()) launch_tiles<8, 8>(c, groups[3]);
+	if (!groups[0].empty()) launch_tiles<16, 16, 2>(c, groups[0]);
+	if (!groups[1].empty()) launch_tiles<8, 16, 1>(c, groups[1]);
+	if (!groups[2].empty()) launch_tiles<4, 16, 1>(c, groups[2]);
+	if (!groups[3].empty()) launch_tiles<8, 8, 1>(c, groups[3]);
 }
 
 }  // namespace armab
