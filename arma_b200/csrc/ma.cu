@@ -6,10 +6,11 @@
 // overlap-add (src/apmath/convolution.hh:58-130), which is the causal linear
 // convolution truncated to the surface; the reference's own test writes the
 // same sum directly (src/test/convolution-test.cc:17-50).  Here it is the
-// direct sum on the CUDA cores: with no feedback the filter is data-parallel
-// and compute-bound (2 P FLOP per point for P taps), and at the reference's
-// orders (up to a few thousand taps) the direct form needs one pass over the
-// noise where an FFT form needs several over padded complex arrays.
+// direct sum (FP64 by matrix instructions, FP32 and short FP64 orders on the CUDA
+// cores): with no feedback the filter is data-parallel and compute-bound (2 P FLOP
+// per point for P taps), and at the reference's orders (up to a few thousand taps)
+// the direct form needs one pass over the noise where an FFT form needs several
+// over padded complex arrays.
 //
 // A block owns a tile of 8 time steps x 16 rows (x) x 16 R columns (y), R = 4
 // for FP64 and 8 for FP32 (register budget: 2 blocks of 256 threads per SM); each
@@ -125,6 +126,34 @@ __device__ __forceinline__ void ma_slice(T (&acc)[kMaTT][R], const T* buf, const
 	}
 }
 
+// Noise slice s (its part under a tile) and its taps into shared memory, one
+// cp.async group.
+template <class T>
+__device__ __forceinline__ void ma_stage(const T* __restrict__ eps, const T* __restrict__ K, T* dst,
+                                         T* cdst, int tid, int s, int nt, int nx, int ny, int pt,
+                                         int px, int py, int i0, int ni, int x0, int y0, int t0,
+                                         int rows, int cols, int ld) {
+	// a warp to a row: no division by the number of columns
+	const T* src = eps + size_t(s) * nx * ny;
+	for (int rr = tid / 32; rr < rows; rr += kMaThreads / 32) {
+		const int gx = x0 - (px - 1) + rr;
+		const T* row = src + ptrdiff_t(gx) * ny;
+		for (int cc = tid % 32; cc < cols; cc += 32) {
+			const int gy = y0 - (py - 1) + cc;
+			const bool ok = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+			cp_async_elem(dst + rr * ld + cc, ok ? row + gy : eps, ok);
+		}
+	}
+	const size_t plane = size_t(px) * py;
+	for (int idx = tid; idx < ni * py * kMaTT; idx += kMaThreads) {
+		const int tt = idx % kMaTT, ij = idx / kMaTT;  // the tap i0 py + ij of its plane
+		const int k = t0 + tt - s;
+		const bool ok = k >= 0 && k < pt && t0 + tt < nt;
+		cp_async_elem(cdst + idx, ok ? K + k * plane + i0 * py + ij : K, ok);
+	}
+	asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 template <class T>
 __global__ void __launch_bounds__(kMaThreads)
 ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restrict__ K, int nt,
@@ -147,25 +176,9 @@ ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restri
 #pragma unroll
 		for (int r = 0; r < R; ++r) acc[tt][r] = T(0);
 
-	// noise slice s and its taps into buffer b, one cp.async group
 	auto load = [&](int s, int b) {
-		const T* src = eps + size_t(s) * plane;
-		T* dst = ebuf + b * tile;
-		for (int idx = tid; idx < rows * cols; idx += kMaThreads) {
-			const int rr = idx / cols, cc = idx - rr * cols;
-			const int gx = x0 - (px - 1) + rr, gy = y0 - (py - 1) + cc;
-			const bool ok = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-			cp_async_elem(dst + rr * ld + cc, ok ? src + size_t(gx) * ny + gy : eps, ok);
-		}
-		T* cdst = cbuf + b * ctile;
-		for (int idx = tid; idx < ctile; idx += kMaThreads) {
-			const int tt = idx % TT, ij = idx / TT;
-			const int j = ij % py, i = i0 + ij / py;
-			const int k = t0 + tt - s;
-			const bool ok = k >= 0 && k < pt && t0 + tt < nt;
-			cp_async_elem(cdst + idx, ok ? K + (size_t(k) * px + i) * py + j : K, ok);
-		}
-		asm volatile("cp.async.commit_group;" ::: "memory");
+		ma_stage<T>(eps, K, ebuf + b * tile, cbuf + b * ctile, tid, s, nt, nx, ny, pt, px, py, i0, ni,
+		            x0, y0, t0, rows, cols, ld);
 	};
 
 	load(s_hi, 0);
@@ -203,6 +216,88 @@ ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restri
 	}
 }
 
+// FP64 by matrix instructions (m8n8k4, the only shape there is for FP64): a slice's
+// taps c(i, j, tt) are the 8 x 4 operand (time steps by four taps (i, j) in a row),
+// the noise under them the 4 x 8 one (taps by columns).  The same tile as above; a
+// warp owns two rows of 8 x 8 columns, whose 16 products share the taps' operand,
+// so a slice costs 2.2 cycles of shared memory per product where the scalar form's
+// 4 noise values and 8 taps per 32 FMAs filled it: 256 x 128 x 128 of order 20 x 10
+// x 10 1040 -> 800 us, bound by the FP64 pipe, the time steps a slice does not reach
+// included (620 us of it at the pipe's rate).
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
+	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+	    : "+d"(d[0]), "+d"(d[1])
+	    : "d"(a), "d"(b));
+}
+
+__global__ void __launch_bounds__(kMaThreads, 2)
+ma_mma_kernel(const double* __restrict__ eps, double* __restrict__ zeta,
+              const double* __restrict__ K, int nt, int nx, int ny, int pt, int px, int py, int i0,
+              int i1, int accumulate) {
+	constexpr int TT = kMaTT, TX = 16, NT = 8, TY = 8 * NT;
+	extern __shared__ __align__(16) unsigned char ma_smem[];
+	const int rows = TX + px - 1, cols = TY + py - 1, ld = ma_pitch<double>(cols);
+	const int tile = ma_tile_elems<double>(px, py);
+	const int ni = i1 - i0, taps = ni * py, quads = (taps + 3) / 4, ctile = quads * 4 * TT;
+	double* ebuf = reinterpret_cast<double*>(ma_smem);
+	double* cbuf = ebuf + 2 * tile;
+	int* off = reinterpret_cast<int*>(cbuf + 2 * ctile);  // of a tap's noise, in doubles
+	const int y0 = blockIdx.x * TY, x0 = blockIdx.y * TX, t0 = blockIdx.z * TT;
+	const int tid = threadIdx.x, lane = tid % 32, kk = lane % 4, n = lane / 4;
+	const int xl = tid / 32 * 2;
+	const int s_hi = min(nt - 1, t0 + TT - 1), s_lo = max(0, t0 - (pt - 1));
+
+	double acc[2][NT][2];
+#pragma unroll
+	for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+		for (int m = 0; m < NT; ++m) acc[rr][m][0] = acc[rr][m][1] = 0.0;
+	// the last four taps are filled up with zeros
+	for (int q = tid; q < quads * 4; q += kMaThreads)
+		off[q] = q < taps ? -((i0 + q / py) * ld + q % py) : 0;
+	for (int q = taps * TT + tid; q < ctile; q += kMaThreads) cbuf[q] = cbuf[ctile + q] = 0.0;
+
+	auto load = [&](int s, int b) {
+		ma_stage<double>(eps, K, ebuf + b * tile, cbuf + b * ctile, tid, s, nt, nx, ny, pt, px, py,
+		                 i0, ni, x0, y0, t0, rows, cols, ld);
+	};
+	load(s_hi, 0);
+	int b = 0;
+	for (int s = s_hi; s >= s_lo; --s, b ^= 1) {
+		if (s > s_lo) load(s - 1, b ^ 1);
+		else asm volatile("cp.async.commit_group;" ::: "memory");
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
+		__syncthreads();
+		const double* src = ebuf + b * tile + (xl + px - 1) * ld + py - 1 + n;
+		const double* ca = cbuf + b * ctile + kk * TT + n;
+		for (int q = 0; q < quads; ++q) {
+			const double a = ca[q * 4 * TT];
+			const double* v = src + off[q * 4 + kk];
+#pragma unroll
+			for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+				for (int m = 0; m < NT; ++m) mma_f64(acc[rr][m], a, v[rr * ld + 8 * m]);
+		}
+		__syncthreads();
+	}
+	const int t = t0 + n;
+	if (t >= nt) return;
+#pragma unroll
+	for (int rr = 0; rr < 2; ++rr) {
+		const int x = x0 + xl + rr;
+		if (x >= nx) break;
+#pragma unroll
+		for (int m = 0; m < NT; ++m)
+#pragma unroll
+			for (int e = 0; e < 2; ++e) {
+				const int y = y0 + 8 * m + 2 * kk + e;
+				if (y >= ny) continue;
+				double* p = zeta + (size_t(t) * nx + x) * ny + y;
+				*p = accumulate ? *p + acc[rr][m][e] : acc[rr][m][e];
+			}
+	}
+}
+
 // Rows of taps (values of i) per launch: both tap buffers within kMaTapBytes.
 template <class T>
 int ma_rows_per_launch(int px, int py) {
@@ -237,8 +332,27 @@ void ma_filter_impl(Ctx* c, const double* theta, const int order[3], const int s
 	                (shape[0] + kMaTT - 1) / kMaTT);
 	ARMA_REQUIRE(grid.y <= 65535 && grid.z <= 65535, ARMA_EINVAL, "surface too large");
 	const int rows_per = ma_rows_per_launch<T>(px, py);
+	// the taps filled up to four, and their offsets
+	const size_t mma_smem = smem + 2 * 3 * kMaTT * sizeof(T) + (size_t(rows_per) * py + 3) * sizeof(int);
+	// matrix instructions take the 8 time steps whole, also on the slices that reach
+	// only some, and taps by fours: 256 x 128 x 128, us, by them / scalar: order 20 x
+	// 10 x 10 800 / 987, 4 x 5 x 5 118 / 116, 3 x 10 x 10 305 / 298, 1 x 10 x 10 247 /
+	// 218, 8 x 1 x 1 48 / 40; 24 x 128 x 20 of 6 x 6 x 6 55 / 63; 64 x 32 x 32 of 5 x
+	// 3 x 3 30 / 31
+	const bool mma = sizeof(T) == 8 && pt >= 5 && px * py >= 8 && mma_smem <= size_t(kMaSmemLimit);
+	if (mma)
+		ARMA_CUDA_TRY(cudaFuncSetAttribute(ma_mma_kernel,
+		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kMaSmemLimit));
 	for (int i0 = 0; i0 < px; i0 += rows_per) {
 		const int i1 = std::min(px, i0 + rows_per);
+		if constexpr (sizeof(T) == 8)
+			if (mma) {
+				ma_mma_kernel<<<grid, kMaThreads, mma_smem, c->stream>>>(
+				    eps, zeta, dK, shape[0], shape[1], shape[2], pt, px, py, i0, i1, i0 > 0 ? 1 : 0);
+				ARMA_CUDA_TRY(cudaGetLastError());
+				++c->launches;
+				continue;
+			}
 		ma_fir_kernel<T><<<grid, dim3(16, 16), smem, c->stream>>>(
 		    eps, zeta, dK, shape[0], shape[1], shape[2], pt, px, py, i0, i1, i0 > 0 ? 1 : 0);
 		ARMA_CUDA_TRY(cudaGetLastError());
