@@ -1285,7 +1285,7 @@ template <int M, int NY, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
 velocity_real_kernel(const VelSlice<float>* __restrict__ sl, const double* __restrict__ kinfo,
                      const double* __restrict__ zs, double depth, float2* __restrict__ spectra,
-                     int part) {
+                     int part, int z0) {
 	constexpr int NX = 2 * M, LD = RealLd<M, NY>::v;
 	constexpr int L = NX > NY ? NX : NY;  // twiddle table: W_L^j
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1318,7 +1318,7 @@ velocity_real_kernel(const VelSlice<float>* __restrict__ sl, const double* __res
 			return;
 		}
 	}
-	const int iz = part == kRealDepth ? blockIdx.y : 0;
+	const int iz = part == kRealDepth ? z0 + int(blockIdx.y) : 0;
 	const double wx = 1.0 / kinfo[s * 4 + 0], wy = 1.0 / kinfo[s * 4 + 1];
 	const double dkx = wx / (NX - 1), dky = wy / (NY - 1);
 	const float inv = float(1.0 / double(M * NY));
@@ -1391,14 +1391,14 @@ bool launch_real_shape(Ctx* c, const VelSlice<float>* d_sl, int ns, int nx, int 
 		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
 		auto kernel = velocity_real_kernel<M, NY, NT>;
 		if (nz == 1) {
-			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealAll);
+			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealAll, 0);
 		} else {
-			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealSpectrum);
+			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealSpectrum, 0);
 			ARMA_CUDA_TRY(cudaGetLastError());
 			c->launches += 1;
 			for (int z0 = 0; z0 < nz; z0 += 65535)
 				kernel<<<dim3(ns, std::min(nz - z0, 65535)), NT, smem, c->stream>>>(
-				    d_sl, d_k, d_z, depth, spectra, kRealDepth);
+				    d_sl, d_k, d_z, depth, spectra, kRealDepth, z0);
 		}
 		return true;
 	}

@@ -53,3 +53,23 @@ def test_window_and_split(ctx, shape, depth, zs, high_amplitude):
                             high_amplitude=high_amplitude)
         got = out.cpu().numpy().astype(np.float64)
         assert np.abs(got - ref).max() <= tol * scale, (prec, np.abs(got - ref).max() / scale)
+
+
+def test_more_depths_than_a_grid_dimension(ctx):
+    """65540 depths of one small slice: the last ones as a call of their own has them."""
+    rng = np.random.default_rng(3)
+    z = torch.tensor(rng.standard_normal((3, 32, 16)), dtype=torch.float32, device="cuda")
+    zs = np.linspace(0.0, -4.0, 65540)
+
+    def run(levels):
+        out = torch.full((1, len(levels), 32, 16), np.nan, dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        ctx.velocity_linear(z.data_ptr(), (3, 32, 16), A.FP32C, (1.0, 1.0, 1.0), np.inf,
+                            list(levels), [1], out.data_ptr())
+        ctx.synchronize()
+        return out
+
+    whole = run(zs)
+    assert torch.isfinite(whole).all()
+    for part in (slice(0, 3), slice(65533, 65540)):
+        assert torch.equal(whole[:, part], run(zs[part]))
