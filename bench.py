@@ -364,14 +364,14 @@ def gpu_arm(args):
         ctx.set_tuning(tuned_dev)  # the device-resident legs below
     del bufs32
 
-    # ---- plain FP64 path on the same batch (surface after surface)
+    # ---- plain FP64 path on the same batch
     plain = None
     if not args.skip_plain:
         bufs64 = [torch.empty(s["shape"], dtype=torch.float64, device="cuda") for s in batch]
         surf64 = [capi.make_surface(s["shape"], s["phi"], s["var"], s["acf0"],
                                     sets[s["mtset"] % len(sets)], s["seed"], b.data_ptr())
                   for s, b in zip(batch, bufs64)]
-        ctx.batch_generate(surf64, A.FP64)  # builds and caches the plane graphs
+        ctx.batch_generate(surf64, A.FP64)  # warm-up: scratch and jump tables
         barrier()
         t0 = time.perf_counter()
         ctx.batch_generate(surf64, A.FP64)

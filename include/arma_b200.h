@@ -74,6 +74,8 @@ int arma_last_error(char* buf, size_t len);
 int arma_ctx_create(int device, arma_ctx** out);
 int arma_ctx_destroy(arma_ctx* ctx);
 int arma_ctx_set_stream(arma_ctx* ctx, void* cuda_stream);
+/* Waits for the context's stream; ARMA_ETIMEDOUT when a bounded device wait of
+ * an earlier asynchronous call ran out. */
 int arma_ctx_synchronize(arma_ctx* ctx);
 /* Kernel launches issued through this context since creation (counter). */
 int arma_ctx_launch_count(arma_ctx* ctx, uint64_t* count);
@@ -91,9 +93,10 @@ int arma_ctx_profile_reset(arma_ctx* ctx);
 /* Settings of the batched calls that change their speed but never their
  * results (no counterpart in the reference):
  *   mt_log2_segment  the dcmt stream of a surface is cut into segments of
- *                    2^v words generated by one CTA each, v in [16, 22]
- *                    (default 20); shorter segments give more CTAs and more
- *                    jump-ahead work;
+ *                    at most 2^v words generated by one CTA each, v in
+ *                    [16, 22] (default 20; few or short streams take
+ *                    shorter ones); shorter segments give more CTAs and
+ *                    more jump-ahead work;
  *   ar_ctas_per_sm   CTAs of the persistent FP32 filter launch per SM, 0 =
  *                    one, two or as many as fit, by how many of the batch's
  *                    tiles can run at once (default);
@@ -311,8 +314,10 @@ typedef struct {
 } arma_surface;
 
 /* White noise + AR filter (+ renormalisation) for n independent surfaces.
- * ARMA_FP32C runs all surfaces in one persistent launch; ARMA_FP64 runs the
- * plain filter surface by surface. */
+ * Both precisions run all surfaces in one persistent launch (ARMA_FP64: a
+ * launch per tile shape, and per hyperplane for models whose coefficients are
+ * not finite); a device wait of the FP64 filter that ran out is reported by the
+ * next arma_ctx_synchronize. */
 int arma_batch_generate(arma_ctx* ctx, arma_surface* surfaces, int n,
                         int precision);
 /* Same, writing each surface into a HOST buffer (d_zeta is then a host
