@@ -154,10 +154,11 @@ __device__ __forceinline__ void ma_stage(const T* __restrict__ eps, const T* __r
 	asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
+// The scalar form of one block's tile.
 template <class T>
-__global__ void __launch_bounds__(kMaThreads)
-ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restrict__ K, int nt,
-              int nx, int ny, int pt, int px, int py, int i0, int i1, int accumulate) {
+__device__ __forceinline__ void ma_block(const T* __restrict__ eps, T* __restrict__ zeta,
+                                         const T* __restrict__ K, int nt, int nx, int ny, int pt,
+                                         int px, int py, int i0, int i1, int accumulate, int tid) {
 	constexpr int R = MaShape<T>::R, TT = kMaTT, TY = 16 * R, TX = 16;
 	extern __shared__ __align__(16) unsigned char ma_smem[];
 	const int rows = TX + px - 1, cols = TY + py - 1, ld = ma_pitch<T>(cols);
@@ -166,7 +167,7 @@ ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restri
 	T* ebuf = reinterpret_cast<T*>(ma_smem);
 	T* cbuf = ebuf + 2 * tile;
 	const int y0 = blockIdx.x * TY, x0 = blockIdx.y * TX, t0 = blockIdx.z * TT;
-	const int lane = threadIdx.x, xl = threadIdx.y, tid = xl * 16 + lane;
+	const int lane = tid % 16, xl = tid / 16;
 	const int s_hi = min(nt - 1, t0 + TT - 1), s_lo = max(0, t0 - (pt - 1));
 	const size_t plane = size_t(nx) * ny;
 
@@ -214,6 +215,20 @@ ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restri
 			*p = accumulate ? *p + acc[tt][r] : acc[tt][r];
 		}
 	}
+}
+
+template <class T>
+__global__ void __launch_bounds__(kMaThreads)
+ma_fir_kernel(const T* __restrict__ eps, T* __restrict__ zeta, const T* __restrict__ K, int nt,
+              int nx, int ny, int pt, int px, int py, int i0, int i1, int accumulate) {
+	ma_block<T>(eps, zeta, K, nt, nx, ny, pt, px, py, i0, i1, accumulate, threadIdx.x);
+}
+
+// Out of line: its registers are not the matrix form's.
+__device__ __noinline__ void ma_block_scalar(const double* eps, double* zeta, const double* K,
+                                             int nt, int nx, int ny, int pt, int px, int py, int i0,
+                                             int i1, int accumulate) {
+	ma_block<double>(eps, zeta, K, nt, nx, ny, pt, px, py, i0, i1, accumulate, threadIdx.x);
 }
 
 // FP64 by matrix instructions (m8n8k4, the only shape there is for FP64): a slice's
@@ -279,6 +294,17 @@ ma_mma_kernel(const double* __restrict__ eps, double* __restrict__ zeta,
 				for (int m = 0; m < NT; ++m) mma_f64(acc[rr][m], a, v[rr * ld + 8 * m]);
 		}
 		__syncthreads();
+	}
+	// the zeros of time steps that a slice does not reach, times noise that is not
+	// finite, are not zero: such a tile is summed again by the scalar form
+	bool odd = false;
+#pragma unroll
+	for (int rr = 0; rr < 2; ++rr)
+#pragma unroll
+		for (int m = 0; m < NT; ++m) odd = odd || !isfinite(acc[rr][m][0]) || !isfinite(acc[rr][m][1]);
+	if (__syncthreads_or(odd)) {
+		ma_block_scalar(eps, zeta, K, nt, nx, ny, pt, px, py, i0, i1, accumulate);
+		return;
 	}
 	const int t = t0 + n;
 	if (t >= nt) return;
@@ -353,7 +379,7 @@ void ma_filter_impl(Ctx* c, const double* theta, const int order[3], const int s
 				++c->launches;
 				continue;
 			}
-		ma_fir_kernel<T><<<grid, dim3(16, 16), smem, c->stream>>>(
+		ma_fir_kernel<T><<<grid, kMaThreads, smem, c->stream>>>(
 		    eps, zeta, dK, shape[0], shape[1], shape[2], pt, px, py, i0, i1, i0 > 0 ? 1 : 0);
 		ARMA_CUDA_TRY(cudaGetLastError());
 		++c->launches;

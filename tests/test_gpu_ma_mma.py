@@ -30,3 +30,29 @@ def test_against_direct_sum(shape, order):
     # each side sums P products in some order: P 2^-53 of the sum of magnitudes
     bound = 2 * theta.size * 2.0 ** -53 * (1.0 + np.abs(theta).sum()) * np.abs(eps).max()
     assert np.max(np.abs(z.cpu().numpy() - O.ma_filter(eps, theta))) <= bound
+
+
+def test_noise_that_is_not_finite_stays_where_it_reaches():
+    """An infinity in slice 5 meets, in the scalar form, the time steps 4 and later
+    of its block: the steps before it keep their values."""
+    shape, order = (24, 20, 70), (6, 3, 4)
+    rng = np.random.default_rng(8)
+    theta = rng.uniform(-1.0, 1.0, order)
+    eps = rng.standard_normal(shape)
+    got = []
+    with A.Context(0) as ctx:
+        for bad in (False, True):
+            e = torch.tensor(eps, device="cuda")
+            if bad:
+                e[5, 7, 30] = np.inf
+            z = torch.full(shape, np.nan, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            ctx.ma_filter(theta, shape, A.FP64, e.data_ptr(), z.data_ptr())
+            ctx.synchronize()
+            got.append(z.cpu().numpy())
+    bound = 2 * theta.size * 2.0 ** -53 * (1.0 + np.abs(theta).sum()) * np.abs(eps).max()
+    assert np.max(np.abs(got[0][:4] - got[1][:4])) <= bound
+    assert np.isposinf(got[1][5, 7, 30])
+    reached = np.zeros(shape, bool)
+    reached[:, 7:7 + order[1], 30:30 + order[2]] = True
+    assert np.max(np.abs(got[0] - got[1])[~reached]) <= bound
