@@ -155,8 +155,9 @@ constexpr int kHalfQ = 10;     // slots per lane: mm <= 320
 constexpr int kHalfWarps = 4;  // warps (segments) per CTA
 constexpr int kHalfMaxN = 2 * 32 * kHalfQ;
 
+// (mm > 2: half_four reads up to x[t + 2] of a step before it exists)
 __host__ __device__ inline bool half_set(const arma_mt_params& p) {
-	return p.nn == 2 * p.mm && p.mm <= 32 * kHalfQ;
+	return p.nn == 2 * p.mm && p.mm > 2 && p.mm <= 32 * kHalfQ;
 }
 
 // One step of the warp generator: slots of step s from those of steps s-2 (a)
@@ -676,7 +677,7 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 	// are many, one CTA each when they are few; the others one CTA each in the
 	// general form
 	auto half = [&](const SegJob& j) {
-		return half_set(j.p) && j.p.mm > 2 && j.count < (1ull << 30) &&
+		return half_set(j.p) && j.count < (1ull << 30) &&
 		       j.offset < (1ull << 30) && j.first < (1ull << 40);
 	};
 	std::stable_partition(seg.begin(), seg.end(), half);

@@ -56,6 +56,12 @@ def test_shapes(ctx, nn, mm, rr, n):
     check(ctx, shaped(nn, mm, rr, 0x9908b0df), 4, n)
 
 
+# windows too short for the four-step recurrence, over several jumps
+@pytest.mark.parametrize("nn,mm,rr", [(2, 1, 3), (4, 2, 1), (6, 3, 1)])
+def test_shortest_windows(ctx, nn, mm, rr):
+    check(ctx, shaped(nn, mm, rr, 0x9908b0df), 4, 7 * SEG + 11)
+
+
 def test_many_segments_by_warp(ctx):
     """More than six segments per SM: 900 streams of 2^18 words and one longer,
     through a batch's noise of two surfaces (the longer one cut)."""
