@@ -505,6 +505,10 @@ const uint32_t* jump_table(Ctx* c, const arma_mt_params& p, int e) {
 	return g_tables.emplace(key, d).first->second;
 }
 
+// Dynamic shared memory a jump can have: the CTA's most less the kernel's sums.
+constexpr size_t kJumpSmem = 227 * 1024 - sizeof(uint32_t) * kJumpSpan;
+size_t jump_smem(const arma_mt_params& p) { return sizeof(uint32_t) * size_t(jump_words(p)); }
+
 // Streams up to this length stay one segment: 85 us for its one CTA.
 constexpr unsigned long long kWhole = 1ull << 18;
 
@@ -571,8 +575,9 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 			continue;
 		}
 		K[q] = int(segments_of(total, v[q], log2_seg));
-		// not a full-period set: one sequential segment
-		if (K[q] > 1 && !jump_table(c, jobs[q].p, v[q])) K[q] = 1;
+		// one sequential segment where the jump's words do not fit in shared memory
+		// or no polynomial of the state's degree was found
+		if (K[q] > 1 && (jump_smem(jobs[q].p) > kJumpSmem || !jump_table(c, jobs[q].p, v[q]))) K[q] = 1;
 		if (K[q] > 1) nstates += size_t(K[q]) * jobs[q].p.nn;
 		if (K[q] > 1) Kmax = std::max(Kmax, K[q]);
 	}
@@ -612,7 +617,7 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 		size_t smem = 0;
 		for (size_t q = 0; q < jobs.size(); ++q)
 			if (K[q] > 1 && !ready[q])
-				smem = std::max(smem, sizeof(uint32_t) * size_t(jump_words(jobs[q].p)));
+				smem = std::max(smem, jump_smem(jobs[q].p));
 		std::vector<JumpJob> jj;
 		std::vector<size_t> level_at(levels + 1, 0);  // level lv: entries from level_at[lv + 1] on
 		for (int lv = levels - 1; lv >= 0; --lv) {

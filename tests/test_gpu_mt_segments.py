@@ -62,6 +62,12 @@ def test_shortest_windows(ctx, nn, mm, rr):
     check(ctx, shaped(nn, mm, rr, 0x9908b0df), 4, 7 * SEG + 11)
 
 
+@pytest.mark.parametrize("n", [1 << 19, 5 << 18])
+def test_state_too_large_to_jump(ctx, n):
+    """A state whose jump does not fit in shared memory: one sequential segment."""
+    check(ctx, shaped(2000, 1000, 5, 0x9908b0df), 4, n)
+
+
 def test_many_segments_by_warp(ctx):
     """More than six segments per SM: 900 streams of 2^18 words and one longer,
     through a batch's noise of two surfaces (the longer one cut)."""
