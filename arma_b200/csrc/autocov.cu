@@ -330,12 +330,6 @@ columns_kernel(double2* __restrict__ w, int cols, int band, const double2* __res
 	}
 }
 
-template <class K>
-void allow_smem(K* kernel, size_t bytes) {
-	ARMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                   int(bytes)));
-}
-
 // Points of a band: enough bands for four per SM, within [kAcLeast, kAcBand].
 int band_points(Ctx* c, long long total) {
 	return int(std::min<long long>(kAcBand, std::max<long long>(kAcLeast, total / (4ll * c->num_sms))));

@@ -114,6 +114,18 @@ struct Divider {
 	__device__ int div(int q) const { return m ? int(__umulhi(unsigned(q), m)) : q; }
 };
 
+// Lets launches of a kernel with `fixed` bytes of static shared memory take the
+// rest of what a CTA can have.  The attribute belongs to the function on the
+// device, which all contexts share: it is the same from every call, so that none
+// lowers it between another thread's call and its launch.
+constexpr size_t kSmemOptin = 227 * 1024;
+template <class K>
+void allow_smem(K* kernel, size_t bytes, size_t fixed = 0) {
+	ARMA_REQUIRE(bytes + fixed <= kSmemOptin, ARMA_ECUDA, "the kernel's shared memory does not fit");
+	ARMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                                   int(kSmemOptin - fixed)));
+}
+
 // cudaMemcpyAsync that counts the bytes a context moves between host and
 // device (arma_ctx_transfer_bytes).
 inline cudaError_t copy_async(Ctx* c, void* dst, const void* src, size_t bytes,
