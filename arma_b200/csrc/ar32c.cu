@@ -737,6 +737,8 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 	}
 }
 
+constexpr size_t kStaticSmem = 256;  // no less than ar32c_kernel has: ticket, progress, lo rows
+
 size_t smem_bytes(int pt, int px, int py) {
 	const Layout l = tile_layout(pt, px, py);
 	return sizeof(float) * (size_t(l.slots) * l.slot_sz + 2 * size_t(l.taps) + TX * HS + TX * SW +
@@ -830,8 +832,7 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task) * tasks.size(),
 	                              cudaMemcpyHostToDevice, c->stream));
 	ARMA_CUDA_TRY(cudaMemsetAsync(d_ticket, 0, sizeof(int), c->stream));
-	ARMA_CUDA_TRY(cudaFuncSetAttribute(ar32c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                   int(smem)));
+	allow_smem(ar32c_kernel, smem, kStaticSmem);
 	int per_sm = 0;
 	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel, NTHREADS,
 	                                                            smem));
@@ -963,12 +964,12 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 	if (cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
 	    cudaSuccess)
 		return fail(ARMA_ECUDA, "shared-memory limit query failed");
-	if (smem > size_t(smem_optin))
+	if (smem + kStaticSmem > size_t(smem_optin))
 		return fail(ARMA_ENOTSUP, "AR order needs more shared memory than the device has");
 	unsigned char* base = static_scratch(dev);
 	if (!base) return fail(ARMA_ECUDA, "cudaGetSymbolAddress of the static scratch failed");
 	if (cudaFuncSetAttribute(ar32c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                         int(smem)) != cudaSuccess)
+	                         int(kSmemOptin - kStaticSmem)) != cudaSuccess)
 		return fail(ARMA_ECUDA, "cudaFuncSetAttribute failed");
 	float* d_coef = reinterpret_cast<float*>(base + kOffCoef);
 	// the context path's tables (hi/lo split, lo-row selection, H), built into

@@ -506,7 +506,7 @@ const uint32_t* jump_table(Ctx* c, const arma_mt_params& p, int e) {
 }
 
 // Dynamic shared memory a jump can have: the CTA's most less the kernel's sums.
-constexpr size_t kJumpSmem = 227 * 1024 - sizeof(uint32_t) * kJumpSpan;
+constexpr size_t kJumpSmem = kSmemOptin - sizeof(uint32_t) * kJumpSpan;
 size_t jump_smem(const arma_mt_params& p) { return sizeof(uint32_t) * size_t(jump_words(p)); }
 
 // Streams up to this length stay one segment: 85 us for its one CTA.
@@ -639,8 +639,7 @@ void mt_batch(Ctx* c, const std::vector<MtJob>& jobs, int log2_seg, std::vector<
 		                              cudaMemcpyHostToDevice, c->stream));
 		mt_seed_kernel<<<int(ps.size()), 32, 0, c->stream>>>(d_ps, d_seeds, d_src, d_dst);
 		c->launches += 1;
-		ARMA_CUDA_TRY(cudaFuncSetAttribute(mt_jump_kernel,
-		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		allow_smem(mt_jump_kernel, smem, sizeof(uint32_t) * kJumpSpan);
 		for (int lv = levels - 1; lv >= 0; --lv) {
 			const size_t at = level_at[lv + 1], n = level_at[lv] - at;
 			if (n == 0) continue;

@@ -648,6 +648,7 @@ __device__ __forceinline__ double exp_near(double x, const double* tab) {
 }
 
 constexpr int kExpTable = 64;
+constexpr size_t kExpBytes = sizeof(double) * kExpTable;  // static shared memory of the kernels with a window
 __device__ __forceinline__ void make_exp_table(double* tab) {
 	if (threadIdx.x < kExpTable) tab[threadIdx.x] = exp2(double(threadIdx.x) / kExpTable);
 }
@@ -1387,8 +1388,7 @@ bool launch_real_shape(Ctx* c, const VelSlice<float>* d_sl, int ns, int nx, int 
 		constexpr int NT = M * NY >= 16384 ? 512 : 256;
 		constexpr int L = 2 * M > NY ? 2 * M : NY;
 		const size_t smem = sizeof(float2) * (size_t(M) * RealLd<M, NY>::v + L);
-		ARMA_CUDA_TRY(cudaFuncSetAttribute(velocity_real_kernel<M, NY, NT>,
-		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		allow_smem(velocity_real_kernel<M, NY, NT>, smem, kExpBytes);
 		auto kernel = velocity_real_kernel<M, NY, NT>;
 		if (nz == 1) {
 			kernel<<<ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, depth, spectra, kRealAll, 0);
@@ -1552,8 +1552,7 @@ bool launch_velocity_real(Ctx* c, const VelSlice<float>* d_sl, int ns, int nx, i
 	if (nx == 256 && ny == 256) {  // two CTAs per slice
 		constexpr int M = 128, NY = 256, NT = 512, H = M / 2;
 		const size_t smem = sizeof(float2) * (size_t(H) * RealLd<H, NY>::v + 256);
-		ARMA_CUDA_TRY(cudaFuncSetAttribute(velocity_real2_kernel<M, NY, NT>,
-		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		allow_smem(velocity_real2_kernel<M, NY, NT>, smem, kExpBytes);
 		velocity_real2_kernel<M, NY, NT><<<2 * ns, NT, smem, c->stream>>>(d_sl, d_k, d_z, nz, depth,
 		                                                                  spectra);
 		return true;
@@ -1734,12 +1733,9 @@ void velocity_general(Ctx* c, const VelSlice<T>* d_sl, int ns, int nx, int ny, c
 	const size_t s2 = sizeof(V) * ((nz > 1 ? 2 : 1) * size_t(nx) * CB + nx) +
 	                  sizeof(int) * (size_t(nx) + CB);
 	const size_t s3 = sizeof(V) * (size_t(R + 1) * (ny + 1) + ny);
-	ARMA_CUDA_TRY(cudaFuncSetAttribute(vel_rows_fwd<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                   int(s1)));
-	ARMA_CUDA_TRY(cudaFuncSetAttribute(vel_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                   int(s2)));
-	ARMA_CUDA_TRY(cudaFuncSetAttribute(vel_rows_inv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                   int(s3)));
+	allow_smem(vel_rows_fwd<T>, s1);
+	allow_smem(vel_cols<T>, s2, kExpBytes);
+	allow_smem(vel_rows_inv<T>, s3);
 	const int bands = (nx + R - 1) / R, cbands = (ny + CB - 1) / CB;
 	vel_rows_fwd<T><<<dim3(bands, ns), 256, s1, c->stream>>>(d_sl, nx, ny, R, py, A);
 	vel_cols<T><<<dim3(cbands, ns), 256, s2, c->stream>>>(nx, ny, px, py, CB, d_k, d_z, nz, depth,
@@ -1780,8 +1776,7 @@ void velocity_slices(Ctx* c, const std::vector<VelSlice<T>>& slices, int nx, int
 		const int nseg = std::max(ny * p0, nx * p1);
 		const size_t fw_smem = seg_region_bytes(std::max(nseg, fwarps)) +
 		                       sizeof(T) * size_t(fwarps) * fw_tiles<T>() * 32 * kFwTile;
-		ARMA_CUDA_TRY(cudaFuncSetAttribute(factor_waves_kernel<T>,
-		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(fw_smem)));
+		allow_smem(factor_waves_kernel<T>, fw_smem);
 		factor_waves_kernel<T><<<2 * ns, 32 * fwarps, fw_smem, c->stream>>>(d_sl, nx, ny, p0, p1, d_k);
 	}
 	ARMA_CUDA_TRY(cudaGetLastError());
@@ -1800,8 +1795,7 @@ void velocity_slices(Ctx* c, const std::vector<VelSlice<T>>& slices, int nx, int
 	}
 	if (sizeof(T) == sizeof(float) && n2 <= kFuseMax) {
 		const size_t smem = sizeof(float2) * (size_t(nx) * (ny + 1) + nx + ny) + sizeof(int) * (nx + ny);
-		ARMA_CUDA_TRY(cudaFuncSetAttribute(velocity_fused_kernel,
-		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+		allow_smem(velocity_fused_kernel, smem, kExpBytes);
 		float2* spectra =
 		    nz > 1 ? static_cast<float2*>(scratch_take(c, sizeof(float2) * n2 * ns)) : nullptr;
 		velocity_fused_kernel<<<ns, kFuseThreads, smem, c->stream>>>(

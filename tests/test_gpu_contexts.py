@@ -56,3 +56,47 @@ def autocov(shape):
 
 def test_auto_covariance():
     both(autocov((4, 4, 4)), autocov((3, 1021, 4)))
+
+
+def fp32_filter(order):
+    def make(ctx):
+        z = torch.zeros((2, 8, 8), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        return lambda: ctx.ar_filter(np.zeros(order), z.shape, A.FP32C, z.data_ptr())
+    return make
+
+
+def test_fp32_filter():
+    both(fp32_filter((1, 1, 1)), fp32_filter((16, 13, 13)))
+
+
+def words(params):
+    def make(ctx):
+        out = torch.zeros(1 << 19, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        return lambda: ctx.mt_genrand(params, 1, 1 << 19, out.data_ptr())
+    return make
+
+
+def test_jumps():
+    short, long = A.mt19937_params(), A.mt19937_params()
+    short.nn, short.mm = 16, 8
+    both(words(short), words(long))
+
+
+def potentials(shape, precision, dtype):
+    def make(ctx):
+        z = torch.zeros(shape, dtype=dtype, device="cuda")
+        out = torch.zeros((1, 2) + shape[1:], dtype=dtype, device="cuda")
+        torch.cuda.synchronize()
+        return lambda: ctx.velocity_linear(z.data_ptr(), shape, precision, (1.0, 1.0, 1.0), np.inf,
+                                           [0.0, -1.0], [1], out.data_ptr())
+    return make
+
+
+@pytest.mark.parametrize("precision,dtype,large", [
+    (A.FP64, torch.float64, (3, 1000, 100)), (A.FP32C, torch.float32, (3, 120, 130)),
+    (A.FP32C, torch.float32, (3, 1000, 1000)),
+])
+def test_velocity(precision, dtype, large):
+    both(potentials((3, 5, 6), precision, dtype), potentials(large, precision, dtype))
