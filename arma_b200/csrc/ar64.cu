@@ -712,7 +712,6 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 	                                           flags + tickets, c->d_err);
 	ARMA_CUDA_TRY(cudaGetLastError());
 	c->launches += 1;
-	c->check_pending = true;
 }
 
 }  // namespace

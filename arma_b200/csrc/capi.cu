@@ -278,7 +278,6 @@ void resolve_profile(Ctx* c) {
 
 void check_device_error(Ctx* c) {
 	int h = 0;
-	c->check_pending = false;
 	ARMA_CUDA_TRY(copy_async(c, &h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 	ARMA_CUDA_TRY(cudaStreamSynchronize(c->stream));
 	if (h == DEV_TIMEOUT) {
@@ -367,7 +366,6 @@ int arma_ctx_synchronize(arma_ctx* ctx) {
 	return guard([&] {
 		ARMA_REQUIRE(ctx, ARMA_EINVAL, "null context");
 		ARMA_CUDA_TRY(cudaSetDevice(ctx->c.device));
-		if (ctx->c.check_pending) check_device_error(&ctx->c);
 		ARMA_CUDA_TRY(cudaStreamSynchronize(ctx->c.stream));
 	});
 }
@@ -752,7 +750,7 @@ std::vector<Ar32Surface> ar32_surfaces(Ctx* c, int n, const double* const* phis,
 }
 
 // The FP64 filter of n surfaces in one launch, their coefficients in one
-// upload (a copy from pageable memory has been staged when it returns).
+// upload; its error word is read before anything uses the surfaces.
 void ar64_surfaces(Ctx* c, int n, const double* const* phis, const int* const* orders,
                    const int* const* shapes, double* const* zetas) {
 	std::vector<size_t> off(n + 1, 0);
@@ -771,6 +769,7 @@ void ar64_surfaces(Ctx* c, int n, const double* const* phis, const int* const* o
 	ARMA_CUDA_TRY(copy_async(c, d, buf.data(), sizeof(double) * buf.size(),
 	                         cudaMemcpyHostToDevice, c->stream));
 	launch_ar64(c, s);
+	check_device_error(c);
 }
 
 void ar_filter(Ctx* c, const double* phi, const int order[3], const int shape[3],
@@ -1006,7 +1005,6 @@ void batch(Ctx* c, arma_surface* s, int n, int precision, bool host, bool redo =
 		}
 		ar64_surfaces(c, n, phis.data(), ords.data(), shps.data(), zs.data());
 		renorm_surfaces(c, s, n, precision, dz, host, luts);
-		check_device_error(c);
 		return;
 	}
 	long long* d_pairs = nullptr;

@@ -58,8 +58,6 @@ struct Ctx {
 	uint64_t h2d_bytes = 0;          // bytes copied host -> device through copy_async
 	uint64_t d2h_bytes = 0;          // bytes copied device -> host through copy_async
 	int num_sms = 148;
-	// a launch whose bounded waits nothing has checked yet (check_device_error)
-	bool check_pending = false;
 	// NIT inverse-CDF tables by specification (double table, then float table)
 	std::map<std::vector<double>, double*> nit_tables;
 	// optional per-kernel-class timing with CUDA events on `stream`
@@ -236,8 +234,8 @@ void enqueue_white_noise_batch(Ctx* c, const std::vector<NoiseSpec>& specs, int 
                                long long* d_pairs);
 
 // FP64 exact-order AR filter of a batch of surfaces, in place (ar64.cu).
-// Asynchronous; the error word of its bounded waits is left for the next
-// check_device_error.
+// Asynchronous: the caller reads the error word of its bounded waits
+// (check_device_error).
 struct Ar64Surface {
 	int nt, nx, ny;
 	int pt, px, py;

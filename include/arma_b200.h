@@ -74,8 +74,6 @@ int arma_last_error(char* buf, size_t len);
 int arma_ctx_create(int device, arma_ctx** out);
 int arma_ctx_destroy(arma_ctx* ctx);
 int arma_ctx_set_stream(arma_ctx* ctx, void* cuda_stream);
-/* Waits for the context's stream; ARMA_ETIMEDOUT when a bounded device wait of
- * an earlier asynchronous call ran out. */
 int arma_ctx_synchronize(arma_ctx* ctx);
 /* Kernel launches issued through this context since creation (counter). */
 int arma_ctx_launch_count(arma_ctx* ctx, uint64_t* count);
@@ -205,7 +203,8 @@ int arma_white_noise(arma_ctx* ctx, const arma_mt_params* p, uint32_t seed,
  * ARMA_FP64 follows the reference's summation order exactly;
  * ARMA_FP32C runs the compensated FP32 tile wavefront, for orders with
  * px <= 17, py <= 13 and pt * px <= 221 (others: ARMA_ENOTSUP).  Either
- * form takes orders of at most 16 per axis. */
+ * form takes orders of at most 16 per axis and returns when it has run and its
+ * bounded device waits have been checked (ARMA_ETIMEDOUT). */
 int arma_ar_filter(arma_ctx* ctx, const double* phi, const int order[3],
                    const int shape[3], int precision, void* d_zeta);
 
@@ -316,8 +315,7 @@ typedef struct {
 /* White noise + AR filter (+ renormalisation) for n independent surfaces.
  * Both precisions run all surfaces in one persistent launch (ARMA_FP64: a
  * launch per tile shape, and per hyperplane for models whose coefficients are
- * not finite); a device wait of the FP64 filter that ran out is reported by the
- * next arma_ctx_synchronize. */
+ * not finite); ARMA_ETIMEDOUT when a bounded device wait ran out. */
 int arma_batch_generate(arma_ctx* ctx, arma_surface* surfaces, int n,
                         int precision);
 /* Same, writing each surface into a HOST buffer (d_zeta is then a host
