@@ -547,8 +547,8 @@ class Context:
                                                 zsp, len(zs)))
 
     def selftest_wait(self):
-        """The filter's bounded wait on a flag nothing sets: raises ArmaError
-        (ARMA_ETIMEDOUT) after about a second; the context stays usable."""
+        """The filters' bounded waits on a tile that never runs: raises ArmaError
+        (ARMA_ETIMEDOUT) after some milliseconds; the context stays usable."""
         _check(lib().arma_selftest_wait(self._h))
 
     def auto_covariance(self, d_in: int, shape, precision: int, d_out: int):

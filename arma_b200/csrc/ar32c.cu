@@ -88,7 +88,7 @@ constexpr int HUNITS = 2 * HPAIR; // H work units per tile slice (<= NCOMP)
 constexpr int PS = 2 * R + 4;     // partial record stride (bank spread)
 static_assert(TX == 16 && TY == 4 * R && HUNITS <= NCOMP, "H work-unit table assumes 16 x 4R tiles");
 constexpr int kMaxTapRows = MAXO * (TX + 1);  // (k, i) tap rows per model: pt * px
-constexpr long long kSpinLimit = 1ll << 24;
+constexpr int kSpinLimit = 1 << 24;
 
 struct Task {
 	int nt, nx, ny, pt, px, py;
@@ -96,6 +96,7 @@ struct Task {
 	int given_tx;  // tile rows [0, given_tx) are given (an x-strip's upper band): read, never written
 	int tiles_x, tiles_y;
 	int ticket_base;
+	int polls;  // of the neighbours without progress before the wait gives up
 	float* zeta;
 	const float* phi;     // hi part, pt*px*py
 	const float* phi_lo;  // lo part: phi - hi, pt*px*py
@@ -183,19 +184,6 @@ __device__ bool flags_reached(const int* f0, const int* f1, const int* f2, int n
 	seen[1] = f1 ? b : INT_MAX;
 	seen[2] = f2 ? c : INT_MAX;
 	return a >= need && b >= need && c >= need;
-}
-
-// Waits for that; gives up after kSpinLimit polls (or when another CTA already
-// gave up) and reports DEV_TIMEOUT; returns false then.
-__device__ bool wait_flags(const int* f0, const int* f1, const int* f2, int need, int* seen,
-                           int* err) {
-	for (long long it = 0; it < kSpinLimit; ++it) {
-		if (flags_reached(f0, f1, f2, need, seen)) return true;
-		if ((it & 63) == 63 && *((volatile int*)err) != DEV_OK) return false;
-		__nanosleep(64);
-	}
-	atomicExch(err, DEV_TIMEOUT);
-	return false;
 }
 
 // zeta = H * S over the quarter plane of one tile, cut into work units of
@@ -340,9 +328,8 @@ struct Progress {
 //   halo, a slice ahead of them: once slice t-2 is done (the last to
 //   read the old contents of slot t) it clears slot t and, when the three
 //   neighbour tiles have published slice t, loads slice t's halo.
-// Waiting for the neighbours runs out after kSpinLimit rounds without
-// progress: the error word is set, the tile runs on without its halo, and
-// the call fails.
+// Waiting for the neighbours runs out after the task's polls without progress:
+// the error word is set, the tile runs on without its halo, and the call fails.
 __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Layout& L, float* ring,
                                        Progress* sh, int* err) {
 	const int lane = threadIdx.x & 31;
@@ -374,7 +361,10 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 		}
 		if (t >= tk.nt || done < t - 1) {
 			++idle;  // the compute warps are at work: they end every slice
-			if (idle > 64 * kSpinLimit) break;
+			if (idle > 64ll * kSpinLimit) {
+				if (lane == 0) atomicExch(err, DEV_TIMEOUT);
+				break;
+			}
 			__nanosleep(100);
 			continue;
 		}
@@ -389,7 +379,7 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 		if (lane == 0) {
 			ok = flags_reached(fW, fN, fNW, t + 1, seen) ? 1 : 0;
 			if (!ok && (idle & 63) == 63 && *((volatile int*)err) != DEV_OK) ok = 1;
-			if (!ok && idle > kSpinLimit) {
+			if (!ok && idle > tk.polls) {
 				atomicExch(err, DEV_TIMEOUT);
 				ok = 1;
 			}
@@ -633,7 +623,7 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 		// the barrier's previous round is over once the publication warp has
 		// left it (it waits for nothing but these barriers)
 		for (long long it = 0; *((volatile int*)&sh->published) < t + 1 - PUB_BARS; ++it)
-			if (it == 64 * kSpinLimit) {
+			if (it == 64ll * kSpinLimit) {
 				atomicExch(err, DEV_TIMEOUT);
 				break;
 			}
@@ -758,20 +748,31 @@ int ctas_per_sm(double tiles, int sms, int most) {
 	return n < 3 ? std::min(n, most) : most;
 }
 
-// The filter's neighbour wait on a tile flag that nothing publishes: it runs
-// out after kSpinLimit polls and sets the error word (the failure path of
-// every bounded wait, exercised on purpose).
-__global__ void wait_selftest_kernel(const int* flag, int* err) {
-	int seen[3] = {-1, -1, -1};
-	if (threadIdx.x == 0) wait_flags(flag, nullptr, nullptr, 1, seen, err);
-}
-
 }  // namespace
 
-void launch_wait_selftest(Ctx* c) {
-	int* flag = static_cast<int*>(scratch_take(c, sizeof(int)));
-	ARMA_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), c->stream));
-	wait_selftest_kernel<<<1, 32, 0, c->stream>>>(flag, c->d_err);
+void launch_ar32c_starved(Ctx* c) {
+	const size_t words = 2 * size_t(TX) * 2 * TY + 2 * 2 + size_t(TX) * TY;
+	auto* zeta = static_cast<float*>(scratch_take(c, sizeof(float) * words));
+	int* flags = static_cast<int*>(scratch_take(c, sizeof(int) * 3));
+	ARMA_CUDA_TRY(cudaMemsetAsync(zeta, 0, sizeof(float) * words, c->stream));
+	Task t{};
+	t.nt = 2; t.nx = TX; t.ny = 2 * TY;
+	t.pt = t.px = 1; t.py = 2;
+	t.tiles_x = 1; t.tiles_y = 2;
+	t.polls = kStarvedPolls;
+	t.zeta = zeta;
+	t.phi = zeta + 2 * size_t(TX) * 2 * TY;
+	t.phi_lo = t.phi + 2;
+	t.h = t.phi_lo + 2;
+	t.flags = flags;
+	auto* d_task = static_cast<Task*>(scratch_take(c, sizeof(Task)));
+	const int start[3] = {0, 0, 1};  // nothing published; the next ticket: the second tile
+	ARMA_CUDA_TRY(copy_async(c, d_task, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
+	ARMA_CUDA_TRY(copy_async(c, flags, start, sizeof(start), cudaMemcpyHostToDevice, c->stream));
+	const size_t smem = smem_bytes(t.pt, t.px, t.py);
+	allow_smem(ar32c_kernel, smem, kStaticSmem);
+	ProfScope prof_(c, "ar32c");
+	ar32c_kernel<<<1, NTHREADS, smem, c->stream>>>(d_task, 1, 2, flags + 2, c->d_err);
 	ARMA_CUDA_TRY(cudaGetLastError());
 	c->launches += 1;
 }
@@ -821,6 +822,7 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 		t.given_tx = s.given_tx;
 		t.tiles_x = s.tiles_x; t.tiles_y = s.tiles_y;
 		t.ticket_base = total;
+		t.polls = kSpinLimit;
 		t.zeta = s.zeta; t.phi = s.phi; t.phi_lo = s.phi_lo; t.h = s.h;
 		t.flags = flags + foff;
 		foff += size_t(s.tiles_x) * s.tiles_y;
@@ -984,6 +986,7 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 	t.given_tx = 0;
 	t.tiles_x = tiles_x; t.tiles_y = tiles_y;
 	t.ticket_base = 0;
+	t.polls = kSpinLimit;
 	t.zeta = d_zeta;
 	t.phi = d_coef;
 	t.phi_lo = d_coef + P;

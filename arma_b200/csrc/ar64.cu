@@ -48,7 +48,7 @@
 namespace armab {
 namespace {
 
-constexpr long long kSpinLimit = 1ll << 24;
+constexpr int kSpinLimit = 1 << 24;
 constexpr size_t kSmemLimit = 227 * 1024 - 64;  // less the kernel's static shared memory
 constexpr int kMaxAhead = 4;   // steps of halo kept ahead of their use
 constexpr int kUpstream = 5;   // tiles a tile's halo can come from
@@ -61,6 +61,7 @@ struct Task64 {
 	int nbx, nc;      // tile rows, tiles per tile row
 	int ticket_base;
 	int ahead;        // halo steps kept ahead of their use
+	int polls;        // of the upstream tiles without progress before the wait gives up
 	double* zeta;
 	const double* phi;
 	int* flags;       // per tile: the step (t + u) up to which it is done
@@ -249,7 +250,7 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 		// the steps n .. hi whose upstream values are there and whose ring
 		// slots are free (and whose barriers' previous round is over)
 		int hi = -1;
-		for (long long it = 0; it < kSpinLimit; ++it) {
+		for (int it = 0; it < tk.polls; ++it) {
 			const int freed = ld_acquire_cta(&sh->done) + tk.ahead;
 			hi = min(freed, known == INT_MAX ? INT_MAX : known - U0);
 			hi = min(__reduce_min_sync(0xffffffffu, hi), steps - 1);
@@ -416,7 +417,7 @@ __device__ __forceinline__ void compute_tile(const Task64& tk, int bx, int c, co
 		// the barrier's previous round is over once the publication warp has
 		// left it (it waits for nothing but these barriers)
 		for (long long it = 0; *((volatile int*)&sh->published) < n + 1 - kPubBars; ++it)
-			if (it == kSpinLimit * 64) {
+			if (it == 64ll * kSpinLimit) {
 				atomicCAS(err, DEV_OK, DEV_TIMEOUT);
 				break;
 			}
@@ -533,7 +534,7 @@ __device__ __forceinline__ void compute_pairs(const Task64& tk, int bx, int c, c
 		// the barrier's previous round is over once the publication warp has
 		// left it (it waits for nothing but these barriers)
 		for (long long it = 0; *((volatile int*)&sh->published) < n + 1 - kPubBars; ++it)
-			if (it == kSpinLimit * 64) {
+			if (it == 64ll * kSpinLimit) {
 				atomicCAS(err, DEV_OK, DEV_TIMEOUT);
 				break;
 			}
@@ -685,6 +686,7 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 		t.nc = tiles_per_row(TX, TU, s.ny);
 		t.ticket_base = int(tickets);
 		t.ahead = ahead_of(TX, TU, s);
+		t.polls = kSpinLimit;
 		t.zeta = s.zeta;
 		t.phi = s.phi;
 		t.flags = nullptr;
@@ -750,6 +752,37 @@ void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces) {
 	if (!groups[1].empty()) launch_tiles<8, 16, 1>(c, groups[1]);
 	if (!groups[2].empty()) launch_tiles<4, 16, 1>(c, groups[2]);
 	if (!groups[3].empty()) launch_tiles<8, 8, 1>(c, groups[3]);
+}
+
+void launch_ar64_starved(Ctx* c) {
+	constexpr int TX = 8, TU = 16;
+	const size_t cells = 2 * size_t(TX) * TU;
+	auto* zeta = static_cast<double*>(scratch_take(c, sizeof(double) * (cells + 2)));
+	int* flags = static_cast<int*>(scratch_take(c, sizeof(int) * 3));
+	ARMA_CUDA_TRY(cudaMemsetAsync(zeta, 0, sizeof(double) * (cells + 2), c->stream));
+	Task64 t{};
+	t.nt = 2; t.nx = TX; t.ny = TU;
+	t.pt = t.px = 1; t.py = 2;
+	t.nbx = 1;
+	t.nc = tiles_per_row(TX, TU, TU);  // 2
+	t.ahead = 1;
+	t.polls = kStarvedPolls;
+	t.zeta = zeta;
+	t.phi = zeta + cells;
+	t.flags = flags;
+	auto* d_task = static_cast<Task64*>(scratch_take(c, sizeof(Task64)));
+	const int start[3] = {0, 0, 1};  // nothing done; the next ticket: the second tile
+	ARMA_CUDA_TRY(copy_async(c, d_task, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
+	ARMA_CUDA_TRY(copy_async(c, flags, start, sizeof(start), cudaMemcpyHostToDevice, c->stream));
+	const size_t smem = layout64(TX, TU, t.pt, t.px, t.py, t.ahead).bytes;
+	ARMA_CUDA_TRY(cudaFuncSetAttribute(ar64_tile_kernel<TX, TU, 1>,
+	                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                                   int(kSmemLimit)));
+	ProfScope prof_(c, "ar64");
+	ar64_tile_kernel<TX, TU, 1><<<1, TX * TU + 64, smem, c->stream>>>(d_task, 1, t.nc, flags + 2,
+	                                                                  c->d_err);
+	ARMA_CUDA_TRY(cudaGetLastError());
+	c->launches += 1;
 }
 
 }  // namespace armab

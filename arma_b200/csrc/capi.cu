@@ -1564,8 +1564,18 @@ int arma_selftest_wait(arma_ctx* ctx) {
 		ARMA_REQUIRE(ctx, ARMA_EINVAL, "null argument");
 		ARMA_CUDA_TRY(cudaSetDevice(ctx->c.device));
 		scratch_begin(&ctx->c, 0);
-		launch_wait_selftest(&ctx->c);
-		check_device_error(&ctx->c);  // ARMA_ETIMEDOUT, error word cleared
+		launch_ar32c_starved(&ctx->c);
+		bool gave_up = false;
+		try {
+			check_device_error(&ctx->c);  // ARMA_ETIMEDOUT, error word cleared
+		} catch (const Error& e) {
+			if (e.code != ARMA_ETIMEDOUT) throw;
+			gave_up = true;
+		}
+		ARMA_REQUIRE(gave_up, ARMA_ECUDA, "the FP32 filter's wait did not give up");
+		launch_ar64_starved(&ctx->c);
+		check_device_error(&ctx->c);
+		throw Error{ARMA_ECUDA, "the FP64 filter's wait did not give up"};
 	});
 }
 
