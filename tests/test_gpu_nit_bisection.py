@@ -53,3 +53,29 @@ def test_same_as_evaluating_every_point(ctx, dist, params, interval, eps, max_it
         torch.cuda.synchronize()
         apply(few)
         assert np.array_equal(few.cpu().numpy(), big[at:at + 8].cpu().numpy(), equal_nan=True), at
+
+
+@pytest.mark.parametrize("params,interval", [
+    ([1e6, -3e5], (-10.0, 10.0)), ([1e9, 0.0], (0.9, 1.1)), ([-1e9, 3.0], (-1.02, -0.97)),
+    ([3e6, 0.0], (0.99, 1.01)), ([1e12, 0.0], (0.5, 1.2)), ([3e6, 0.0], (0.9999, 1.0001)),
+    ([0.0, 4e5], (1.7, 1.75)),
+])
+def test_values_far_above_one(ctx, params, interval):
+    """A Gram-Charlier CDF of such skewness and kurtosis rounds at its own size, not
+    at that of a probability: to the last bit of the bracket."""
+    import torch
+    rng = np.random.default_rng(5)
+    v = rng.normal(0.0, 1.2, 1 << 18)
+    big = torch.from_numpy(v.copy()).cuda()
+    few = torch.from_numpy(v.copy()).cuda()
+    torch.cuda.synchronize()
+
+    def apply(z):
+        ctx.nit_apply(GRAM, params, 1.2, A.NIT_BISECTION, z.numel(), A.FP64, z.data_ptr(),
+                      interval=interval, eps=1e-300, max_iter=200)
+
+    apply(big)
+    for part in few.split(256):  # too few points for cubics: every F(c) evaluated
+        apply(part)
+    ctx.synchronize()
+    assert torch.equal(big, few)
