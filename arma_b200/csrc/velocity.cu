@@ -654,8 +654,8 @@ __device__ __forceinline__ void make_exp_table(double* tab) {
 }
 
 // window_fixed for entries where nothing overflows (-350 <= l z <= 0, l finite and
-// positive: no entry of the reference's formula is non-finite there, so no fix
-// applies): with A = exp(l z), B = exp(-l (z + 2 h)) the window is 4 pi (A + B) /
+// positive, h positive and not NaN: no entry of the reference's formula is
+// non-finite there, so no fix applies): with A = exp(l z), B = exp(-l (z + 2 h)) the window is 4 pi (A + B) /
 // (1 + A B), the same quotient as above.  At infinite depth one exponential and no
 // division: 30 FP64 instructions instead of 78 (400 x 128 x 128 FP32 at four
 // depths spent 205 us of the solver's 540 on windows).
@@ -670,7 +670,7 @@ __device__ __forceinline__ double window_at(int i, int j, int nx, int ny, double
 	const double az = k2Pi * sqrt(s2) * z;
 	// exp(-l z)^2 overflows: the entry is non-finite, 0 away from row and column 0
 	if (az < -360.0 && i > 0 && j > 0) return 0.0;
-	if (s2 > 0.0 && s2 <= DBL_MAX && az <= 0.0 && az >= -350.0) {
+	if (s2 > 0.0 && s2 <= DBL_MAX && az <= 0.0 && az >= -350.0 && h >= 0.0) {
 		const double A = exp_near(az, tab);
 		if (h == INFINITY) return k2Pi * 2.0 * A;
 		// -l (z + 2 h), formed as the reference's -2 l h minus l z

@@ -73,3 +73,20 @@ def test_more_depths_than_a_grid_dimension(ctx):
     assert torch.isfinite(whole).all()
     for part in (slice(0, 3), slice(65533, 65540)):
         assert torch.equal(whole[:, part], run(zs[part]))
+
+
+@pytest.mark.parametrize("shape", [(3, 32, 16), (2, 37, 53), (3, 256, 256)])
+def test_depth_that_is_not_a_number(ctx, shape):
+    """Every entry of the window is then non-finite and becomes 0, as in the reference."""
+    rng = np.random.default_rng(4)
+    zeta = rng.standard_normal(shape)
+    ref = O.velocity_linear(zeta, (1.0, 1.0, 1.0), np.nan, [-1.0, -2.0], [1])
+    assert not ref.any()
+    for prec, dt in [(A.FP64, torch.float64), (A.FP32C, torch.float32)]:
+        z = torch.tensor(zeta, dtype=dt, device="cuda")
+        out = torch.ones(ref.shape, dtype=dt, device="cuda")
+        torch.cuda.synchronize()
+        ctx.velocity_linear(z.data_ptr(), shape, prec, (1.0, 1.0, 1.0), np.nan, [-1.0, -2.0], [1],
+                            out.data_ptr())
+        ctx.synchronize()
+        assert not out.cpu().numpy().any()
