@@ -753,18 +753,25 @@ std::vector<Ar32Surface> ar32_surfaces(Ctx* c, int n, const double* const* phis,
 // upload; its error word is read before anything uses the surfaces.
 void ar64_surfaces(Ctx* c, int n, const double* const* phis, const int* const* orders,
                    const int* const* shapes, double* const* zetas) {
+	// lags that no point of the surface has are left out: the reference's sums are
+	// truncated at the array's start, and a tile pays for them as for any other
+	// (1 x 500 x 500 of order 16^3: 170 ms with them, 14 without)
+	auto lags = [&](int k, int axis) { return std::min(orders[k][axis], shapes[k][axis]); };
 	std::vector<size_t> off(n + 1, 0);
 	for (int k = 0; k < n; ++k)
-		off[k + 1] = off[k] + size_t(orders[k][0]) * orders[k][1] * orders[k][2];
+		off[k + 1] = off[k] + size_t(lags(k, 0)) * lags(k, 1) * lags(k, 2);
 	std::vector<double> buf(off[n]);
 	double* d = static_cast<double*>(scratch_take(c, sizeof(double) * buf.size()));
 	std::vector<Ar64Surface> s(n);
 	for (int k = 0; k < n; ++k) {
-		std::copy(phis[k], phis[k] + (off[k + 1] - off[k]), buf.begin() + off[k]);
-		const bool finite = std::all_of(phis[k], phis[k] + (off[k + 1] - off[k]),
-		                                [](double v) { return std::isfinite(v); });
-		s[k] = Ar64Surface{shapes[k][0], shapes[k][1], shapes[k][2], orders[k][0], orders[k][1],
-		                   orders[k][2], zetas[k],     d + off[k],   finite};
+		const int pt = lags(k, 0), px = lags(k, 1), py = lags(k, 2);
+		double* p = buf.data() + off[k];
+		for (int a = 0; a < pt; ++a)
+			for (int b = 0; b < px; ++b)
+				p = std::copy_n(phis[k] + (size_t(a) * orders[k][1] + b) * orders[k][2], py, p);
+		const bool finite = std::all_of(buf.data() + off[k], p, [](double v) { return std::isfinite(v); });
+		s[k] = Ar64Surface{shapes[k][0], shapes[k][1], shapes[k][2], pt,    px, py,
+		                   zetas[k],     d + off[k],   finite};
 	}
 	ARMA_CUDA_TRY(copy_async(c, d, buf.data(), sizeof(double) * buf.size(),
 	                         cudaMemcpyHostToDevice, c->stream));

@@ -73,6 +73,19 @@ def test_coefficients_that_are_not_finite(ctx, bad):
     assert np.isfinite(got).any() and np.array_equal(got, ref, equal_nan=True)
 
 
+@pytest.mark.parametrize("shape,order", [((1, 1, 1), (16, 16, 16)), ((2, 30, 40), (9, 4, 4)),
+                                         ((20, 3, 40), (3, 8, 4)), ((20, 40, 2), (3, 4, 11)),
+                                         ((1, 50, 50), (5, 6, 7))])
+def test_order_longer_than_the_surface(ctx, shape, order):
+    """Lags that no point has, infinite ones among them, are not part of any sum."""
+    rng = np.random.default_rng(8)
+    phi, eps = model(order, rng), rng.standard_normal(shape)
+    outside = np.logical_or.reduce([i >= n for i, n in zip(np.indices(order), shape)])
+    phi[outside] = np.inf
+    ref = O.ar_filter(eps, phi)
+    assert np.isfinite(ref).all() and np.array_equal(run(ctx, eps, phi), ref)
+
+
 def test_noise_that_is_not_finite(ctx):
     rng = np.random.default_rng(7)
     phi, eps = model((3, 3, 4), rng), rng.standard_normal((6, 20, 37))
