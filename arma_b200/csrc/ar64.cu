@@ -65,6 +65,7 @@ struct Task64 {
 	double* zeta;
 	const double* phi;
 	int* flags;       // per tile: the step (t + u) up to which it is done
+	const int* tiles; // tile of each ticket, or null: row by row
 };
 
 // Layout of a tile's shared memory (doubles unless said otherwise).
@@ -567,7 +568,9 @@ ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
 			if (tasks[mid].ticket_base <= ticket) lo = mid; else hi = mid - 1;
 		}
 		const Task64 tk = tasks[lo];
-		const int bx = (ticket - tk.ticket_base) / tk.nc, c = (ticket - tk.ticket_base) % tk.nc;
+		int tile = ticket - tk.ticket_base;
+		if (tk.tiles) tile = tk.tiles[tile];
+		const int bx = tile / tk.nc, c = tile % tk.nc;
 		const Layout64 L = layout64(TX, TU, tk.pt, tk.px, tk.py, tk.ahead);
 		double* ring = smem64 + kLead;
 		double* sphi = ring + size_t(L.slot) * L.depth;
@@ -664,6 +667,14 @@ int ahead_of(int tx, int tu, const Ar64Surface& s) {
 	return 0;
 }
 
+// A surface's tiles by anti-diagonals (2 bx + c ascending): the tiles that a tile's
+// halo comes from (bx, c - 1 and c - 2; bx - 1, c - 1 to c + 1) come before it.
+void diagonal_order(int nbx, int nc, int* list) {
+	for (int key = 0; key <= 2 * (nbx - 1) + nc - 1; ++key)
+		for (int b = std::max(0, (key - nc + 2) / 2); b < nbx && 2 * b <= key; ++b)
+			*list++ = b * nc + key - 2 * b;
+}
+
 int tiles_per_row(int tx, int tu, int ny) { return (ny + tx - 1 + tu - 1) / tu; }
 
 template <int TX, int TU, int CELLS>
@@ -690,6 +701,7 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 		t.zeta = s.zeta;
 		t.phi = s.phi;
 		t.flags = nullptr;
+		t.tiles = nullptr;
 		tickets += (long long)t.nbx * t.nc;
 		ARMA_REQUIRE(tickets < INT_MAX / 4, ARMA_EINVAL, "surface too large");
 		smem = std::max(smem, layout64(TX, TU, s.pt, s.px, s.py, t.ahead).bytes);
@@ -698,10 +710,6 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 	// step counters of every tile, then the ticket counter
 	int* flags = static_cast<int*>(scratch_take(c, sizeof(int) * (size_t(tickets) + 1)));
 	ARMA_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t(tickets) + 1), c->stream));
-	for (Task64& t : tasks) t.flags = flags + t.ticket_base;
-	auto* d_tasks = static_cast<Task64*>(scratch_take(c, sizeof(Task64) * tasks.size()));
-	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task64) * tasks.size(),
-	                         cudaMemcpyHostToDevice, c->stream));
 	constexpr int threads = TX * TU / CELLS + 64;
 	auto kernel = ar64_tile_kernel<TX, TU, CELLS>;
 	ARMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -710,6 +718,27 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
 	ARMA_REQUIRE(per_sm > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
 	const int grid = int(std::min<long long>(tickets, (long long)per_sm * c->num_sms));
+	// Where the tiles do not all run at once they are handed out by anti-diagonals:
+	// row by row, the CTAs hold a band of tile rows end to end, and a surface of few
+	// slices is swept once per band (ms, row by row / by anti-diagonals: 1 x 1000 x
+	// 1000 of order 1 x 16 x 1 51.7 / 10.1, 16 x 500 x 500 of 10^3 28.2 / 13.7, 200^3 of
+	// 10^3 7.7 / 6.7; all at once, 64 x 30 x 1000 of 3 x 6 x 6 2.24 / 2.41).
+	int* d_tiles = nullptr;
+	std::vector<int> tiles;
+	if (tickets > grid) {
+		tiles.resize(size_t(tickets));
+		for (const Task64& t : tasks) diagonal_order(t.nbx, t.nc, tiles.data() + t.ticket_base);
+		d_tiles = static_cast<int*>(scratch_take(c, sizeof(int) * tiles.size()));
+		ARMA_CUDA_TRY(copy_async(c, d_tiles, tiles.data(), sizeof(int) * tiles.size(),
+		                         cudaMemcpyHostToDevice, c->stream));
+	}
+	for (Task64& t : tasks) {
+		t.flags = flags + t.ticket_base;
+		t.tiles = d_tiles ? d_tiles + t.ticket_base : nullptr;
+	}
+	auto* d_tasks = static_cast<Task64*>(scratch_take(c, sizeof(Task64) * tasks.size()));
+	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task64) * tasks.size(),
+	                         cudaMemcpyHostToDevice, c->stream));
 	kernel<<<grid, threads, smem, c->stream>>>(d_tasks, int(tasks.size()), int(tickets),
 	                                           flags + tickets, c->d_err);
 	ARMA_CUDA_TRY(cudaGetLastError());

@@ -53,6 +53,17 @@ def test_tiles_bit_exact(ctx, shape, order):
     assert np.array_equal(run(ctx, eps, phi), O.ar_filter(eps, phi))
 
 
+# more tiles than the device holds at once: handed out by anti-diagonals
+@pytest.mark.parametrize("shape,order", [
+    ((2, 800, 810), (2, 3, 3)), ((1, 60, 9000), (1, 2, 4)), ((1, 9000, 60), (1, 4, 2)),
+    ((3, 700, 500), (1, 16, 1)), ((2, 300, 290), (2, 12, 12)), ((12, 330, 340), (3, 10, 10)),
+])
+def test_more_tiles_than_run_at_once(ctx, shape, order):
+    rng = np.random.default_rng(sum(shape))
+    phi, eps = model(order, rng), rng.standard_normal(shape)
+    assert np.array_equal(run(ctx, eps, phi), O.ar_filter(eps, phi))
+
+
 def test_own_lag_and_overwritten_noise(ctx):
     """A coefficient at lag (0, 0, 0) multiplies the point's own noise."""
     rng = np.random.default_rng(5)
