@@ -195,7 +195,8 @@ constexpr int kHaloBars = kMaxAhead + 1, kPubBars = 8;
 constexpr int kBarHalo = 1, kBarPub = kBarHalo + kHaloBars;
 static_assert(kBarPub + kPubBars <= 16, "named barriers");
 
-// The halo warp: a list of the halo's cells inside the surface, then step
+// The halo warp: a list of the halo's cells inside the surface (column; row in the
+// ring, place in its slot and lag in steps, 12, 12 and 8 bits), then step
 // after step their new values.  A cell in row x' and column u' = U0 + d is read
 // from column max(U0, u' + b) of the tile on (b = X0 - x' rows above it, 0
 // beside it), so step n of the tile brings in its value of t = n - max(0, d +
@@ -228,7 +229,7 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 		const unsigned m = __ballot_sync(0xffffffffu, ok);
 		if (ok)
 			cells[count + __popc(m & ((1u << lane) - 1))] =
-			    make_int2(x * tk.ny + y, (row * L.ld + col) << 8 | rel);
+			    make_int2(y, row << 20 | (row * L.ld + col) << 8 | rel);
 		count += __popc(m);
 	}
 	__syncwarp();
@@ -245,6 +246,8 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 	}
 	constexpr int kThreads = NC + 32;
 	const long long plane = (long long)tk.nx * tk.ny;
+	// row 0 of the ring (a plane can have more than 2^31 points)
+	const double* const top_row = tk.zeta + (long long)(X0 - (px - 1)) * tk.ny;
 	int n = 0;
 	bool failed = false;
 	while (n < steps) {
@@ -289,8 +292,8 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 					const int2 cell = cells[e];
 					const int rel = cell.y & 255, t = st - rel;
 					if (t >= 0 && t < tk.nt) {
-						at[b] = (sm - rel + (sm < rel ? L.depth : 0)) * L.slot + (cell.y >> 8);
-						v[b] = __ldcg(tk.zeta + t * plane + cell.x);
+						at[b] = (sm - rel + (sm < rel ? L.depth : 0)) * L.slot + (cell.y >> 8 & 0xfff);
+						v[b] = __ldcg(top_row + t * plane + (long long)(cell.y >> 20) * tk.ny + cell.x);
 					}
 					e += 32;
 				}

@@ -64,6 +64,24 @@ def test_more_tiles_than_run_at_once(ctx, shape, order):
     assert np.array_equal(run(ctx, eps, phi), O.ar_filter(eps, phi))
 
 
+def test_planes_of_more_than_2_31_points(ctx):
+    """Noise in the last corner of a plane whose points have 64-bit offsets: the
+    filter there is that of the corner alone."""
+    import torch
+    n, corner = 46400, 100
+    rng = np.random.default_rng(9)
+    phi, eps = model((1, 4, 3), rng), rng.standard_normal((1, corner, corner))
+    z = torch.zeros((1, n, n), dtype=torch.float64, device="cuda")
+    z[0, n - corner:, n - corner:] = torch.from_numpy(eps[0]).cuda()
+    torch.cuda.synchronize()
+    ctx.ar_filter(phi, z.shape, A.FP64, z.data_ptr())
+    assert not z[0, :n - corner].any() and not z[0, :, :n - corner].any()
+    got = z[0, n - corner:, n - corner:].cpu().numpy()
+    del z
+    torch.cuda.empty_cache()
+    assert np.array_equal(got, O.ar_filter(eps, phi)[0])
+
+
 def test_own_lag_and_overwritten_noise(ctx):
     """A coefficient at lag (0, 0, 0) multiplies the point's own noise."""
     rng = np.random.default_rng(5)
