@@ -361,11 +361,16 @@ void ma_filter_impl(Ctx* c, const double* theta, const int order[3], const int s
 	// the taps filled up to four, and their offsets
 	const size_t mma_smem = smem + 2 * 3 * kMaTT * sizeof(T) + (size_t(rows_per) * py + 3) * sizeof(int);
 	// matrix instructions take the 8 time steps whole, also on the slices that reach
-	// only some, and taps by fours: 256 x 128 x 128, us, by them / scalar: order 20 x
-	// 10 x 10 800 / 987, 4 x 5 x 5 118 / 116, 3 x 10 x 10 305 / 298, 1 x 10 x 10 247 /
-	// 218, 8 x 1 x 1 48 / 40; 24 x 128 x 20 of 6 x 6 x 6 55 / 63; 64 x 32 x 32 of 5 x
-	// 3 x 3 30 / 31
-	const bool mma = sizeof(T) == 8 && pt >= 5 && px * py >= 8 && mma_smem <= size_t(kMaSmemLimit);
+	// only some, and taps by fours, filled up with zeros: where more than a fifth as
+	// many zeros are added they need more slices.  By them / scalar, 100 x 128 x 128
+	// (and 64 x 32 x 32): order 4 x 10 x 10 1.00 (0.94), 5 x 10 x 10 0.98 (0.91), 20 x 10
+	// x 10 0.80; 5 x 5 x 2 (two zeros to ten taps) 1.10 (1.00), 12 x 5 x 2 1.00 (0.91); 8
+	// x 3 x 3 (three to nine) 1.14 (1.00), 20 x 3 x 3 1.05 (0.96).  Taps of four rows, at
+	// py = 1, meet in the same banks: 8 x 10 x 1 1.31, 32 x 8 x 1 1.14.
+	const int taps = px * py, zeros = (taps + 3) / 4 * 4 - taps;
+	const int slices = 5 * zeros <= taps ? 5 : 16;
+	const bool mma = sizeof(T) == 8 && pt >= slices && taps >= 8 && (py > 1 || px == 1) &&
+	                 mma_smem <= size_t(kMaSmemLimit);
 	if (mma)
 		ARMA_CUDA_TRY(cudaFuncSetAttribute(ma_mma_kernel,
 		                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kMaSmemLimit));

@@ -32,6 +32,15 @@ def test_against_direct_sum(shape, order):
     assert np.max(np.abs(z.cpu().numpy() - O.ma_filter(eps, theta))) <= bound
 
 
+# tap counts that four does not divide and taps of single columns, on both sides
+@pytest.mark.parametrize("shape,order", [
+    ((20, 17, 65), (15, 3, 3)), ((20, 17, 65), (16, 3, 3)), ((9, 17, 65), (5, 5, 2)),
+    ((9, 33, 30), (8, 10, 1)), ((9, 33, 30), (32, 8, 1)),
+])
+def test_sides_of_the_rule(shape, order):
+    test_against_direct_sum(shape, order)
+
+
 def test_noise_that_is_not_finite_stays_where_it_reaches():
     """An infinity in slice 5 meets, in the scalar form, the time steps 4 and later
     of its block: the steps before it keep their values."""
