@@ -335,10 +335,12 @@ int band_points(Ctx* c, long long total) {
 	return int(std::min<long long>(kAcBand, std::max<long long>(kAcLeast, total / (4ll * c->num_sms))));
 }
 
-// Columns per CTA: about `points` points, at least four (64 bytes of a row), the
-// bands of a row equally wide.
-int columns_per_band(int n, int cols, int points) {
-	const int most = std::max(4, points / n);
+// Columns per CTA: about `points` points, at least four (64 bytes of a row) where
+// those make a CTA per SM, fewer down to one where not (lines of a large prime are
+// long and few: 1021 x 2 x 2 976 -> 411 us); the bands of a row equally wide.
+int columns_per_band(Ctx* c, long long slabs, int n, int cols, int points) {
+	const int least = int(std::min(4ll, std::max(1ll, slabs * cols / c->num_sms)));
+	const int most = std::max(least, points / n);
 	const int bands = (cols + most - 1) / most;
 	return (cols + bands - 1) / bands;
 }
@@ -346,7 +348,7 @@ int columns_per_band(int n, int cols, int points) {
 template <int WHAT>
 void launch_columns(Ctx* c, double2* w, long long slabs, int cols, const double2* roots,
                     const AcPlan& P) {
-	const int band = columns_per_band(P.n, cols, band_points(c, slabs * P.n * cols));
+	const int band = columns_per_band(c, slabs, P.n, cols, band_points(c, slabs * P.n * cols));
 	const size_t smem = ac_smem(P, P.n * band);
 	allow_smem(columns_kernel<WHAT>, smem);
 	columns_kernel<WHAT><<<dim3((cols + band - 1) / band, unsigned(slabs)), kAcThreads, smem,
