@@ -55,6 +55,7 @@
 // cache).
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -89,6 +90,9 @@ constexpr int PS = 2 * R + 4;     // partial record stride (bank spread)
 static_assert(TX == 16 && TY == 4 * R && HUNITS <= NCOMP, "H work-unit table assumes 16 x 4R tiles");
 constexpr int kMaxTapRows = MAXO * (TX + 1);  // (k, i) tap rows per model: pt * px
 constexpr int kSpinLimit = 1 << 24;
+constexpr int kAheadPolls = 1 << 12;
+constexpr int kAhead = 2;          // slices, where tiles keep pace
+constexpr int kHeavyTaps = 400;    // taps whose tiles crowd each other out on an SM
 
 struct Task {
 	int nt, nx, ny, pt, px, py;
@@ -315,6 +319,13 @@ __host__ __device__ inline Layout tile_layout(int pt, int px, int py) {
 	return l;
 }
 
+// The slices that both tiles below (x + 1, y + 1) have published; t where none has
+// published any: a tile that is not yet at work holds nobody back.
+__device__ int slices_below(const int* fE, const int* fS, int t) {
+	const int e = fE ? *((volatile const int*)fE) : 0, s = fS ? *((volatile const int*)fS) : 0;
+	return e > 0 && s > 0 ? min(e, s) : e + s > 0 ? e + s : t;
+}
+
 // Where the two sides of a CTA stand on the current tile.
 struct Progress {
 	int done;       // slices finished by the compute warps
@@ -330,6 +341,9 @@ struct Progress {
 //   neighbour tiles have published slice t, loads slice t's halo.
 // Waiting for the neighbours runs out after the task's polls without progress:
 // the error word is set, the tile runs on without its halo, and the call fails.
+// PACE: a tile of many taps, more than kAhead slices ahead of the tiles below it, also
+// holds back its next halo, for kAheadPolls polls at most: it waits for nobody, it gives way.
+template <bool PACE>
 __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Layout& L, float* ring,
                                        Progress* sh, int* err) {
 	const int lane = threadIdx.x & 31;
@@ -343,7 +357,11 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 	const int* fN = (by > 0) ? tk.flags + bx * tk.tiles_y + by - 1 : nullptr;
 	const int* fNW = (bx > 0 && by > 0) ? tk.flags + (bx - 1) * tk.tiles_y + by - 1 : nullptr;
 	int* own_flag = tk.flags + bx * tk.tiles_y + by;
+	const int* fE = by + 1 < tk.tiles_y ? own_flag + 1 : nullptr;
+	const int* fS = bx + 1 < tk.tiles_x ? own_flag + tk.tiles_y : nullptr;
 	int seen[3] = {-1, -1, -1};
+	const bool pace = PACE && tk.pt * tk.px * tk.py >= kHeavyTaps;
+	int below = 0;              // slices that the tiles below have published
 	int pub = tk.t0;            // slices published
 	int t = tk.t0;              // the next slice to bring the halo of
 	bool cleared = false;       // slot t
@@ -378,6 +396,10 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 		int ok = 1;
 		if (lane == 0) {
 			ok = flags_reached(fW, fN, fNW, t + 1, seen) ? 1 : 0;
+			if (pace && ok && t > below + kAhead && idle < kAheadPolls) {
+				below = slices_below(fE, fS, t);
+				ok = t <= below + kAhead;
+			}
 			if (!ok && (idle & 63) == 63 && *((volatile int*)err) != DEV_OK) ok = 1;
 			if (!ok && idle > tk.polls) {
 				atomicExch(err, DEV_TIMEOUT);
@@ -632,7 +654,9 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 	}
 }
 
-// A tile's coefficients, H, zeroed ring and history into shared memory.
+// A tile's coefficients, H, zeroed ring and history into shared memory.  (PACE: each
+// kernel its own copy, whose registers are allocated with the kernel's.)
+template <bool PACE>
 __device__ __noinline__ void stage_tile(const Task& tk, int bx, int by, const Layout& L,
                                         float* smem, unsigned char* s_lo) {
 	const int tid = threadIdx.x;
@@ -672,8 +696,36 @@ __device__ __noinline__ void stage_tile(const Task& tk, int bx, int by, const La
 	}
 }
 
+// Tile k of a grid of a x b tiles by anti-diagonals: a tile's neighbours x - 1, y - 1
+// and both come before it.  For tiles that do not all run at once: those that do are
+// a front across the surface.  (Row by row they are a band of rows end to end, of
+// which only the stretch that nt slices span is at work: 60 x 1024 x 2048 of order 4^3
+// 5.0 / 3.1 ms, 20 x 96 x 1920 of 8^3 0.86 / 0.52, the batch of 256 surfaces 48.3 /
+// 48.3; all at once, 512 x 256 x 256 of 10^3 5.06 / 5.08.)
+__device__ int2 diagonal_tile(int k, int a, int b) {
+	const int m = min(a, b), head = m * (m - 1) / 2;  // tiles on diagonals shorter than m
+	const bool tail = k >= a * b - head;              // the last ones mirror the first
+	if (tail) k = a * b - 1 - k;
+	int2 t;
+	if (k < head) {
+		int d = int((sqrtf(8.0f * float(k) + 1.0f) - 1.0f) * 0.5f);
+		while (d * (d + 1) / 2 > k) --d;
+		while ((d + 1) * (d + 2) / 2 <= k) ++d;
+		t.x = k - d * (d + 1) / 2;
+		t.y = d - t.x;
+	} else {
+		const int q = k - head, d = m - 1 + q / m;
+		t.x = a <= b ? q % m : d - q % m;
+		t.y = d - t.x;
+	}
+	return tail ? make_int2(a - 1 - t.x, b - 1 - t.y) : t;
+}
+
 // One launch for the whole batch: each ticket's surface selects the
-// instantiation for its tap count py (warp-uniform switch).
+// instantiation for its tap count py (warp-uniform switch).  PACE: its tiles of many
+// taps keep pace (a kernel of its own: with the choice in one kernel, 512 x 256 x 256 of
+// order 10^3, which makes none, took 1 % longer).
+template <bool PACE>
 __global__ void __launch_bounds__(NTHREADS, 3)
 ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
              int* __restrict__ ticket_counter, int* __restrict__ err) {
@@ -697,7 +749,12 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 		}
 		const Task tk = tasks[lo];
 		const int local = ticket - tk.ticket_base;
-		const int bx = local / tk.tiles_y, by = local % tk.tiles_y;
+		int bx = local / tk.tiles_y, by = local % tk.tiles_y;
+		if (total_tickets > int(gridDim.x)) {
+			const int2 tile = diagonal_tile(local, tk.tiles_x, tk.tiles_y);
+			bx = tile.x;
+			by = tile.y;
+		}
 		if (bx < tk.given_tx) {
 			// a given tile (the band above an x-strip, holding the upper strip's
 			// finished values): published as complete for every slice at once
@@ -705,14 +762,14 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 			continue;
 		}
 		const Layout L = tile_layout(tk.pt, tk.px, tk.py);
-		stage_tile(tk, bx, by, L, smem, s_lo);
+		stage_tile<PACE>(tk, bx, by, L, smem, s_lo);
 		if (tid == 0) {
 			sh.done = tk.t0;
 			sh.published = tk.t0;
 		}
 		__syncthreads();
 		if (tid >= NCOMP) {
-			halo_warp(tk, bx, by, L, smem, &sh, err);
+			halo_warp<PACE>(tk, bx, by, L, smem, &sh, err);
 		} else {
 			switch (tk.py) {
 #define ARMA_PY_CASE(N) case N: compute_tile<N>(tk, bx, by, L, smem, s_lo, &sh, err); break;
@@ -735,17 +792,68 @@ size_t smem_bytes(int pt, int px, int py) {
 	                        std::max(GROUP * R, HUNITS * PS));
 }
 
-// CTAs per SM for a launch.  `tiles` is the work of all tiles over that of the
-// longest chain of slices: how many tiles run at once if none waits for an SM.
-// CTAs that share an SM slow each other's chains (a slice takes 1.35 and 1.8 times
-// as long with two and three), so below about one tile per SM the longest chain
-// is left an SM to itself, and below 2.4 it shares with one other.  Measured with
-// one, two and three per SM (ms): 0.9 tiles per SM 3.9 / 5.4 / 5.3; 1.3 7.8 / 6.4
-// / 8.4; 1.7 6.4 / 4.8 / 6.0; 2.0 11.2 / 8.6 / 8.9; 2.8 15.0 / 10.6 / 10.1; 3.1
-// 13.3 / 9.5 / 8.8; 4.8 28.4 / 20.2 / 19.0.
-int ctas_per_sm(double tiles, int sms, int most) {
-	const int n = tiles < 1.1 * sms ? 1 : tiles < 2.4 * sms ? 2 : 3;
-	return n < 3 ? std::min(n, most) : most;
+// What decides how many CTAs share an SM.
+struct Load32 {
+	double tiles = 0, work = 0, spread = 0;  // tiles, their slices' cost, their surfaces' chains
+	double chain = 0;                        // the longest chain of slices, by cost
+	int taps = 0;                            // of its surface
+	// a surface's wavefront needs about nt + tiles_x + tiles_y slice steps, each
+	// proportional to its taps and what H and the sums cost (as much as 160 taps)
+	static double chain_of(const Ar32Surface& s) {
+		return double(s.nt - s.t0 + s.tiles_x + s.tiles_y) * (s.pt * s.px * s.py + 160);
+	}
+	void add(const Ar32Surface& s) {
+		const double n = double(s.tiles_x - s.given_tx) * s.tiles_y, c = chain_of(s);
+		tiles += n;
+		work += n * (s.nt - s.t0) * (s.pt * s.px * s.py + 160);
+		spread += n * c;
+		if (c > chain) taps = s.pt * s.px * s.py;
+		chain = std::max(chain, c);
+	}
+};
+
+// CTAs per SM for a launch, of `most` that fit.  Of all tiles, work / chain are at
+// work at once if none waits for an SM.  CTAs that share an SM slow each other's
+// chains, so below about one such tile per SM the longest chain is left an SM to
+// itself.  In a batch of different surfaces it shares with one other below 2.4.
+// Measured with one, two and three per SM (ms): 0.9 tiles per SM 3.9 / 5.4 / 5.3;
+// 1.3 7.8 / 6.4 / 8.4; 1.7 6.4 / 4.8 / 6.0; 2.0 11.2 / 8.6 / 8.9; 2.8 15.0 / 10.6 /
+// 10.1; 3.1 13.3 / 9.5 / 8.8; 4.8 28.4 / 20.2 / 19.0.
+// Where all chains are about as long as the longest (one surface, or many alike),
+// tiles that find no SM make a second wave as long as the first: the fewest waves,
+// each by what its CTAs slow each other (light orders less).  Where few slices leave
+// many of the tiles waiting for their first, only those at work count.  200 slices,
+// with one, two and three per SM (ms): 196 tiles of 10^3 3.7 / 3.1 / 3.1, 400 5.5 /
+// 7.1 / 4.6, 576 7.2 / 7.2 / 10.5, 900 of 4^3 - / 3.1 / 2.7; 60 slices: 400 tiles of
+// 10^3 1.7 / 2.0 / 1.7, of 4^3 0.68 / 0.68 / 0.77.
+int ctas_per_sm(const Load32& l, int sms, int most) {
+	const double at_work = l.work / l.chain;
+	if (at_work < 1.1 * sms) return 1;
+	if (l.spread < 0.9 * l.tiles * l.chain) return at_work < 2.4 * sms ? std::min(2, most) : most;
+	const bool heavy = l.taps >= kHeavyTaps;
+	const double slowed[] = {1.0, heavy ? 1.6 : 1.45, heavy ? 2.45 : 1.9};
+	const bool few = at_work < (heavy ? 0.5 : 0.75) * l.tiles;  // at work at once
+	int best = 1;
+	double least = HUGE_VAL;
+	for (int n = 1; n <= std::min(most, 3); ++n) {
+		const double waves = few ? std::max(1.0, at_work / (n * sms)) : std::ceil(l.tiles / (n * sms));
+		const double time = slowed[n - 1] * waves;
+		if (time < least) {
+			least = time;
+			best = n;
+		}
+	}
+	return best;
+}
+
+// Whether tiles of many taps are to keep pace with the tiles below them: where
+// several run on an SM and all run at once, one that is far ahead takes the SM from
+// the tiles that the rest of the surface waits for (200 slices of 10^3, 400 tiles on
+// 444 CTAs: 4.6 to 7.3 ms, 4.7 keeping pace).  Tiles that wait for a CTA are the
+// sooner served the sooner others end, and tiles of few taps lose more than they gain
+// (1^3, 400 tiles: 1.6 / 2.2 ms).
+bool keep_pace(int taps, int total, int grid, int sms) {
+	return taps >= kHeavyTaps && total <= grid && total > sms;
 }
 
 }  // namespace
@@ -770,9 +878,9 @@ void launch_ar32c_starved(Ctx* c) {
 	ARMA_CUDA_TRY(copy_async(c, d_task, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
 	ARMA_CUDA_TRY(copy_async(c, flags, start, sizeof(start), cudaMemcpyHostToDevice, c->stream));
 	const size_t smem = smem_bytes(t.pt, t.px, t.py);
-	allow_smem(ar32c_kernel, smem, kStaticSmem);
+	allow_smem(ar32c_kernel<false>, smem, kStaticSmem);
 	ProfScope prof_(c, "ar32c");
-	ar32c_kernel<<<1, NTHREADS, smem, c->stream>>>(d_task, 1, 2, flags + 2, c->d_err);
+	ar32c_kernel<false><<<1, NTHREADS, smem, c->stream>>>(d_task, 1, 2, flags + 2, c->d_err);
 	ARMA_CUDA_TRY(cudaGetLastError());
 	c->launches += 1;
 }
@@ -793,20 +901,15 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 		order[k] = int(k);
 		smem = std::max(smem, smem_bytes(s.pt, s.px, s.py));
 	}
-	// longest dependency chains first: a surface's wavefront needs about
-	// nt + tiles_x + tiles_y slice steps, each proportional to its taps and
-	// what H and the sums cost (as much as 160 taps)
-	auto slice = [](const Ar32Surface& s) { return double(s.pt * s.px * s.py + 160); };
-	auto chain = [&](const Ar32Surface& s) {
-		return (s.nt - s.t0 + s.tiles_x + s.tiles_y) * slice(s);
-	};
-	std::sort(order.begin(), order.end(),
-	          [&](int a, int b) { return chain(surfaces[a]) > chain(surfaces[b]); });
+	// longest dependency chains first
+	std::sort(order.begin(), order.end(), [&](int a, int b) {
+		return Load32::chain_of(surfaces[a]) > Load32::chain_of(surfaces[b]);
+	});
 	size_t nflags = 0;
-	double work = 0;
+	Load32 load;
 	for (const auto& s : surfaces) {
 		nflags += size_t(s.tiles_x) * s.tiles_y;
-		work += double(s.tiles_x - s.given_tx) * s.tiles_y * (s.nt - s.t0) * slice(s);
+		load.add(s);
 	}
 	int* flags = static_cast<int*>(scratch_take(c, sizeof(int) * nflags));
 	ARMA_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * nflags, c->stream));
@@ -829,24 +932,28 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 		total += s.tiles_x * s.tiles_y;
 		tasks.push_back(t);
 	}
+	allow_smem(ar32c_kernel<false>, smem, kStaticSmem);
+	int per_sm = 0;
+	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel<false>,
+	                                                            NTHREADS, smem));
+	ARMA_REQUIRE(per_sm > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
+	per_sm = c->tuning.ar_ctas_per_sm > 0 ? std::min(per_sm, c->tuning.ar_ctas_per_sm)
+	                                      : ctas_per_sm(load, c->num_sms, per_sm);
+	const int grid = std::min(total, per_sm * c->num_sms);
+	int taps = 0;
+	for (const Task& t : tasks) taps = std::max(taps, t.pt * t.px * t.py);
 	Task* d_tasks = static_cast<Task*>(scratch_take(c, sizeof(Task) * tasks.size()));
 	int* d_ticket = static_cast<int*>(scratch_take(c, sizeof(int)));
 	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task) * tasks.size(),
 	                              cudaMemcpyHostToDevice, c->stream));
 	ARMA_CUDA_TRY(cudaMemsetAsync(d_ticket, 0, sizeof(int), c->stream));
-	allow_smem(ar32c_kernel, smem, kStaticSmem);
-	int per_sm = 0;
-	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel, NTHREADS,
-	                                                            smem));
-	ARMA_REQUIRE(per_sm > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
-	if (c->tuning.ar_ctas_per_sm > 0)
-		per_sm = std::min(per_sm, c->tuning.ar_ctas_per_sm);
-	else if (!order.empty())
-		per_sm = ctas_per_sm(work / chain(surfaces[order[0]]), c->num_sms, per_sm);
-	const int grid = std::min(total, per_sm * c->num_sms);
 	ProfScope prof_(c, "ar32c");
-	ar32c_kernel<<<grid, NTHREADS, smem, c->stream>>>(d_tasks, int(tasks.size()), total, d_ticket,
-	                                                  c->d_err);
+	auto kernel = ar32c_kernel<false>;
+	if (keep_pace(taps, total, grid, c->num_sms)) {
+		kernel = ar32c_kernel<true>;
+		allow_smem(kernel, smem, kStaticSmem);
+	}
+	kernel<<<grid, NTHREADS, smem, c->stream>>>(d_tasks, int(tasks.size()), total, d_ticket, c->d_err);
 	ARMA_CUDA_TRY(cudaGetLastError());
 	c->launches += 1;
 }
@@ -970,9 +1077,10 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 		return fail(ARMA_ENOTSUP, "AR order needs more shared memory than the device has");
 	unsigned char* base = static_scratch(dev);
 	if (!base) return fail(ARMA_ECUDA, "cudaGetSymbolAddress of the static scratch failed");
-	if (cudaFuncSetAttribute(ar32c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                         int(kSmemOptin - kStaticSmem)) != cudaSuccess)
-		return fail(ARMA_ECUDA, "cudaFuncSetAttribute failed");
+	for (auto kernel : {ar32c_kernel<false>, ar32c_kernel<true>})
+		if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                         int(kSmemOptin - kStaticSmem)) != cudaSuccess)
+			return fail(ARMA_ECUDA, "cudaFuncSetAttribute failed");
 	float* d_coef = reinterpret_cast<float*>(base + kOffCoef);
 	// the context path's tables (hi/lo split, lo-row selection, H), built into
 	// host stack memory: 2P + TX*TY <= kMaxCoefFloats floats
@@ -996,12 +1104,15 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 	int* d_err = reinterpret_cast<int*>(base + kOffErr);
 	const int ntiles = tiles_x * tiles_y;
 	int per_sm = 0, sms = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel, NTHREADS, smem) !=
-	        cudaSuccess ||
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel<false>, NTHREADS,
+	                                                  smem) != cudaSuccess ||
 	    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
 		return fail(ARMA_ECUDA, "occupancy query failed");
 	if (per_sm <= 0) return fail(ARMA_ENOTSUP, "AR tile does not fit in shared memory");
-	per_sm = ctas_per_sm(double(ntiles) * t.nt / (t.nt + tiles_x + tiles_y), sms, per_sm);
+	Load32 load;
+	load.add(Ar32Surface{t.nt, t.nx, t.ny, t.pt, t.px, t.py, d_zeta, t.phi, t.phi_lo, t.h, tiles_x,
+	                     tiles_y});
+	per_sm = ctas_per_sm(load, sms, per_sm);
 	const int grid = std::min(ntiles, per_sm * sms);
 	if (cudaMemcpyAsync(base + kOffTask, &t, sizeof(t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 	    cudaMemcpyAsync(d_coef, cbuf, sizeof(float) * ncoef, cudaMemcpyHostToDevice, st) !=
@@ -1011,8 +1122,9 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 		(void)cudaStreamSynchronize(st);  // the staged host buffers are on this stack
 		return fail(ARMA_ECUDA, "staging the allocation-free AR filter failed");
 	}
-	ar32c_kernel<<<grid, NTHREADS, smem, st>>>(reinterpret_cast<const Task*>(base + kOffTask), 1,
-	                                           ntiles, d_ticket, d_err);
+	auto kernel = keep_pace(P, ntiles, grid, sms) ? ar32c_kernel<true> : ar32c_kernel<false>;
+	kernel<<<grid, NTHREADS, smem, st>>>(reinterpret_cast<const Task*>(base + kOffTask), 1, ntiles,
+	                                     d_ticket, d_err);
 	const bool launched = cudaGetLastError() == cudaSuccess;
 	int herr = 0;
 	const bool copied =
