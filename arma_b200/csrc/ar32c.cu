@@ -97,7 +97,10 @@ constexpr int kHeavyTaps = 400;    // taps whose tiles crowd each other out on a
 struct Task {
 	int nt, nx, ny, pt, px, py;
 	int t0;  // slices [0, t0) are history: read, never written
-	int given_tx;  // tile rows [0, given_tx) are given (an x-strip's upper band): read, never written
+	int given_tx : 29;  // tile rows [0, given_tx) are given (an x-strip's upper band): read, never written
+	unsigned lead : 1;  // slices that the halo comes in ahead; 0: no slot of the ring for it
+	unsigned pace : 1;  // tiles run at most kAhead slices ahead of the tiles below them
+	unsigned diagonal : 1;  // tiles handed out by anti-diagonals, else row by row
 	int tiles_x, tiles_y;
 	int ticket_base;
 	int polls;  // of the neighbours without progress before the wait gives up
@@ -309,11 +312,11 @@ struct Layout {
 	int pyp;
 };
 
-__host__ __device__ inline Layout tile_layout(int pt, int px, int py) {
+__host__ __device__ inline Layout tile_layout(int pt, int px, int py, int lead) {
 	Layout l;
 	l.hx = px - 1;
 	l.slot_sz = (TX + px - 1) * W;
-	l.slots = pt + 1;  // the pt slices in use and the next one's halo
+	l.slots = pt + lead;  // the pt slices in use and the next one's halo
 	l.pyp = (py + 3) & ~3;
 	l.taps = pt * px * l.pyp;
 	return l;
@@ -337,13 +340,14 @@ struct Progress {
 //   publish: a barrier orders the compute warps' global stores of the
 //   slices they have finished before the release store of the count;
 //   halo, a slice ahead of them: once slice t-2 is done (the last to
-//   read the old contents of slot t) it clears slot t and, when the three
-//   neighbour tiles have published slice t, loads slice t's halo.
+//   read the old contents of slot t; t-1 in a ring of pt slots) it clears
+//   slot t and, when the three neighbour tiles have published slice t,
+//   loads slice t's halo.
 // Waiting for the neighbours runs out after the task's polls without progress:
 // the error word is set, the tile runs on without its halo, and the call fails.
-// PACE: a tile of many taps, more than kAhead slices ahead of the tiles below it, also
+// A tile that keeps pace, more than kAhead slices ahead of the tiles below it, also
 // holds back its next halo, for kAheadPolls polls at most: it waits for nobody, it gives way.
-template <bool PACE>
+template <bool BY_TASK>
 __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Layout& L, float* ring,
                                        Progress* sh, int* err) {
 	const int lane = threadIdx.x & 31;
@@ -360,7 +364,8 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 	const int* fE = by + 1 < tk.tiles_y ? own_flag + 1 : nullptr;
 	const int* fS = bx + 1 < tk.tiles_x ? own_flag + tk.tiles_y : nullptr;
 	int seen[3] = {-1, -1, -1};
-	const bool pace = PACE && tk.pt * tk.px * tk.py >= kHeavyTaps;
+	const bool pace = BY_TASK && tk.pace;
+	const int lead = BY_TASK ? tk.lead : 1;
 	int below = 0;              // slices that the tiles below have published
 	int pub = tk.t0;            // slices published
 	int t = tk.t0;              // the next slice to bring the halo of
@@ -377,7 +382,7 @@ __device__ __noinline__ void halo_warp(const Task& tk, int bx, int by, const Lay
 			__syncwarp();
 			idle = 0;
 		}
-		if (t >= tk.nt || done < t - 1) {
+		if (t >= tk.nt || done < t - lead) {
 			++idle;  // the compute warps are at work: they end every slice
 			if (idle > 64ll * kSpinLimit) {
 				if (lane == 0) atomicExch(err, DEV_TIMEOUT);
@@ -654,9 +659,9 @@ __device__ __forceinline__ void compute_tile(const Task& tk, int bx, int by, con
 	}
 }
 
-// A tile's coefficients, H, zeroed ring and history into shared memory.  (PACE: each
-// kernel its own copy, whose registers are allocated with the kernel's.)
-template <bool PACE>
+// A tile's coefficients, H, zeroed ring and history into shared memory.  (Each kernel
+// has its own copy, whose registers are allocated with the kernel's.)
+template <bool BY_TASK>
 __device__ __noinline__ void stage_tile(const Task& tk, int bx, int by, const Layout& L,
                                         float* smem, unsigned char* s_lo) {
 	const int tid = threadIdx.x;
@@ -697,11 +702,7 @@ __device__ __noinline__ void stage_tile(const Task& tk, int bx, int by, const La
 }
 
 // Tile k of a grid of a x b tiles by anti-diagonals: a tile's neighbours x - 1, y - 1
-// and both come before it.  For tiles that do not all run at once: those that do are
-// a front across the surface.  (Row by row they are a band of rows end to end, of
-// which only the stretch that nt slices span is at work: 60 x 1024 x 2048 of order 4^3
-// 5.0 / 3.1 ms, 20 x 96 x 1920 of 8^3 0.86 / 0.52, the batch of 256 surfaces 48.3 /
-// 48.3; all at once, 512 x 256 x 256 of 10^3 5.06 / 5.08.)
+// and both come before it.
 __device__ int2 diagonal_tile(int k, int a, int b) {
 	const int m = min(a, b), head = m * (m - 1) / 2;  // tiles on diagonals shorter than m
 	const bool tail = k >= a * b - head;              // the last ones mirror the first
@@ -722,10 +723,11 @@ __device__ int2 diagonal_tile(int k, int a, int b) {
 }
 
 // One launch for the whole batch: each ticket's surface selects the
-// instantiation for its tap count py (warp-uniform switch).  PACE: its tiles of many
-// taps keep pace (a kernel of its own: with the choice in one kernel, 512 x 256 x 256 of
-// order 10^3, which makes none, took 1 % longer).
-template <bool PACE>
+// instantiation for its tap count py (warp-uniform switch).  BY_TASK: lead, pace and
+// order of tiles as the task says, else 1, none and by anti-diagonals where they do not
+// all run at once (a kernel of its own: with the choice in one, 512 x 256 x 256 of order
+// 10^3, which needs none of it, took 1 to 2 % longer).
+template <bool BY_TASK>
 __global__ void __launch_bounds__(NTHREADS, 3)
 ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
              int* __restrict__ ticket_counter, int* __restrict__ err) {
@@ -750,7 +752,7 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 		const Task tk = tasks[lo];
 		const int local = ticket - tk.ticket_base;
 		int bx = local / tk.tiles_y, by = local % tk.tiles_y;
-		if (total_tickets > int(gridDim.x)) {
+		if (BY_TASK ? tk.diagonal : total_tickets > int(gridDim.x)) {
 			const int2 tile = diagonal_tile(local, tk.tiles_x, tk.tiles_y);
 			bx = tile.x;
 			by = tile.y;
@@ -761,15 +763,15 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 			if (tid == 0) st_release(tk.flags + bx * tk.tiles_y + by, tk.nt);
 			continue;
 		}
-		const Layout L = tile_layout(tk.pt, tk.px, tk.py);
-		stage_tile<PACE>(tk, bx, by, L, smem, s_lo);
+		const Layout L = tile_layout(tk.pt, tk.px, tk.py, BY_TASK ? tk.lead : 1);
+		stage_tile<BY_TASK>(tk, bx, by, L, smem, s_lo);
 		if (tid == 0) {
 			sh.done = tk.t0;
 			sh.published = tk.t0;
 		}
 		__syncthreads();
 		if (tid >= NCOMP) {
-			halo_warp<PACE>(tk, bx, by, L, smem, &sh, err);
+			halo_warp<BY_TASK>(tk, bx, by, L, smem, &sh, err);
 		} else {
 			switch (tk.py) {
 #define ARMA_PY_CASE(N) case N: compute_tile<N>(tk, bx, by, L, smem, s_lo, &sh, err); break;
@@ -786,8 +788,8 @@ ar32c_kernel(const Task* __restrict__ tasks, int ntasks, int total_tickets,
 
 constexpr size_t kStaticSmem = 256;  // no less than ar32c_kernel has: ticket, progress, lo rows
 
-size_t smem_bytes(int pt, int px, int py) {
-	const Layout l = tile_layout(pt, px, py);
+size_t smem_bytes(int pt, int px, int py, int lead) {
+	const Layout l = tile_layout(pt, px, py, lead);
 	return sizeof(float) * (size_t(l.slots) * l.slot_sz + 2 * size_t(l.taps) + TX * HS + TX * SW +
 	                        std::max(GROUP * R, HUNITS * PS));
 }
@@ -810,12 +812,14 @@ struct Load32 {
 		if (c > chain) taps = s.pt * s.px * s.py;
 		chain = std::max(chain, c);
 	}
+	double at_work() const { return work / chain; }
+	bool alike() const { return spread >= 0.9 * tiles * chain; }
 };
 
 // CTAs per SM for a launch, of `most` that fit.  Of all tiles, work / chain are at
 // work at once if none waits for an SM.  CTAs that share an SM slow each other's
-// chains, so below about one such tile per SM the longest chain is left an SM to
-// itself.  In a batch of different surfaces it shares with one other below 2.4.
+// chains: in a batch of different surfaces, below about one such tile per SM the
+// longest chain is left an SM to itself, and below 2.4 it shares with one other.
 // Measured with one, two and three per SM (ms): 0.9 tiles per SM 3.9 / 5.4 / 5.3;
 // 1.3 7.8 / 6.4 / 8.4; 1.7 6.4 / 4.8 / 6.0; 2.0 11.2 / 8.6 / 8.9; 2.8 15.0 / 10.6 /
 // 10.1; 3.1 13.3 / 9.5 / 8.8; 4.8 28.4 / 20.2 / 19.0.
@@ -826,16 +830,18 @@ struct Load32 {
 // with one, two and three per SM (ms): 196 tiles of 10^3 3.7 / 3.1 / 3.1, 400 5.5 /
 // 7.1 / 4.6, 576 7.2 / 7.2 / 10.5, 900 of 4^3 - / 3.1 / 2.7; 60 slices: 400 tiles of
 // 10^3 1.7 / 2.0 / 1.7, of 4^3 0.68 / 0.68 / 0.77.
-int ctas_per_sm(const Load32& l, int sms, int most) {
-	const double at_work = l.work / l.chain;
-	if (at_work < 1.1 * sms) return 1;
-	if (l.spread < 0.9 * l.tiles * l.chain) return at_work < 2.4 * sms ? std::min(2, most) : most;
+// More than `with_lead` CTAs only fit without the halo a slice ahead (launch_ar32c): of
+// tiles alike, where they then all run at once.
+int ctas_per_sm(const Load32& l, int sms, int most, int with_lead) {
+	const double at_work = l.at_work();
+	if (!l.alike()) return at_work < 1.1 * sms ? 1 : at_work < 2.4 * sms ? std::min(2, most) : most;
 	const bool heavy = l.taps >= kHeavyTaps;
 	const double slowed[] = {1.0, heavy ? 1.6 : 1.45, heavy ? 2.45 : 1.9};
 	const bool few = at_work < (heavy ? 0.5 : 0.75) * l.tiles;  // at work at once
 	int best = 1;
 	double least = HUGE_VAL;
 	for (int n = 1; n <= std::min(most, 3); ++n) {
+		if (n > with_lead && l.tiles > n * sms) continue;
 		const double waves = few ? std::max(1.0, at_work / (n * sms)) : std::ceil(l.tiles / (n * sms));
 		const double time = slowed[n - 1] * waves;
 		if (time < least) {
@@ -846,14 +852,25 @@ int ctas_per_sm(const Load32& l, int sms, int most) {
 	return best;
 }
 
-// Whether tiles of many taps are to keep pace with the tiles below them: where
-// several run on an SM and all run at once, one that is far ahead takes the SM from
-// the tiles that the rest of the surface waits for (200 slices of 10^3, 400 tiles on
-// 444 CTAs: 4.6 to 7.3 ms, 4.7 keeping pace).  Tiles that wait for a CTA are the
-// sooner served the sooner others end, and tiles of few taps lose more than they gain
-// (1^3, 400 tiles: 1.6 / 2.2 ms).
-bool keep_pace(int taps, int total, int grid, int sms) {
-	return taps >= kHeavyTaps && total <= grid && total > sms;
+// How a launch's tiles share the device, by task.
+//
+// Tiles of many taps keep pace with the tiles below them where several run on an SM
+// and all run at once: one that is far ahead takes the SM from the tiles that the
+// rest of the surface waits for (200 slices of 10^3, 400 tiles on 444 CTAs: 4.6 to 7.3
+// ms, 4.7 keeping pace).  Tiles that wait for a CTA are the sooner served the sooner
+// others end, and tiles of few taps lose more than they gain (1^3, 400 tiles: 1.6 /
+// 2.2 ms).
+//
+// Tiles that do not all run at once are handed out by anti-diagonals, a front across
+// the surface.  Row by row they are a band of rows end to end, of which only the
+// stretch that the slices span is at work (60 x 1024 x 2048 of order 4^3 5.0 / 3.1 ms,
+// 20 x 96 x 1920 of 8^3 0.86 / 0.52; the batch of 256 surfaces 48.3 / 48.3).  Where that
+// is most of it, tiles of many taps crowd each other out less row by row (200 x 384 x
+// 768 of 10^3 6.9 / 7.2).
+void share_device(Task& t, const Load32& l, int total, int grid, int sms) {
+	t.pace = t.pt * t.px * t.py >= kHeavyTaps && total <= grid && total > sms;
+	t.diagonal = total > grid &&
+	             !(l.alike() && l.taps >= kHeavyTaps && l.at_work() >= 0.75 * l.tiles);
 }
 
 }  // namespace
@@ -866,6 +883,7 @@ void launch_ar32c_starved(Ctx* c) {
 	Task t{};
 	t.nt = 2; t.nx = TX; t.ny = 2 * TY;
 	t.pt = t.px = 1; t.py = 2;
+	t.lead = 1;
 	t.tiles_x = 1; t.tiles_y = 2;
 	t.polls = kStarvedPolls;
 	t.zeta = zeta;
@@ -877,7 +895,7 @@ void launch_ar32c_starved(Ctx* c) {
 	const int start[3] = {0, 0, 1};  // nothing published; the next ticket: the second tile
 	ARMA_CUDA_TRY(copy_async(c, d_task, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
 	ARMA_CUDA_TRY(copy_async(c, flags, start, sizeof(start), cudaMemcpyHostToDevice, c->stream));
-	const size_t smem = smem_bytes(t.pt, t.px, t.py);
+	const size_t smem = smem_bytes(t.pt, t.px, t.py, t.lead);
 	allow_smem(ar32c_kernel<false>, smem, kStaticSmem);
 	ProfScope prof_(c, "ar32c");
 	ar32c_kernel<false><<<1, NTHREADS, smem, c->stream>>>(d_task, 1, 2, flags + 2, c->d_err);
@@ -892,14 +910,15 @@ int ar32c_max_tap_rows() { return kMaxTapRows; }
 void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int ty, int) {
 	ARMA_REQUIRE(tx == TX && ty == TY, ARMA_EINVAL, "unsupported AR tile shape");
 	std::vector<int> order(surfaces.size());
-	size_t smem = 0;
+	size_t most_bytes[2] = {0, 0};  // of a tile, by its lead
 	for (size_t k = 0; k < surfaces.size(); ++k) {
 		const Ar32Surface& s = surfaces[k];
 		ARMA_REQUIRE(s.px <= TX + 1 && s.py <= MAXO && s.pt >= 1 && s.px >= 1 && s.py >= 1 &&
 		                 s.pt * s.px <= kMaxTapRows,
 		             ARMA_ENOTSUP, "AR order not supported by the FP32 tile kernel");
 		order[k] = int(k);
-		smem = std::max(smem, smem_bytes(s.pt, s.px, s.py));
+		for (int lead : {0, 1})
+			most_bytes[lead] = std::max(most_bytes[lead], smem_bytes(s.pt, s.px, s.py, lead));
 	}
 	// longest dependency chains first
 	std::sort(order.begin(), order.end(), [&](int a, int b) {
@@ -932,16 +951,30 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 		total += s.tiles_x * s.tiles_y;
 		tasks.push_back(t);
 	}
-	allow_smem(ar32c_kernel<false>, smem, kStaticSmem);
-	int per_sm = 0;
-	ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel<false>,
-	                                                            NTHREADS, smem));
-	ARMA_REQUIRE(per_sm > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
-	per_sm = c->tuning.ar_ctas_per_sm > 0 ? std::min(per_sm, c->tuning.ar_ctas_per_sm)
-	                                      : ctas_per_sm(load, c->num_sms, per_sm);
+	auto fit = [&](size_t bytes) {  // CTAs on an SM
+		allow_smem(ar32c_kernel<false>, bytes, kStaticSmem);
+		int n = 0;
+		ARMA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ar32c_kernel<false>, NTHREADS,
+		                                                            bytes));
+		return n;
+	};
+	// The halo a slice ahead takes a slot of the ring, which costs the largest orders
+	// a CTA per SM: it is given up where that CTA is wanted (200 x 256 x 512 of order 16
+	// x 13 x 9, one CTA with and two without: 6.4 / 5.4 ms; 200 x 320 x 640 of 11 x 10
+	// x 10, two and three: 5.9 / 5.1).
+	const int with_lead = fit(most_bytes[1]);
+	const int most = with_lead < 3 ? fit(most_bytes[0]) : with_lead;
+	ARMA_REQUIRE(most > 0, ARMA_EINVAL, "AR tile does not fit in shared memory");
+	const int per_sm = c->tuning.ar_ctas_per_sm > 0 ? std::min(most, c->tuning.ar_ctas_per_sm)
+	                                                : ctas_per_sm(load, c->num_sms, most, with_lead);
+	const size_t smem = most_bytes[per_sm <= with_lead ? 1 : 0];
 	const int grid = std::min(total, per_sm * c->num_sms);
-	int taps = 0;
-	for (const Task& t : tasks) taps = std::max(taps, t.pt * t.px * t.py);
+	bool by_task = false;
+	for (Task& t : tasks) {
+		t.lead = smem_bytes(t.pt, t.px, t.py, 1) <= smem;
+		share_device(t, load, total, grid, c->num_sms);
+		by_task = by_task || !t.lead || t.pace || t.diagonal != (total > grid);
+	}
 	Task* d_tasks = static_cast<Task*>(scratch_take(c, sizeof(Task) * tasks.size()));
 	int* d_ticket = static_cast<int*>(scratch_take(c, sizeof(int)));
 	ARMA_CUDA_TRY(copy_async(c, d_tasks, tasks.data(), sizeof(Task) * tasks.size(),
@@ -949,7 +982,7 @@ void launch_ar32c(Ctx* c, const std::vector<Ar32Surface>& surfaces, int tx, int 
 	ARMA_CUDA_TRY(cudaMemsetAsync(d_ticket, 0, sizeof(int), c->stream));
 	ProfScope prof_(c, "ar32c");
 	auto kernel = ar32c_kernel<false>;
-	if (keep_pace(taps, total, grid, c->num_sms)) {
+	if (by_task) {
 		kernel = ar32c_kernel<true>;
 		allow_smem(kernel, smem, kStaticSmem);
 	}
@@ -1068,7 +1101,7 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 	int dev = 0;
 	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
 		return fail(ARMA_ECUDA, "cudaGetDevice failed");
-	const size_t smem = smem_bytes(order[0], order[1], order[2]);
+	size_t smem = smem_bytes(order[0], order[1], order[2], 1);
 	int smem_optin = 0;
 	if (cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
 	    cudaSuccess)
@@ -1103,17 +1136,23 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 	int* d_ticket = reinterpret_cast<int*>(base + kOffTicket);
 	int* d_err = reinterpret_cast<int*>(base + kOffErr);
 	const int ntiles = tiles_x * tiles_y;
-	int per_sm = 0, sms = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ar32c_kernel<false>, NTHREADS,
+	const size_t smem0 = smem_bytes(order[0], order[1], order[2], 0);
+	int with_lead = 0, most = 0, sms = 0;
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&with_lead, ar32c_kernel<false>, NTHREADS,
 	                                                  smem) != cudaSuccess ||
+	    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, ar32c_kernel<false>, NTHREADS, smem0) !=
+	        cudaSuccess ||
 	    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
 		return fail(ARMA_ECUDA, "occupancy query failed");
-	if (per_sm <= 0) return fail(ARMA_ENOTSUP, "AR tile does not fit in shared memory");
+	if (most <= 0) return fail(ARMA_ENOTSUP, "AR tile does not fit in shared memory");
 	Load32 load;
 	load.add(Ar32Surface{t.nt, t.nx, t.ny, t.pt, t.px, t.py, d_zeta, t.phi, t.phi_lo, t.h, tiles_x,
 	                     tiles_y});
-	per_sm = ctas_per_sm(load, sms, per_sm);
+	const int per_sm = ctas_per_sm(load, sms, most, with_lead);
 	const int grid = std::min(ntiles, per_sm * sms);
+	t.lead = per_sm <= with_lead;
+	share_device(t, load, ntiles, grid, sms);
+	if (!t.lead) smem = smem0;
 	if (cudaMemcpyAsync(base + kOffTask, &t, sizeof(t), cudaMemcpyHostToDevice, st) != cudaSuccess ||
 	    cudaMemcpyAsync(d_coef, cbuf, sizeof(float) * ncoef, cudaMemcpyHostToDevice, st) !=
 	        cudaSuccess ||
@@ -1122,7 +1161,8 @@ extern "C" int arma_ar_filter_fp32c_noalloc(void* stream, const double* phi, con
 		(void)cudaStreamSynchronize(st);  // the staged host buffers are on this stack
 		return fail(ARMA_ECUDA, "staging the allocation-free AR filter failed");
 	}
-	auto kernel = keep_pace(P, ntiles, grid, sms) ? ar32c_kernel<true> : ar32c_kernel<false>;
+	const bool by_task = !t.lead || t.pace || t.diagonal != (ntiles > grid);
+	auto kernel = by_task ? ar32c_kernel<true> : ar32c_kernel<false>;
 	kernel<<<grid, NTHREADS, smem, st>>>(reinterpret_cast<const Task*>(base + kOffTask), 1, ntiles,
 	                                     d_ticket, d_err);
 	const bool launched = cudaGetLastError() == cudaSuccess;
