@@ -750,7 +750,7 @@ std::vector<Ar32Surface> ar32_surfaces(Ctx* c, int n, const double* const* phis,
 }
 
 // The FP64 filter of n surfaces in one launch, their coefficients in one
-// upload; its error word is read before anything uses the surfaces.
+// upload (a copy from pageable memory has been staged when it returns).
 void ar64_surfaces(Ctx* c, int n, const double* const* phis, const int* const* orders,
                    const int* const* shapes, double* const* zetas) {
 	// lags that no point of the surface has are left out: the reference's sums are
@@ -776,7 +776,6 @@ void ar64_surfaces(Ctx* c, int n, const double* const* phis, const int* const* o
 	ARMA_CUDA_TRY(copy_async(c, d, buf.data(), sizeof(double) * buf.size(),
 	                         cudaMemcpyHostToDevice, c->stream));
 	launch_ar64(c, s);
-	check_device_error(c);
 }
 
 void ar_filter(Ctx* c, const double* phi, const int order[3], const int shape[3],
@@ -784,6 +783,7 @@ void ar_filter(Ctx* c, const double* phi, const int order[3], const int shape[3]
 	if (precision == ARMA_FP64) {
 		double* z = static_cast<double*>(d_zeta);
 		ar64_surfaces(c, 1, &phi, &order, &shape, &z);
+		check_device_error(c);
 	} else {
 		const int tx = ar32c_tile_x(), ty = ar32c_tile_y();
 		float* z = static_cast<float*>(d_zeta);
@@ -1012,6 +1012,9 @@ void batch(Ctx* c, arma_surface* s, int n, int precision, bool host, bool redo =
 		}
 		ar64_surfaces(c, n, phis.data(), ords.data(), shps.data(), zs.data());
 		renorm_surfaces(c, s, n, precision, dz, host, luts);
+		// (read here, the host has not waited between the two; a call that fails
+		// leaves surfaces and scales that are not to be used)
+		check_device_error(c);
 		return;
 	}
 	long long* d_pairs = nullptr;
