@@ -61,7 +61,6 @@ struct Task64 {
 	int nbx, nc;      // tile rows, tiles per tile row
 	int ticket_base;
 	int ahead;        // halo steps kept ahead of their use
-	int polls;        // of the upstream tiles without progress before the wait gives up
 	double* zeta;
 	const double* phi;
 	int* flags;       // per tile: the step (t + u) up to which it is done
@@ -195,8 +194,8 @@ constexpr int kHaloBars = kMaxAhead + 1, kPubBars = 8;
 constexpr int kBarHalo = 1, kBarPub = kBarHalo + kHaloBars;
 static_assert(kBarPub + kPubBars <= 16, "named barriers");
 
-// The halo warp: a list of the halo's cells inside the surface (column; row in the
-// ring, place in its slot and lag in steps, 12, 12 and 8 bits), then step
+// The halo warp: a list of the halo's cells inside the surface (offset in a slice, which
+// has less than 2^31 points; place in a ring slot and lag in steps), then step
 // after step their new values.  A cell in row x' and column u' = U0 + d is read
 // from column max(U0, u' + b) of the tile on (b = X0 - x' rows above it, 0
 // beside it), so step n of the tile brings in its value of t = n - max(0, d +
@@ -204,7 +203,7 @@ static_assert(kBarPub + kPubBars <= 16, "named barriers");
 // further up than the five polled here are therefore covered by those, whose
 // own steps waited for them.  A wait that runs out sets the error word and lets
 // the compute warps run on without the halo: they end, and the call fails.
-template <int TX, int TU, int NC>
+template <int TX, int TU, int NC, int POLLS>
 __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const Layout64& L, double* ring,
                           int2* cells, Shared64* sh, int* err) {
 	const int lane = threadIdx.x & 31;
@@ -229,7 +228,7 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 		const unsigned m = __ballot_sync(0xffffffffu, ok);
 		if (ok)
 			cells[count + __popc(m & ((1u << lane) - 1))] =
-			    make_int2(y, row << 20 | (row * L.ld + col) << 8 | rel);
+			    make_int2(x * tk.ny + y, (row * L.ld + col) << 8 | rel);
 		count += __popc(m);
 	}
 	__syncwarp();
@@ -246,15 +245,13 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 	}
 	constexpr int kThreads = NC + 32;
 	const long long plane = (long long)tk.nx * tk.ny;
-	// row 0 of the ring (a plane can have more than 2^31 points)
-	const double* const top_row = tk.zeta + (long long)(X0 - (px - 1)) * tk.ny;
 	int n = 0;
 	bool failed = false;
 	while (n < steps) {
 		// the steps n .. hi whose upstream values are there and whose ring
 		// slots are free (and whose barriers' previous round is over)
 		int hi = -1;
-		for (int it = 0; it < tk.polls; ++it) {
+		for (int it = 0; it < POLLS; ++it) {
 			const int freed = ld_acquire_cta(&sh->done) + tk.ahead;
 			hi = min(freed, known == INT_MAX ? INT_MAX : known - U0);
 			hi = min(__reduce_min_sync(0xffffffffu, hi), steps - 1);
@@ -292,8 +289,8 @@ __device__ __forceinline__ void halo_warp(const Task64& tk, int bx, int c, const
 					const int2 cell = cells[e];
 					const int rel = cell.y & 255, t = st - rel;
 					if (t >= 0 && t < tk.nt) {
-						at[b] = (sm - rel + (sm < rel ? L.depth : 0)) * L.slot + (cell.y >> 8 & 0xfff);
-						v[b] = __ldcg(top_row + t * plane + (long long)(cell.y >> 20) * tk.ny + cell.x);
+						at[b] = (sm - rel + (sm < rel ? L.depth : 0)) * L.slot + (cell.y >> 8);
+						v[b] = __ldcg(tk.zeta + t * plane + cell.x);
 					}
 					e += 32;
 				}
@@ -550,7 +547,9 @@ __device__ __forceinline__ void compute_pairs(const Task64& tk, int bx, int c, c
 	}
 }
 
-template <int TX, int TU, int CELLS>
+// POLLS: of the upstream tiles without progress before the wait gives up (a constant:
+// read from the task, surfaces of few taps took 1 to 2 % longer).
+template <int TX, int TU, int CELLS, int POLLS = kSpinLimit>
 __global__ void __launch_bounds__(TX * TU / CELLS + 64)
 ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
                  int* __restrict__ counter, int* __restrict__ err) {
@@ -593,7 +592,7 @@ ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
 		if (tid >= NC + 32) {
 			pub_warp<TX, TU, NC>(tk, bx, c, &sh);
 		} else if (tid >= NC) {
-			halo_warp<TX, TU, NC>(tk, bx, c, L, ring, cells, &sh, err);
+			halo_warp<TX, TU, NC, POLLS>(tk, bx, c, L, ring, cells, &sh, err);
 		} else if constexpr (CELLS == 2) {
 			switch (tk.py) {
 #define ARMA_PY_CASE(N) case N: compute_pairs<N, TX, TU>(tk, bx, c, L, ring, sphi, &sh, err); break;
@@ -619,7 +618,7 @@ ar64_tile_kernel(const Task64* __restrict__ tasks, int ntasks, int tickets,
 
 // One launch per hyperplane, every thread the reference's truncated sum: for
 // coefficients that are not finite, whose products with the tiles' zero padding
-// would not vanish.
+// would not vanish, and slices of 2^31 points and more.
 constexpr int kPlaneThreads = 128;
 __global__ void __launch_bounds__(kPlaneThreads)
 ar64_plane_kernel(double* __restrict__ zeta, const double* __restrict__ phi,
@@ -663,6 +662,11 @@ void launch_planes(Ctx* c, const Ar64Surface& s) {
 	}
 }
 
+// Whether the tiles take a surface: finite coefficients, offsets in a slice of 32 bits.
+bool by_tiles(const Ar64Surface& s) {
+	return s.finite && (long long)s.nx * s.ny <= INT_MAX;
+}
+
 // The halo steps a tile of this shape can keep ahead; 0: it does not fit.
 int ahead_of(int tx, int tu, const Ar64Surface& s) {
 	for (int a = kMaxAhead; a > 0; --a)
@@ -700,11 +704,9 @@ void launch_tiles(Ctx* c, std::vector<Ar64Surface> surfs) {
 		t.nc = tiles_per_row(TX, TU, s.ny);
 		t.ticket_base = int(tickets);
 		t.ahead = ahead_of(TX, TU, s);
-		t.polls = kSpinLimit;
 		t.zeta = s.zeta;
 		t.phi = s.phi;
 		t.flags = nullptr;
-		t.tiles = nullptr;
 		tickets += (long long)t.nbx * t.nc;
 		ARMA_REQUIRE(tickets < INT_MAX / 4, ARMA_EINVAL, "surface too large");
 		smem = std::max(smem, layout64(TX, TU, s.pt, s.px, s.py, t.ahead).bytes);
@@ -766,7 +768,7 @@ void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces) {
 	long long t4 = 0;
 	double work = 0, chain = 0;
 	for (const Ar64Surface& s : surfaces)
-		if (s.finite) {
+		if (by_tiles(s)) {
 			const double taps = double(s.pt) * s.px * s.py;
 			t4 += (long long)((s.nx + 3) / 4) * tiles_per_row(4, 16, s.ny);
 			work += 256.0 * ((s.nx + 15) / 16) * tiles_per_row(16, 16, s.ny) * (s.nt + 15) * taps;
@@ -774,7 +776,7 @@ void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces) {
 		}
 	const int want = t4 <= c->num_sms ? 2 : work <= 96.0 * c->num_sms * chain ? 1 : 0;
 	for (const Ar64Surface& s : surfaces) {
-		if (!s.finite) launch_planes(c, s);
+		if (!by_tiles(s)) launch_planes(c, s);
 		else if (want == 0 && s.py <= kPairTaps && ahead_of(16, 16, s)) groups[0].push_back(s);
 		else if (want <= 1 && ahead_of(8, 16, s)) groups[1].push_back(s);
 		else if (ahead_of(4, 16, s)) groups[2].push_back(s);
@@ -798,7 +800,6 @@ void launch_ar64_starved(Ctx* c) {
 	t.nbx = 1;
 	t.nc = tiles_per_row(TX, TU, TU);  // 2
 	t.ahead = 1;
-	t.polls = kStarvedPolls;
 	t.zeta = zeta;
 	t.phi = zeta + cells;
 	t.flags = flags;
@@ -807,12 +808,11 @@ void launch_ar64_starved(Ctx* c) {
 	ARMA_CUDA_TRY(copy_async(c, d_task, &t, sizeof(t), cudaMemcpyHostToDevice, c->stream));
 	ARMA_CUDA_TRY(copy_async(c, flags, start, sizeof(start), cudaMemcpyHostToDevice, c->stream));
 	const size_t smem = layout64(TX, TU, t.pt, t.px, t.py, t.ahead).bytes;
-	ARMA_CUDA_TRY(cudaFuncSetAttribute(ar64_tile_kernel<TX, TU, 1>,
-	                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+	auto kernel = ar64_tile_kernel<TX, TU, 1, kStarvedPolls>;
+	ARMA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                   int(kSmemLimit)));
 	ProfScope prof_(c, "ar64");
-	ar64_tile_kernel<TX, TU, 1><<<1, TX * TU + 64, smem, c->stream>>>(d_task, 1, t.nc, flags + 2,
-	                                                                  c->d_err);
+	kernel<<<1, TX * TU + 64, smem, c->stream>>>(d_task, 1, t.nc, flags + 2, c->d_err);
 	ARMA_CUDA_TRY(cudaGetLastError());
 	c->launches += 1;
 }

@@ -29,7 +29,7 @@
 namespace armab {
 
 // Defined in mt_jump.cc: the coefficients of t^(2^e) mod phi, bit i of word i /
-// 32; false when the set has not full period.
+// 32; false when no polynomial of degree 32 nn - rr is found that the sequence obeys.
 bool mt_jump_bits(const arma_mt_params& prm, int e, std::vector<uint32_t>* bits);
 
 namespace {
@@ -242,12 +242,6 @@ mt_generate_half_kernel(const SegJob* __restrict__ jobs, int njobs) {
 	}
 }
 
-// The same sets with one CTA per segment, a thread per slot, for few segments.
-// Words are a CTA's time here, not the GPU's, so a barrier is paid once per four
-// steps: from the window of the last two steps (x[0 .. 2 mm)) thread t computes
-// its own slot's next four words C, D, E, F, and its right neighbour's C and D,
-// which E and F need, once more from the window.  The neighbours of the last two
-// slots are the first words of the next step (x[2 mm], x[2 mm + 1]).
 // A set's recurrence and tempering constants held in registers (opaque to the
 // compiler, which otherwise loads them again in every step).
 __device__ __forceinline__ arma_mt_params in_registers(arma_mt_params p) {
@@ -262,6 +256,12 @@ __device__ __forceinline__ uint32_t twist(uint32_t u, uint32_t v, const arma_mt_
 	return (y >> 1) ^ ((y & 1u) ? p.aaa : 0u);
 }
 
+// The same sets with one CTA per segment, a thread per slot, for few segments.
+// Words are a CTA's time here, not the GPU's, so a barrier is paid once per four
+// steps: from the window of the last two steps (x[0 .. 2 mm)) thread t computes
+// its own slot's next four words C, D, E, F, and its right neighbour's C and D,
+// which E and F need, once more from the window.  The neighbours of the last two
+// slots are the first words of the next step (x[2 mm], x[2 mm + 1]).
 __device__ __forceinline__ void half_four(const uint32_t* x, int t, int mm,
                                           const arma_mt_params& p, uint32_t (&w)[4]) {
 	const uint32_t a0 = x[t], a1 = x[t + 1], a2 = x[t + 2], b0 = x[mm + t];
@@ -487,7 +487,7 @@ std::vector<uint32_t> params_key(const arma_mt_params& p) {
 std::mutex g_table_mutex;
 std::map<std::vector<uint32_t>, uint32_t*> g_tables;
 
-// The device's t^(2^e) mod phi of a set, or null when it has not full period.
+// The device's t^(2^e) mod phi of a set, or null when there is no such phi.
 const uint32_t* jump_table(Ctx* c, const arma_mt_params& p, int e) {
 	auto key = params_key(p);
 	key.push_back(uint32_t(c->device));

@@ -118,7 +118,7 @@ Bits berlekamp_massey(const std::vector<uint8_t>& s, int* degree) {
 // A parameter set's powers t^(2^e) mod phi, e = 0, 1, ...: found once, extended
 // as larger exponents are asked for.
 struct JumpPowers {
-	Bits phi;             // empty: not a full-period set
+	Bits phi;             // empty: no polynomial of the state's degree
 	std::vector<Bits> g;  // g[e] = t^(2^e) mod phi
 };
 
@@ -148,7 +148,7 @@ JumpPowers find_powers(const arma_mt_params& prm) {
 		for (size_t j = 0; j < s.size(); ++j) s[j] = uint8_t(x[start + j] & 1u);
 		int L = 0;
 		r.phi = berlekamp_massey(s, &L);
-		if (L != p) {  // not a full-period set: the caller generates sequentially
+		if (L != p) {  // the caller generates sequentially
 			r.phi.clear();
 			return r;
 		}
