@@ -654,8 +654,8 @@ __device__ __forceinline__ void make_exp_table(double* tab) {
 }
 
 // window_fixed for entries where nothing overflows (-350 <= l z <= 0, l finite and
-// positive, h positive and not NaN: no entry of the reference's formula is
-// non-finite there, so no fix applies): with A = exp(l z), B = exp(-l (z + 2 h)) the window is 4 pi (A + B) /
+// positive: no entry of the reference's formula is non-finite there, so no fix
+// applies; h is not NaN, velocity_slices): with A = exp(l z), B = exp(-l (z + 2 h)) the window is 4 pi (A + B) /
 // (1 + A B), the same quotient as above.  At infinite depth one exponential and no
 // division: 30 FP64 instructions instead of 78 (400 x 128 x 128 FP32 at four
 // depths spent 205 us of the solver's 540 on windows).
@@ -670,7 +670,7 @@ __device__ __forceinline__ double window_at(int i, int j, int nx, int ny, double
 	const double az = k2Pi * sqrt(s2) * z;
 	// exp(-l z)^2 overflows: the entry is non-finite, 0 away from row and column 0
 	if (az < -360.0 && i > 0 && j > 0) return 0.0;
-	if (s2 > 0.0 && s2 <= DBL_MAX && az <= 0.0 && az >= -350.0 && h >= 0.0) {
+	if (s2 > 0.0 && s2 <= DBL_MAX && az <= 0.0 && az >= -350.0) {
 		const double A = exp_near(az, tab);
 		if (h == INFINITY) return k2Pi * 2.0 * A;
 		// -l (z + 2 h), formed as the reference's -2 l h minus l z
@@ -1756,6 +1756,10 @@ void velocity_slices(Ctx* c, const std::vector<VelSlice<T>>& slices, int nx, int
 	ARMA_REQUIRE(nz >= 1, ARMA_EINVAL, "no z levels");
 	const int ns = int(slices.size());
 	if (ns == 0) return;
+	// a depth that is not a number makes every entry of the window non-finite, as
+	// levels that are none do: those take the reference's formula (window_at)
+	const std::vector<double> none(std::isnan(depth) ? nz : 0, NAN);
+	if (!none.empty()) z = none.data();
 	const long long n2 = (long long)nx * ny;
 	auto* d_sl = static_cast<VelSlice<T>*>(scratch_take(c, sizeof(VelSlice<T>) * ns));
 	double* d_z = static_cast<double*>(scratch_take(c, sizeof(double) * nz));
