@@ -26,7 +26,8 @@
 // The ring has one slot more than the slices in use, so that the halo of slice
 // t+1 comes in while slice t is computed (512 x 256 x 256 points of order 10^3,
 // one tile per SM: 5.42 -> 5.20 ms; the batch of 256 surfaces 52.3 -> 51.8 ms;
-// one 64 x 32 x 32 surface 258 -> 241 us).
+// one 64 x 32 x 32 surface 258 -> 241 us); the largest orders can go without it
+// (launch_ar32c).
 // The coefficients are carried as hi + lo float pairs (rounding phi to one
 // float perturbs a high-gain recursion far more than FP32 summation does):
 // each (k,i) row of taps feeds two FP32 FMA chains over one register window,

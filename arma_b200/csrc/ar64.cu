@@ -35,7 +35,7 @@
 // two, against 8.2 for the chain.  Where throughput counts, a thread owns two
 // cells, (x, y) and (x+1, y-1) of one u, that share the taps and all but one
 // operand of a row (compute_pairs): four warps then move 256 cells in 21 cycles, 16
-// mixed surfaces 11.9 -> 10.2 ms.  Two warps of pairs are no faster than four of
+// mixed surfaces 11.9 -> 10.2 ms (9.4 by anti-diagonals, launch_tiles).  Two warps of pairs are no faster than four of
 // single cells (13.5 and 13.9): a lone warp's issue bounds them.
 #include <algorithm>
 #include <climits>
@@ -758,8 +758,8 @@ void launch_ar64(Ctx* c, const std::vector<Ar64Surface>& surfaces) {
 	// SM (all steps of all tiles over the longest chain).  16 x 16 by pairs moves
 	// the most cells per cycle and is the slowest step (21 cycles a tap): taken
 	// where more than 96 cells per SM are at work.  8 x 16 (14 cycles a tap) below
-	// that, 4 x 16 (11) where all its tiles have an SM to themselves.  Measured, 16
-	// x 16 / 8 x 16 / 4 x 16 (ms): 40 cells per SM 3.9 / 2.7 / 3.1; 79 (400 x 128 x
+	// that, 4 x 16 (11) where all its tiles have an SM to themselves.  Measured (tiles
+	// row by row), 16 x 16 / 8 x 16 / 4 x 16 (ms): 40 cells per SM 3.9 / 2.7 / 3.1; 79 (400 x 128 x
 	// 128 of order 10^3) 7.0 / 4.9 / 5.5; 108 3.7 / 4.4 / 4.6; 142 10.1 / 10.9 /
 	// 12.1; 415 (16 mixed surfaces) 10.2 / 13.7 / 17.5; 200 x 40 x 40 alone, 30 tiles
 	// of 4 x 16, 1.14 / 0.76 / 0.65.  8 x 16 too for rows of more taps than a pair's
